@@ -226,21 +226,21 @@ int32_t vfs_model_get_neighbor_capacity(const vfs_model* m);
  * particle whose list was built from 125 provably distinct cell keys sums the list instead of
  * walking the 27 buckets of CalculateDensities (wcsph_with_boundary_model.slang:153-197). The
  * in-range sets are the reference's; the sums follow the visiting order of the last build. Lists
- * that go stale within 12 substeps of their build (a build substep costs about two walks) make
- * the scene wait up to 256 substeps before building again (it walks meanwhile), so the lists pay
- * off where the fastest particle moves less than about h skin / 24 per substep and cost a few
- * percent where particles move faster. skin in [0, 0.5],
+ * that go stale within 4 substeps of their build (12 in scenes below 32,768 particles, 2 from
+ * 262,144 on, where a build substep costs about one and a half walks) make the scene wait up to 256 substeps before
+ * building again (it walks meanwhile), so the lists pay off where the fastest particle moves less
+ * than about h skin / 4 per substep and cost a few percent where particles move faster. skin in [0, 0.5],
  * default 0.05; 0 walks the buckets every substep. Models of up to ~39,000 particles (three lanes
- * per particle in the density pass) and models whose lists do not fit in device memory (224 bytes
+ * per particle in the density pass) and models whose lists do not fit in device memory (433 bytes
  * per particle) have no lists; the getter then reports 0. */
 int vfs_model_set_skin(vfs_model* m, float skin);
 int vfs_model_get_skin(const vfs_model* m, float* skin);
 /* Block-per-cell staging in the density pass's bucket walk (CalculateDensities,
- * wcsph_with_boundary_model.slang:153-197): a warp whose particles share one row of
- * cells loads the 3 x 3 rows of cells around it into shared memory once and tests every staged
- * particle against each of its own, instead of each thread walking its 27 buckets from global
- * memory. Results are bit-identical either way. Off by default; the autotuner's choice
- * (vfs_tune_config.walk_staging) turns it on for workloads where it is faster. */
+ * wcsph_with_boundary_model.slang:153-197) where a crowd of a single scene's particles has no
+ * usable skin list (a dense blob): a warp whose particles share a few rows of cells loads the
+ * 3 x 3 rows of cells around them into shared memory once and tests every staged particle against
+ * each of its own on the tensor cores, instead of a warp walking one particle's 27 buckets.
+ * Results are bit-identical either way. On by default (vfs_tune_config.walk_staging). */
 int vfs_model_set_walk_staging(vfs_model* m, int32_t enable);
 /* Number of list builds so far (synchronises the handle's stream). */
 int vfs_model_get_skin_builds(vfs_model* m, uint32_t* builds);
@@ -312,7 +312,7 @@ typedef struct vfs_tune_config {
     int32_t cell_block;      /* keys per block of the cell-range / reorder kernel: 128, 256, 512 */
     int32_t force_block;     /* force pass: threads per block and minimum resident blocks per */
     int32_t force_min_blocks;/* SM, the same four shapes; 0, 0 = the neighbour passes' shape */
-    int32_t walk_staging;    /* block-per-cell staging of the density walk: 1 on, 0 off */
+    int32_t walk_staging;    /* block-per-cell staging of a crowd's density walk: 1 on, 0 off */
 } vfs_tune_config;
 /* Times every candidate of each stage (sort, neighbour passes, cell ranges) for `repeats`
  * substeps from the model's current state, keeps the fastest, and restores the state (the

@@ -618,7 +618,7 @@ int Model::init() {
     return refresh_params();
 }
 
-// Candidate lists with a skin, 228 bytes per particle. Three-lane (small) models do not use them,
+// Candidate lists with a skin, 433 bytes per particle. Three-lane (small) models do not use them,
 // and a model too large for them on this device runs without (every particle walks its buckets).
 int Model::alloc_skin() {
     if (n == 0 || planes_mode(n)) return VFS_OK;
@@ -635,7 +635,7 @@ int Model::alloc_skin() {
         cudaMalloc(&s.ctl, scenes.size() * kSkinCtl * sizeof(uint32_t)) != cudaSuccess ||
         cudaMalloc(&s.queue, N * sizeof(uint32_t)) != cudaSuccess ||
         cudaMalloc(&s.seg_n, ((N + 127) / 128) * sizeof(uint32_t)) != cudaSuccess ||
-        cudaMalloc(&s.wcount, sizeof(uint32_t)) != cudaSuccess) {
+        cudaMalloc(&s.wcount, 2 * sizeof(uint32_t)) != cudaSuccess) {
         cudaGetLastError();  // out of memory is not sticky: clear it and go on without lists
         cudaFree(s.list);
         cudaFree(s.count);
@@ -653,7 +653,7 @@ int Model::alloc_skin() {
     VFS_CUDA_TRY(cudaMemset(s.count, 0, N * sizeof(uint32_t)));
     VFS_CUDA_TRY(cudaMemset(s.b_of_id, 0, N * sizeof(uint32_t)));  // any index below n until a build
     VFS_CUDA_TRY(cudaMemset(s.stale, 0, scenes.size() * sizeof(uint32_t)));
-    VFS_CUDA_TRY(cudaMemset(s.wcount, 0, sizeof(uint32_t)));
+    VFS_CUDA_TRY(cudaMemset(s.wcount, 0, 2 * sizeof(uint32_t)));
     skin = s;
     return invalidate_skin();
 }

@@ -3,8 +3,6 @@
 //   * the radix sort's digit width (6, 7 or 8 bits) and items per thread (8, 12 or 16),
 //   * the neighbour passes' block shape (threads per block x minimum resident blocks per SM),
 //   * the cells-per-block of the cell-range / reorder kernel (128, 256 or 512 keys),
-//   * whether the density walk stages a warp's row of cells in shared memory (block-per-cell
-//     staging; it helps where walking warps share rows and the per-thread walk prunes little).
 // None of these changes any result: the sort is stable whatever its digits, and every particle's
 // sums are accumulated by one thread in the same order whatever the block shape. Candidates are
 // timed with CUDA events on the model's stream from the same saved state (restored before every
@@ -179,10 +177,10 @@ int autotune(Model& m, int repeats, bool use_cache, vfs_tune_config* chosen) {
                 }
             }
     }
-    // The walk kernel's shape and staging matter only in substeps that walk (no lists, a stale
-    // scene, a list build); while a scene's lists are current it returns at once, and a
-    // comparison there would pick by noise. So stages 2 and 3 run with the lists off (every
-    // substep walks); they are switched back on afterwards, and rebuilt by the next substep.
+    // The walk kernel's shape matters only in substeps that walk (no lists, a stale scene that
+    // waits); while a scene's lists are summed it returns at once, and a comparison there would
+    // pick by noise. So stage 2 runs with the lists off (every substep walks); they are switched
+    // back on afterwards, and rebuilt by the next substep.
     const float keep_skin = m.skin_fraction;
     if (rc == VFS_OK && keep_skin > 0.0f) rc = set_skin(m, 0.0f);
     // Stage 2: block shapes of the density and force passes (independent kernels, one sweep).
@@ -206,25 +204,11 @@ int autotune(Model& m, int repeats, bool use_cache, vfs_tune_config* chosen) {
             }
         }
     }
-    // Stage 3: staging of the density walk, with the chosen density shape.
-    if (rc == VFS_OK) {
-        float best_t = 1e30f;
-        vfs_tune_config c = best;
-        for (int st : {0, 1}) {
-            c.walk_staging = st;
-            measure(c, ph);
-            if (rc) break;
-            if (ph[3] < best_t) {
-                best_t = ph[3];
-                best.walk_staging = st;
-            }
-        }
-    }
     if (keep_skin > 0.0f) {
         const int rs = set_skin(m, keep_skin);
         if (rc == VFS_OK) rc = rs;
     }
-    // Stage 4: cells per block of the cell-range / reorder kernel.
+    // Stage 3: cells per block of the cell-range / reorder kernel.
     if (rc == VFS_OK) {
         float best_t = 1e30f;
         vfs_tune_config c = best;
@@ -283,7 +267,7 @@ int tune_cache_load(const char* path) {
         char key[256];
         vfs_tune_config c{};
         // Lines of 6 values (no force shape) take the neighbour shape for the force pass; lines
-        // without the walk-staging value (6 or 8 values) walk per thread.
+        // without the walk-staging value (6 or 8 values) walk a crowd without tiles.
         c.walk_staging = 0;
         const int got = std::sscanf(line, "%255s %d %d %d %d %d %d %d %d", key, &c.sort_digit_bits,
                                     &c.sort_tile_items, &c.nbr_block, &c.nbr_min_blocks,

@@ -124,20 +124,21 @@ SortConfig make_sort_config(uint32_t n, int digit_bits, int tile_items, int key_
 
 // Launch shapes of the neighbour passes: threads per block x minimum resident blocks per SM.
 enum NbrShape : int { kNbr128x6 = 0, kNbr128x8 = 1, kNbr96x8 = 2, kNbr64x12 = 3, kNumNbrShapes = 4 };
-// Candidate lists with a skin (Verlet lists). A build, in a density pass, lists for every particle
-// the particles within h (1 + skin), in the reference's visiting order, under the particles' sorted
-// indices of that substep (their build indices), and keeps each particle's position. Until some
+// Candidate lists with a skin (Verlet lists). A build, at the start of a density pass, lists for
+// every particle the particles within h (1 + skin) (and a few just beyond), in the reference's
+// visiting order, under the particles' sorted indices of that substep (their build indices), and
+// keeps each particle's position. Until some
 // particle of the scene has moved more than h skin / 2 since then, every pair within h is in the
 // lists, and a particle whose list is usable sums it instead of walking the 27 buckets (same
 // in-range set, multiplicity one). The cell pass keeps `cur`, the current sorted index of every
 // build index, checks every displacement against `x_build` and marks the scene stale; in a stale
 // scene every particle walks, and the lists are rebuilt when the scene's build policy allows it.
-// The force pass runs the policy: a stale scene walks at least one substep before it rebuilds;
-// lists that went stale within kSkinMinLife substeps of their build, or a build that left fewer
-// than half of the scene's lists usable, double the substeps it walks before the next build
-// (from kSkinMinWait to kSkinMaxWait); longer-lived lists rebuild as soon as they go stale. A
-// single scene whose last build left most lists unusable is walked in index order, as a stale
-// one is, until its next build.
+// The force pass runs the policy: lists that went stale within kSkinMinLife... substeps of their
+// build (by the scene's size), or a build that left more than one in kSkinPoorPart particles
+// without a usable list, double the substeps the scene walks before the next build (from
+// kSkinMinWait to kSkinMaxWait); longer-lived lists are rebuilt in the substep they go stale in
+// (small scenes: in the next). A single scene whose last build left too many lists unusable is
+// walked in index order, as a stale one that waits is, until its next build.
 struct SkinLists {
     uint32_t* list = nullptr;     // slot-major: list[k * total + b] = build index of candidate k of b
     uint32_t* count = nullptr;    // per build index: list length, kSkinUsable when it can be summed
@@ -149,14 +150,15 @@ struct SkinLists {
                                   // index (w, as bits), written by the cell pass
     uint32_t* stale = nullptr;    // per scene: nonzero when some particle moved past h skin / 2
     uint32_t* ctl = nullptr;      // per scene, kSkinCtl words: the build policy's state (kCtl*)
-    uint32_t* queue = nullptr;    // the particles the density pass walks this substep: those of
+    uint32_t* queue = nullptr;    // the particles the density pass walks this substep; a batch's of
                                   // list block b at [128 b, 128 b + seg_n[b]), in index order
-    uint32_t* seg_n = nullptr;    // per list block (128 particles): its walkers
-    uint32_t* wcount = nullptr;   // single scene: walkers in `queue`, packed from 0 (one word)
+    uint32_t* seg_n = nullptr;    // batched: per list block (128 particles) its walkers
+    uint32_t* wcount = nullptr;   // two words: a single scene's walkers in `queue`, packed from 0;
+                                  // nonzero when some scene's build is due this substep
     uint32_t cap = 0;             // slots per particle
 };
 constexpr uint32_t kSkinUsable = 1u << 31;
-constexpr uint32_t kSkinCtl = 8;       // words of policy state per scene:
+constexpr uint32_t kSkinCtl = 16;      // words of policy state per scene:
 constexpr uint32_t kCtlAllow = 0;      //   a stale scene may rebuild this substep
 constexpr uint32_t kCtlAge = 1;        //   substeps since the last build
 constexpr uint32_t kCtlWait = 2;       //   stale substeps to walk before the next build
@@ -164,19 +166,35 @@ constexpr uint32_t kCtlBuilds = 3;     //   builds so far
 constexpr uint32_t kCtlFresh = 4;      //   the lists of the last build have not gone stale yet
 constexpr uint32_t kCtlSince = 5;      //   stale substeps since the lists went stale
 constexpr uint32_t kCtlUsable = 6;     //   usable lists left by this substep's build
-constexpr uint32_t kCtlPoor = 7;       //   the last build left fewer than half of them usable
-constexpr uint32_t kSkinMinLife = 12;  // a build substep costs about two walks; a list pass saves ~0.45 of one
+constexpr uint32_t kCtlPoor = 7;       //   the last build left too few of them usable
+constexpr uint32_t kCtlYoung = 8;      //   lists in a row that died young
+// Lists that die younger than this were not worth their build. A full GPU (1M particles): a build
+// substep 650 us, a list pass 195, a walk 450, so two substeps of use pay; a scene of 64,000
+// particles, where all three are latency: 90, 33 and 49 us, so four do; a small scene of a batch
+// walks beside the others' queues for nothing, while its build's 40 us are on the batch's critical
+// path (20 scenes of 2,500 to 21,500 particles: 194 us a substep at four, 184 at twelve).
+constexpr uint32_t kSkinSmallScene = 32768u, kSkinFullScene = 262144u;
+constexpr uint32_t kSkinMinLifeSmall = 12;
+constexpr uint32_t kSkinMinLife = 4;
+constexpr uint32_t kSkinMinLifeFull = 2;
+// A full scene's lists that die young once (a state set from outside just after a build) are
+// rebuilt all the same: that costs a third of a walk, waiting would cost half a walk each substep.
+constexpr uint32_t kSkinGrace = 1;
+// More than one in so many without a usable list: the list pass and their scattered walk together
+// cost more than walking every particle (1M settled particles, a third over 64 slots: 910 us against 690
+// a substep).
+constexpr uint32_t kSkinPoorPart = 8;
 constexpr uint32_t kSkinMinWait = 8;
 constexpr uint32_t kSkinMaxWait = 256;
-constexpr uint32_t kSkinCap = 48;  // also the density walk's shared list, where a build is staged
+constexpr uint32_t kSkinCap = 96;  // candidates within 1.05 h: ~39 at spacing h / 2, ~49 in a settled fluid (0.46 h),
+                                   // ~74 there at a skin of 0.2
 
 // Launch shapes chosen per model (by default or by the autotuner); none changes any result.
 struct KernelConfig {
-    int nbr_shape = kNbr96x8;     // density pass (and the adjoint's recomputed forward)
+    int nbr_shape = kNbr96x8;     // density pass's per-thread walk (and the adjoint's recomputed forward)
     int force_shape = kNbr128x8;  // force pass (no shared memory: it takes the larger blocks)
     int cell_block = 256;  // keys per block of the cell-range / reorder kernel: 128, 256 or 512
-    int walk_staging = 0;  // density walk: warps whose particles share a row of cells stage it
-                           // (off by default: the autotuner turns it on where it is faster)
+    int walk_staging = 1;  // a crowd of queued walkers is walked as staged tiles (0: a warp per walker)
 };
 size_t sort_scratch_words(const SortConfig& c);
 
@@ -235,7 +253,8 @@ cudaError_t launch_lookback_selftest(bool published, uint32_t spin_limit, uint32
 bool planes_mode(uint32_t total);
 // Boundary volume + density + EOS epilogue; writes each particle's neighbour list.
 // Also writes rec[2i], rec[2i+1] = (x, y, z, p/rho^2), (v, m/max(rho, 1e-6)) for the force pass.
-// With skin lists (sk.list set): sums the lists where they are usable and rebuilds flagged scenes.
+// With skin lists (sk.list set): rebuilds flagged scenes, sums the lists where they are usable and
+// walks the rest (kc.walk_staging: see KernelConfig).
 // walk_sched: two device words, zero between launches (the walk kernel's run counter, put back to
 // zero by its last warp).
 cudaError_t launch_density(const StepLaunch& L, const float4* pos, const float4* vel, float4* rec,

@@ -1,10 +1,11 @@
 // sm_103a kernels of one WCSPH-with-boundary substep (VkFluidSim's
 // WCSPHWithBoundaryModel::Step, src/models/wcsph_with_boundary_model.cpp:81-117):
 //
-//   k_keys            key[i] = HashCell3D(floor(x_i / h)) % N  + per-pass digit histograms
+//   k_keys_flags      key[i] = HashCell3D(floor(x_i / h)) % N, moved flags, digit histograms
 //   k_onesweep        stable LSD radix pass of (key, index) with decoupled look-back
 //   k_cells_reorder   cell_scan[] (lower bound of every key) + gather of x, v (and ids in x.w)
-//   k_density         volume-map boundary terms + density + Tait EOS epilogue
+//   k_density_list    volume-map boundary terms + density + Tait EOS epilogue over the skin lists
+//                     (k_skin_build builds them; k_walk_queue and k_walk walk what has none)
 //   k_force           pressure + viscosity + wall penalty + symplectic Euler
 //
 // Data layout: particle state is float4 SoA (x,y,z,id-bits) and (vx,vy,vz,0) in sorted order;
@@ -528,8 +529,9 @@ __global__ void __launch_bounds__(kCellBlock)
                     uint32_t* __restrict__ pkeys_out, uint32_t* guess,
                     const uint32_t* __restrict__ b_of_id, float4* __restrict__ xcur,
                     const float4* __restrict__ x_build, uint32_t* __restrict__ stale,
-                    const uint32_t* __restrict__ ctl) {
+                    const uint32_t* __restrict__ ctl, uint32_t* __restrict__ wcount) {
     __shared__ uint32_t s_lo, s_hi;
+    if (wcount && blockIdx.x == 0 && threadIdx.x == 0) wcount[0] = 0u;  // the list pass's queue
     // The sort is done with its scratch (histograms, tile counters, look-back status): clear it
     // for the next substep here instead of in a separate memset.
     for (uint32_t w = blockIdx.x * kCellBlock + threadIdx.x; w < zero_words; w += gridDim.x * kCellBlock)
@@ -587,8 +589,10 @@ __global__ void __launch_bounds__(kCellBlock)
         const uint32_t m = __ballot_sync(0xffffffffu, exceed);
         if (exceed) {
             const uint32_t g = __match_any_sync(m, exceed_sc);
-            if ((tid & 31u) == (uint32_t)(__ffs(g) - 1) && ld_volatile(stale + exceed_sc) == 0u)
+            if ((tid & 31u) == (uint32_t)(__ffs(g) - 1) && ld_volatile(stale + exceed_sc) == 0u) {
                 atomicOr(stale + exceed_sc, 1u);
+                if (ctl[exceed_sc * kSkinCtl + kCtlAllow]) wcount[1] = 1u;  // a build is due
+            }
         }
     }
     __syncthreads();
@@ -734,169 +738,33 @@ __device__ __forceinline__ float in_range2(const float4& xi, const float4& xj) {
     return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
 }
 
-// Along one axis, how many of the cells c-2..c+2 share the 50-cell hash block of c-2 (5 when all
-// do). Five consecutive cells span at most two blocks: the short block before the 2^32 wrap of
-// cell + 25 is 46 cells long.
-__device__ __forceinline__ int first_block_cells(uint32_t c) {
-    const uint32_t b0 = (c - 2u + 25u) / 50u;
-    int n = 1;
-#pragma unroll
-    for (int t = 1; t < 5; t++) n += (c - 2u + (uint32_t)t + 25u) / 50u == b0 ? 1 : 0;
-    return n;
-}
-
-// Whether box a (keys (ka + x + 50 y + 2500 z) mod n for x, y, z below its widths wa) and box b
-// (keys from kb, widths wb) share a key: each key of a, minus kb modulo n, is one of b's offsets
-// exactly when its digits in base 50 / 2500 lie below b's widths (every offset is < 5 + 50 * 5 +
-// 2500 * 5 < n, so the decomposition is unique). Kept out of line: it runs for few particles, and
-// inlined into the walk kernel it cost the 1M scene's list-building substep half again (density
-// 0.94 ms against 0.60, same rule, same decisions).
-__device__ __noinline__ bool boxes_share_a_key(uint32_t ka, uint32_t wax, uint32_t way, uint32_t waz,
-                                               uint32_t kb, uint32_t wbx, uint32_t wby, uint32_t wbz,
-                                               uint32_t n) {
-#pragma unroll 1
-    for (uint32_t z = 0; z < waz; z++)
-#pragma unroll 1
-        for (uint32_t y = 0; y < way; y++)
-#pragma unroll 1
-            for (uint32_t x = 0; x < wax; x++) {
-                uint32_t key = ka + x + 50u * y + 2500u * z;
-                if (key >= n) key -= n;  // ka < n and the offset is below n
-                const uint32_t d = key >= kb ? key - kb : key + (n - kb);
-                const uint32_t oz = d / 2500u, r = d - 2500u * oz, oy = r / 50u, ox = r - 50u * oy;
-                if (ox < wbx && oy < wby && oz < wbz) return true;
-            }
-    return false;
-}
-
-// Box `slot` of the 5 x 5 x 5 block around (cx, cy, cz): bit 0 (1, 2) of the slot picks the
-// cells of the block's first or second 50-cell hash block along x (y, z). Returns false when the
-// slot is not a box of this block (the block lies in one hash block along that axis); otherwise
-// its first key k, the span of its hashes (its last minus its first) and its widths, or wraps =
-// true when its hashes wrap 2^32. Computed from the slot alone, so no per-box array is kept.
-__device__ __forceinline__ bool key_box(const SceneParams& p, uint32_t cx, uint32_t cy, uint32_t cz,
-                                        uint32_t fx, uint32_t fy, uint32_t fz, uint32_t slot,
-                                        uint32_t& k, uint32_t& span, uint32_t w[3], bool& wraps) {
-    const bool bx = slot & 1u, by = slot & 2u, bz = slot & 4u;
-    if ((bx && fx == 5u) || (by && fy == 5u) || (bz && fz == 5u)) return false;
-    const uint32_t x0 = bx ? fx : 0u, x1 = bx ? 4u : fx - 1u;
-    const uint32_t y0 = by ? fy : 0u, y1 = by ? 4u : fy - 1u;
-    const uint32_t z0 = bz ? fz : 0u, z1 = bz ? 4u : fz - 1u;
-    const uint32_t lo = hash_cell(cx - 2u + x0, cy - 2u + y0, cz - 2u + z0);
-    const uint32_t hi = hash_cell(cx - 2u + x1, cy - 2u + y1, cz - 2u + z1);
-    wraps = hi < lo;
-    k = key_mod(lo, p.mod_magic, p.n);
-    span = hi - lo;
-    w[0] = x1 - x0 + 1u;
-    w[1] = y1 - y0 + 1u;
-    w[2] = z1 - z0 + 1u;
-    return true;
-}
-
-// True when the 125 cells around (cx, cy, cz) have distinct keys, so that a walk of their buckets
-// meets every particle once. The block splits into at most eight boxes, one per hash block it
-// touches; inside a box the hashes are hmin + lx + 50 ly + 2500 lz, so its keys lie in the
-// circular interval [hmin mod n, hmin mod n + span] (span <= 10204) and are distinct when
-// n > 10204 and the box's hashes do not wrap 2^32. Boxes whose intervals are disjoint modulo n
-// share no key; boxes whose intervals overlap are compared key by key (boxes_share_a_key), so
-// the answer is exact under those two conditions. Most blocks lie in one hash block (one box, no
-// pair to compare); the boxes of a pair are recomputed from their slots rather than kept in a
-// per-thread array, which would live in local memory.
-__device__ __forceinline__ bool skin_keys_distinct(const SceneParams& p, uint32_t cx, uint32_t cy,
-                                                   uint32_t cz) {
-    if (p.n <= 10204u) return false;
-    const uint32_t fx = (uint32_t)first_block_cells(cx), fy = (uint32_t)first_block_cells(cy),
-                   fz = (uint32_t)first_block_cells(cz);
-    uint32_t ka, sa, wa[3], kb, sb, wb[3];
-    bool wraps;
-#pragma unroll 1
-    for (uint32_t a = 0; a < 8u; a++) {
-        if (!key_box(p, cx, cy, cz, fx, fy, fz, a, ka, sa, wa, wraps)) continue;
-        if (wraps) return false;
-#pragma unroll 1
-        for (uint32_t b = 0; b < a; b++) {
-            if (!key_box(p, cx, cy, cz, fx, fy, fz, b, kb, sb, wb, wraps)) continue;
-            const uint32_t ab = kb >= ka ? kb - ka : kb + (p.n - ka);  // (k_b - k_a) mod n
-            const uint32_t ba = ka >= kb ? ka - kb : ka + (p.n - kb);
-            if ((ab <= sa || ba <= sb) &&
-                boxes_share_a_key(ka, wa[0], wa[1], wa[2], kb, wb[0], wb[1], wb[2], p.n))
-                return false;
-        }
-    }
-    return true;
-}
-
-// Squared distance, in h^2, from a particle at fraction f of its cell to the slab of cells at
-// offset d in [-2, 2] along one axis.
-__device__ __forceinline__ float slab_dist2(int d, float f) {
-    const float l = d < 0 ? f + (float)(-d - 1) : (d > 0 ? (float)d - f : 0.0f);
-    const float c = fmaxf(l, 0.0f);
-    return c * c;
-}
-
-// The list build of a particle whose 125 keys are distinct: the sorted indices (this substep's,
-// which become the build indices) of every particle within h (1 + skin), stored at out[k stride],
-// from the 5x5x5 cells around (cx, cy, cz) whose boxes lie within that radius: planes dz and
-// rows dy in increasing order, the cells of a row in increasing x as runs of consecutive keys (a
-// run ends at a hash-block boundary; a run whose keys pass n - 1 continues at key 0) - the
-// reference's visiting order restricted to its 27 cells. Returns the number found (ids past
-// `cap` are not stored).
-__device__ __forceinline__ uint32_t skin_walk(const SceneParams& p, const uint32_t* __restrict__ scan,
-                                              const float4* __restrict__ pos, const float4& xi,
-                                              uint32_t cx, uint32_t cy, uint32_t cz,
-                                              uint32_t* __restrict__ out, size_t stride,
-                                              uint32_t cap) {
-    const float fx = fmaf(-(float)(int)cx, p.h, xi.x) * p.inv_h;
-    const float fy = fmaf(-(float)(int)cy, p.h, xi.y) * p.inv_h;
-    const float fz = fmaf(-(float)(int)cz, p.h, xi.z) * p.inv_h;
-    const float lim = p.skin_lim;
-    const uint32_t* sc = scan + p.off;
-    uint32_t c = 0;
-    auto walk = [&](uint32_t b, uint32_t e) {
-#pragma unroll 1
-        for (uint32_t j = b; j < e; j++) {
-            const float4 xj = __ldg(pos + j);
-            if (in_range2(xi, xj) <= p.skin_r2) {
-                if (c < cap) out[c * stride] = j;
-                c++;
-            }
-        }
-    };
-#pragma unroll 1
-    for (int dz = -2; dz <= 2; dz++) {
-        const float sz = slab_dist2(dz, fz);
-        if (sz > lim) continue;
-#pragma unroll 1
-        for (int dy = -2; dy <= 2; dy++) {
-            const float syz = sz + slab_dist2(dy, fy);
-            if (syz > lim) continue;
-            int xl = -2, xr = 2;  // cell 0 is always within the limit here
-            while (xl < 0 && syz + slab_dist2(xl, fx) > lim) xl++;
-            while (xr > 0 && syz + slab_dist2(xr, fx) > lim) xr--;
-            const uint32_t ry = cy + (uint32_t)dy, rz = cz + (uint32_t)dz;
-#pragma unroll 1
-            for (int x = xl; x <= xr;) {
-                const uint32_t bx = (cx + (uint32_t)x + 25u) / 50u;
-                int xe = x;
-                while (xe < xr && (cx + (uint32_t)(xe + 1) + 25u) / 50u == bx) xe++;
-                const uint32_t k0 = key_mod(hash_cell(cx + (uint32_t)x, ry, rz), p.mod_magic, p.n);
-                const uint32_t len = (uint32_t)(xe - x + 1);
-                if (k0 + len <= p.n) {
-                    walk(__ldg(sc + k0), __ldg(sc + k0 + len));
-                } else {
-                    walk(__ldg(sc + k0), __ldg(sc + p.n));
-                    walk(__ldg(sc), __ldg(sc + (k0 + len - p.n)));
-                }
-                x = xe + 1;
-            }
-        }
-    }
-    return c;
-}
-
 // Threads per block of the density pass over the skin lists; the walk queue is kept in segments of
 // one such block.
 constexpr int kListBlock = 128;
+
+// A single scene's queue of at least this many walkers is walked in runs of 32 (where one wave of
+// warps, ~2,400, has three particles each to walk a warp per walker); a smaller one a warp per walker.
+constexpr uint32_t kWalkerCrowd = 8192;
+
+// 1 / sqrt(x) for a normal x (the form without ftz spends four more instructions on denormals).
+__device__ __forceinline__ float rsqrt_normal(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// W(|x_j - x_i|) / sigma from r2 = in_range2(x_i, x_j), explicitly rounded, so every walk and
+// launch shape gives the same sums. Branch-free: 2 (1-q)^3 above q = 1/2, 6q^3 - 6q^2 + 1 below,
+// 0 past 1. (A denormal r2 counts as 0: W is 1 either way.)
+__device__ __forceinline__ float w_over_sigma_r2(float r2, float inv_h) {
+    const float r = r2 > 1.0e-37f ? __fmul_rn(r2, rsqrt_normal(r2)) : 0.0f;
+    const float q = __fmul_rn(r, inv_h);
+    const float t = __fsub_rn(1.0f, q);
+    const float w_out = __fmul_rn(__fmul_rn(__fmul_rn(t, t), t), 2.0f);
+    const float q2 = __fmul_rn(q, q);
+    const float w_in = __fmaf_rn(6.0f, __fmul_rn(q2, q), __fmaf_rn(-6.0f, q2, 1.0f));
+    return q <= 1.0f ? (q > 0.5f ? w_out : w_in) : 0.0f;
+}
 
 // Particle i's density sum and neighbour list as the density pass builds them: add() takes one
 // in-range neighbour, adds its W / sigma (explicitly rounded, so every launch shape and both the
@@ -907,21 +775,14 @@ struct DensitySum {
     uint32_t* out;  // slot `listed` of i's list (slot-major, stride = particles)
     __device__ __forceinline__ void add(uint32_t i, const float4& xi, uint32_t j, const float4& xj,
                                         float inv_h, uint32_t cap, uint32_t stride) {
-        add_r2(i, j, in_range2(xi, xj), inv_h, cap, stride);
+        add_r2(i, j, in_range2(xi, xj), true, inv_h, cap, stride);
     }
-    // The same with r2 = in_range2(x_i, x_j) already computed (by the in-range test).
-    __device__ __forceinline__ void add_r2(uint32_t i, uint32_t j, float r2, float inv_h,
+    // The same with r2 = in_range2(x_i, x_j) already computed, for a candidate that counts only
+    // when `in` (adding 0 leaves the sum as it is).
+    __device__ __forceinline__ void add_r2(uint32_t i, uint32_t j, float r2, bool in, float inv_h,
                                            uint32_t cap, uint32_t stride) {
-        const float r = r2 > 0.0f ? __fmul_rn(r2, rsqrtf(r2)) : 0.0f;
-        // W(q) / sigma, branch-free: 2 (1-q)^3 above q = 1/2, 6q^3 - 6q^2 + 1 below, 0 past 1.
-        const float q = __fmul_rn(r, inv_h);
-        const float t = __fsub_rn(1.0f, q);
-        const float w_out = __fmul_rn(__fmul_rn(__fmul_rn(t, t), t), 2.0f);
-        const float q2 = __fmul_rn(q, q);
-        const float w_in = __fmaf_rn(6.0f, __fmul_rn(q2, q), __fmaf_rn(-6.0f, q2, 1.0f));
-        const float w = q <= 1.0f ? (q > 0.5f ? w_out : w_in) : 0.0f;
-        rho = __fadd_rn(rho, w);
-        if (j != i) {
+        rho = __fadd_rn(rho, in ? w_over_sigma_r2(r2, inv_h) : 0.0f);
+        if (in && j != i) {
             if (listed < cap) {
                 *out = j;
                 out += stride;
@@ -960,132 +821,753 @@ __device__ __forceinline__ void density_finish(const SceneParams& p, uint32_t i,
     bnd[i] = make_float4(bgx, bgy, bgz, bd);
 }
 
-// Block-per-cell staging of the neighbourhood, one warp at a time: when a warp's particles share
-// one row of cells (same scene, same y and z cells, at most four consecutive x cells) and the
-// 3 x 3 rows of cells around them (x from the first cell - 1 to the last + 1) lie in one 50^3 hash
-// block whose keys do not wrap, every row of that union is one run of consecutive keys, hence one
-// contiguous range of the sorted particles, and all of the union's keys are distinct (n > 5110:
-// the union's hashes span at most 5105). The warp then stages each row's particles in shared
-// memory 32 at a time and every lane tests all of them against its particle. Every in-range
-// candidate of a particle lies in its own 27 cells, each of its 27 buckets is met once (distinct
-// keys), and rows and candidates are met in the reference's visiting order, so the in-range
-// sequence and hence the sum are exactly the bucket walk's. Returns false when the warp does not
-// qualify; otherwise the union's first x cell's row keys start at index key_lo of the cell scan
-// (the leader's scene offset included) and each row spans `width` keys. Warp-uniform: every test
-// reads the leader's scene (an idle lane of a batched launch holds a slot of another scene), so
-// all 32 lanes take the same branch and stage the same rows.
-__device__ __forceinline__ bool warp_row_union(const SceneParams& p, bool act, bool ok, uint32_t cx,
-                                               uint32_t cy, uint32_t cz, uint32_t sc,
-                                               uint32_t& key_lo, uint32_t& width) {
-    const uint32_t am = __ballot_sync(0xffffffffu, act);
-    const int leader = __ffs(am) - 1;
-    const uint32_t cy0 = __shfl_sync(0xffffffffu, cy, leader);
-    const uint32_t cz0 = __shfl_sync(0xffffffffu, cz, leader);
-    const uint32_t sc0 = __shfl_sync(0xffffffffu, sc, leader);
-    const uint32_t n0 = __shfl_sync(0xffffffffu, p.n, leader);
-    const uint32_t off0 = __shfl_sync(0xffffffffu, p.off, leader);
-    const unsigned long long magic0 =
-        __shfl_sync(0xffffffffu, (unsigned long long)p.mod_magic, leader);
-    int lo = act ? (int)cx : INT_MAX, hi = act ? (int)cx : INT_MIN;
+// ---- tiles: 32 particles of a few cells against the union of their neighbour cells
+
+// Particles consecutive in sorted order lie in one row of cells, or in a few. A warp's 32
+// particles are split into groups of one row (same scene, same y and z cell, x cells within
+// kTileCells); the group's neighbour cells are rows of x runs (3 x 3 rows for the walk, 5 x 5 for a
+// list build), and when the keys of the union are distinct (checked run against run), every
+// particle of the group meets each of its candidates exactly once among the union's buckets.
+//   Stage: the union's particles are loaded 32 at a time in visiting order, and those within the
+//     radius of the group's bounding box are kept, packed, in shared memory.
+//   Filter: |x_j - x_i|^2 - limit of 32 particles x 128 candidates comes from the tensor cores:
+//     (-2 x_i, 1) . (x_j, |x_j|^2) + (|x_i|^2 - limit) with m16n8k4 TF32 MMAs. Only its sign is
+//     kept, one funnel shift per value, as a bit per (particle, candidate). TF32 rounds to 2^-11
+//     relative. With coordinates from the group's centre, at most M_a for its particles on axis a
+//     and M_a + R for a candidate within the radius R, rounding them moves a pair's distance by at
+//     most e = 2^-11 |2 M + R| and its square by 2 R e + e^2, and rounding |x_j|^2 adds
+//     2^-11 |M + R|^2. The limit is raised by that bound (~0.013 h^2 for a group of four cells, 1.8%
+//     more candidates), so no candidate within the radius is missed; the few beyond it are what a
+//     second, exact test (the walk) or a slightly longer list (the build) is for. Two TF32 terms per
+//     value (m16n8k8) would keep only 0.7% too many, but took the build from 470 to 660 us at 1M.
+//   Each lane then goes through its own particle's bits, in visiting order.
+// What bounds it: issue slots. Per 32 particles with ~500 kept candidates the filter costs ~1.7
+// instructions per candidate, where a thread's own distance test costs ~12 over the ~165
+// candidates left by its pruning. The MMA columns are permuted so that lane (g, q) of a quad holds
+// candidates [32 q, 32 q + 32) of its four rows: whole words in visiting order. Lane 4 g + q owns
+// particle g + 8 q, the row order of the accumulators.
+constexpr int kTileWarps = 4;          // warps per block; a warp works alone
+constexpr int kTileBlocks = 4;         // MMA blocks (128 candidates) of a fill
+constexpr int kTileWordStride = 34;    // staged candidates per word: 32 and 2 of padding (bank conflicts)
+constexpr int kTileMaskStride = 132;   // words per MMA block: 4 rows of 33 (bank conflicts)
+constexpr uint32_t kTileCells = 6;     // x cells of a group
+constexpr int kTileGroups = 8;         // more groups than this in a warp: no tiles
+constexpr float kTileSlack = 0.03f;    // of h: how far a particle may lie outside its cell's place
+
+struct TileSmem {
+    union {
+        struct {
+            float4 cand[kTileBlocks * 4 * kTileWordStride];  // x, y, z, |x - centre|^2 (rounded to TF32)
+            uint32_t id[kTileBlocks * 4 * kTileWordStride];  // sorted index
+            uint32_t mask[kTileBlocks * kTileMaskStride];    // word q' of particle g + 8 p: 33 p + 4 g + q'
+        } t;
+        uint32_t j[kListCap * 32];  // per-thread walk: slot-major candidate lists
+    };
+};
+
+__device__ __forceinline__ float to_tf32(float x) {
+    uint32_t r;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+    return __uint_as_float(r);
+}
+
+__device__ __forceinline__ void mma_m16n8k4(float d[4], float a0, float a1, float b, float c0, float c1) {
+    asm("mma.sync.aligned.m16n8k4.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%8,%8};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(__float_as_uint(b)), "f"(c0), "f"(c1));
+}
+
+__device__ __forceinline__ float warp_min(float x) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+__device__ __forceinline__ float warp_max(float x) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// A fill in progress: `blocks` MMA blocks are done (their masks written), `pending` candidates of
+// the current group are staged behind them.
+struct TileFill {
+    int blocks = 0, pending = 0;
+};
+
+// The group's side of the MMAs: A fragments, accumulator seeds and the centre component of lane
+// (g, q)'s B column.
+struct TileRows {
+    float a[4], c[4], oq;
+};
+
+// Filters the pending candidates: pads them to whole blocks and writes their mask words.
+__device__ __forceinline__ void tile_filter(TileSmem& S, TileFill& f, const TileRows& R) {
+    const uint32_t lane = threadIdx.x & 31u, g = lane >> 2, q = lane & 3u;
+    const int nb = (f.pending + 127) >> 7;
+    float4* cand = S.t.cand + f.blocks * 4 * kTileWordStride;
+    for (int k = f.pending + (int)lane; k < nb * 128; k += 32)
+        cand[k + 2 * (k >> 5)] = make_float4(0.0f, 0.0f, 0.0f, 1.0e30f);
+    __syncwarp();
+    const float* fb = reinterpret_cast<const float*>(cand) + 4u * ((g >> 1) * kTileWordStride + (g & 1u)) + q;
+    uint32_t* mw = S.t.mask + f.blocks * kTileMaskStride + lane;
+    for (int b = 0; b < nb; b++, fb += 16 * kTileWordStride, mw += kTileMaskStride) {
+        uint32_t m[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        for (int k = 0; k < 16; k++) {
+            const float bv = to_tf32(fb[8 * k] - R.oq);
+            float d[4];
+            mma_m16n8k4(d, R.a[0], R.a[1], bv, R.c[0], R.c[1]);
+            m[0] = __funnelshift_l(__float_as_uint(d[0]), m[0], 1);
+            m[0] = __funnelshift_l(__float_as_uint(d[1]), m[0], 1);
+            m[1] = __funnelshift_l(__float_as_uint(d[2]), m[1], 1);
+            m[1] = __funnelshift_l(__float_as_uint(d[3]), m[1], 1);
+            mma_m16n8k4(d, R.a[2], R.a[3], bv, R.c[2], R.c[3]);
+            m[2] = __funnelshift_l(__float_as_uint(d[0]), m[2], 1);
+            m[2] = __funnelshift_l(__float_as_uint(d[1]), m[2], 1);
+            m[3] = __funnelshift_l(__float_as_uint(d[2]), m[3], 1);
+            m[3] = __funnelshift_l(__float_as_uint(d[3]), m[3], 1);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) mw[33 * k] = m[k];
     }
-    const bool same = !act || (ok && cy == cy0 && cz == cz0 && sc == sc0);
-    if (!__all_sync(0xffffffffu, same)) return false;
-    if ((int64_t)hi - (int64_t)lo > 3 || n0 <= 5110u) return false;
-    const uint32_t c0 = (uint32_t)lo - 1u, c1 = (uint32_t)hi + 1u;
-    if ((c0 + 25u) / 50u != (c1 + 25u) / 50u || (cy0 + 24u) / 50u != (cy0 + 26u) / 50u ||
-        (cz0 + 24u) / 50u != (cz0 + 26u) / 50u)
-        return false;
-    const uint32_t h_lo = hash_cell(c0, cy0 - 1u, cz0 - 1u);
-    const uint32_t h_hi = hash_cell(c1, cy0 + 1u, cz0 + 1u);
-    if (h_hi < h_lo) return false;  // the block's hashes wrap past 2^32
-    const uint32_t k_lo = key_mod(h_lo, (uint64_t)magic0, n0);
-    if ((uint64_t)k_lo + (h_hi - h_lo) >= n0) return false;  // keys wrap past n - 1
-    key_lo = off0 + k_lo;
-    width = c1 - c0 + 1u;
+    f.blocks += nb;
+    f.pending = 0;
+}
+
+// The mask words of this lane's particle: word k at [(k >> 2) * kTileMaskStride + (k & 3)].
+__device__ __forceinline__ const uint32_t* tile_masks(const TileSmem& S) {
+    const uint32_t lane = threadIdx.x & 31u;
+    return S.t.mask + 33u * (lane & 3u) + (lane & ~3u);
+}
+
+// Stages and filters one group (mask `grp` of the warp's lanes; cells cx in [c0, c1], cy, cz) of
+// particles at xi against everything within `radius` (radius <= reach h) of them. consume(blocks)
+// is called whenever a fill is full; what is left in `f` at the end is the caller's to consume.
+// Returns false, with nothing staged, when the group does not qualify: its union's keys are not
+// distinct, or a particle lies far outside its cell's place (a saturated cell coordinate). p is the
+// group's scene's; every argument but xi is warp-uniform.
+template <uint32_t kReach, typename Consume>
+__device__ __forceinline__ bool tile_group(TileSmem& S, TileFill& f, uint32_t grp, const SceneParams& p,
+                                           const uint32_t* __restrict__ scan,
+                                           const float4* __restrict__ pos, const float4& xi,
+                                           uint32_t c0, uint32_t c1, uint32_t cy, uint32_t cz,
+                                           float radius2, Consume&& consume) {
+    constexpr uint32_t kSide = 2u * kReach + 1u, kRows = kSide * kSide;
+    const uint32_t lane = threadIdx.x & 31u;
+    const bool mine = (grp >> lane) & 1u;
+    const float h = p.h;
+    // Centre of the group's cells; every particle must be near its cell.
+    const float hw = 0.5f * (float)(c1 - c0 + 1u);
+    const float ox = ((float)(int)c0 + hw) * h;
+    const float oy = ((float)(int)cy + 0.5f) * h, oz = ((float)(int)cz + 0.5f) * h;
+    const float rx = xi.x - ox, ry = xi.y - oy, rz = xi.z - oz;
+    const bool near = fabsf(rx) <= (hw + 0.02f) * h && fabsf(ry) <= 0.52f * h && fabsf(rz) <= 0.52f * h;
+    if (!__all_sync(0xffffffffu, !mine || near)) return false;
+    // Lane r holds row r of the union's cells, in visiting order: one run of keys, or two when it
+    // crosses a 50-cell hash block along x or its keys pass n - 1.
+    const uint32_t xa = c0 - kReach, width = c1 - c0 + 1u + 2u * kReach;
+    const uint32_t block_a = (xa + 25u) / 50u, block_b = (xa + width + 24u) / 50u;
+    uint32_t n_first = width;  // cells of a row in the hash block of its first cell
+    if (block_a != block_b) {
+        n_first = 1u;
+        while ((xa + n_first + 25u) / 50u == block_a) n_first++;
+        if ((xa + n_first + 25u) / 50u != block_b) return false;
+    }
+    const uint32_t row_y = lane % kSide, row_z = lane / kSide;  // cell offsets from -kReach
+    uint32_t k0 = 0u, l0 = 0u, k1 = 0u, l1 = 0u;
+    bool ok = true;
+    if (lane < kRows) {
+        const uint32_t y = cy + row_y - kReach, z = cz + row_z - kReach;
+        const uint32_t hash = hash_cell(xa, y, z);
+        k0 = key_mod(hash, p.mod_magic, p.n);
+        l0 = n_first;
+        ok = hash <= 0xFFFFFFFFu - l0;
+        if (n_first != width) {
+            const uint32_t hash1 = hash_cell(xa + n_first, y, z);
+            k1 = key_mod(hash1, p.mod_magic, p.n);
+            l1 = width - n_first;
+            ok = ok && hash1 <= 0xFFFFFFFFu - l1 && k0 + l0 <= p.n && k1 + l1 <= p.n;
+        } else if (k0 + l0 > p.n) {
+            l1 = k0 + l0 - p.n;  // continues at key 0
+            l0 -= l1;
+            ok = ok && l1 <= p.n;
+        }
+    }
+    const bool two = __any_sync(0xffffffffu, l1 != 0u);
+    // Pairwise disjoint runs modulo n, so every key of the union is met once.
+    auto apart = [&](uint32_t ka, uint32_t la, uint32_t kb, uint32_t lb) {
+        const uint32_t up = kb >= ka ? kb - ka : kb + (p.n - ka), dn = ka >= kb ? ka - kb : ka + (p.n - kb);
+        return la == 0u || lb == 0u || (up >= la && dn >= lb);
+    };
+    if (two) ok = ok && apart(k0, l0, k1, l1);
+    for (uint32_t s = 1u; s <= kRows / 2u; s++) {
+        const int o = (int)((lane + s >= kRows ? lane + s - kRows : lane + s) & 31u);
+        const uint32_t ka = __shfl_sync(0xffffffffu, k0, o), la = __shfl_sync(0xffffffffu, l0, o);
+        bool fine = apart(k0, l0, ka, la);
+        if (two) {
+            const uint32_t kb = __shfl_sync(0xffffffffu, k1, o), lb = __shfl_sync(0xffffffffu, l1, o);
+            fine = fine && apart(k0, l0, kb, lb) && apart(k1, l1, ka, la) && apart(k1, l1, kb, lb);
+        }
+        ok = ok && (lane >= kRows || fine);
+    }
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    // The group's bounding box (from its centre), and how much of each row lies within the radius
+    // of it; a particle may lie kTileSlack h outside its cell's place.
+    const float big = 3.0e38f;
+    const float bx0 = warp_min(mine ? rx : big), bx1 = warp_max(mine ? rx : -big);
+    const float by0 = warp_min(mine ? ry : big), by1 = warp_max(mine ? ry : -big);
+    const float bz0 = warp_min(mine ? rz : big), bz1 = warp_max(mine ? rz : -big);
+    uint32_t b0 = 0u, n0 = 0u, b1 = 0u, n1 = 0u;
+    if (lane < kRows) {
+        const float sy = ((float)row_y - (float)kReach - 0.5f) * h, sz = ((float)row_z - (float)kReach - 0.5f) * h;
+        const float dy = fmaxf(fmaxf(by0 - (sy + h), sy - by1) - kTileSlack * h, 0.0f);
+        const float dz = fmaxf(fmaxf(bz0 - (sz + h), sz - bz1) - kTileSlack * h, 0.0f);
+        const float left = radius2 - dy * dy - dz * dz;
+        if (left >= 0.0f) {
+            const float half = sqrtf(left) + kTileSlack * h;
+            // Cells [ta, tb) of the row, counted from xa.
+            const float fa_ = floorf((bx0 - half) * p.inv_h + hw) + (float)kReach;
+            const float fb_ = floorf((bx1 + half) * p.inv_h + hw) + (float)kReach;
+            const uint32_t ta = (uint32_t)fminf(fmaxf(fa_, 0.0f), (float)width);
+            const uint32_t tb = (uint32_t)fminf(fmaxf(fb_ + 1.0f, 0.0f), (float)width);
+            const uint32_t* sc = scan + p.off;
+            const uint32_t a0 = min(ta, l0), e0 = min(tb, l0);
+            if (a0 < e0) {
+                b0 = __ldg(sc + k0 + a0);
+                n0 = __ldg(sc + k0 + e0) - b0;
+            }
+            const uint32_t a1 = ta > l0 ? ta - l0 : 0u, e1 = tb > l0 ? tb - l0 : 0u;
+            if (a1 < e1 && l1) {
+                b1 = __ldg(sc + k1 + a1);
+                n1 = __ldg(sc + k1 + min(e1, l1)) - b1;
+            }
+        }
+    }
+    // Rows are loaded in words of at most 32 consecutive particles: the words before row r.
+    const uint32_t w0 = (n0 + 31u) >> 5, w_row = w0 + ((n1 + 31u) >> 5);
+    uint32_t first_word = w_row;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, first_word, o);
+        if ((int)lane >= o) first_word += v;
+    }
+    const uint32_t n_words = __shfl_sync(0xffffffffu, first_word, 31);
+    first_word -= w_row;
+    // Rows g, g + 8 of the first MMA and g + 16, g + 24 of the second are particles g + 8 p, owned by
+    // lanes 4 g + p. Lanes outside the group have no candidate.
+    const uint32_t g = lane >> 2, q = lane & 3u;
+    TileRows R;
+    {
+        const float tx = to_tf32(rx), ty = to_tf32(ry), tz = to_tf32(rz);
+        // The filter's error bound (see above), and 5% and 2^-13 R^2 for its own single precision.
+        const float R_ = sqrtf(radius2);
+        const float mx = fmaxf(-bx0, bx1), my = fmaxf(-by0, by1), mz = fmaxf(-bz0, bz1);
+        const float sx = 2.0f * mx + R_, sy = 2.0f * my + R_, sz = 2.0f * mz + R_;
+        const float e = 4.8828125e-4f * sqrtf(fmaf(sx, sx, fmaf(sy, sy, sz * sz)));
+        const float wx = mx + R_, wy = my + R_, wz = mz + R_;
+        const float err = fmaf(e, 2.0f * R_ + e, 4.8828125e-4f * fmaf(wx, wx, fmaf(wy, wy, wz * wz)));
+        const float lim = radius2 * 1.00012207f + 1.05f * err;
+        const float own = mine ? fmaf(tx, tx, fmaf(ty, ty, fmaf(tz, tz, -lim))) : big;
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const int src = (int)(4u * g) + r;
+            const float ax = __shfl_sync(0xffffffffu, tx, src), ay = __shfl_sync(0xffffffffu, ty, src),
+                        az = __shfl_sync(0xffffffffu, tz, src);
+            R.c[r] = __shfl_sync(0xffffffffu, own, src);
+            const float v = q == 0u ? ax : (q == 1u ? ay : az);
+            R.a[r] = q == 3u ? 1.0f : (R.c[r] < big ? -2.0f * v : 0.0f);
+        }
+        R.oq = q == 0u ? ox : (q == 1u ? oy : (q == 2u ? oz : 0.0f));
+    }
+    const float keep2 = 1.001f * radius2;
+    for (uint32_t w32 = 0; w32 < n_words; w32 += 32u) {
+        // Lane l describes word w32 + l: its row is the last one starting at or before it.
+        uint32_t r = 0u;
+#pragma unroll
+        for (uint32_t step = 16u; step >= 1u; step >>= 1) {
+            const uint32_t probe = __shfl_sync(0xffffffffu, first_word, (int)((r + step) & 31u));
+            if (r + step < kRows && probe <= w32 + lane) r += step;
+        }
+        const uint32_t lw = w32 + lane - __shfl_sync(0xffffffffu, first_word, (int)r);
+        const uint32_t rw0 = __shfl_sync(0xffffffffu, w0, (int)r);
+        const uint32_t rb0 = __shfl_sync(0xffffffffu, b0, (int)r), rn0 = __shfl_sync(0xffffffffu, n0, (int)r);
+        const uint32_t rb1 = __shfl_sync(0xffffffffu, b1, (int)r), rn1 = __shfl_sync(0xffffffffu, n1, (int)r);
+        const bool second = lw >= rw0;
+        const uint32_t in_run = 32u * (second ? lw - rw0 : lw);
+        const uint32_t wj = (second ? rb1 : rb0) + in_run;            // its first particle
+        const uint32_t run_n = second ? rn1 : rn0;
+        const uint32_t wn = w32 + lane < n_words && run_n > in_run ? run_n - in_run : 0u;  // and how many (or more than 31)
+        const uint32_t here = min(32u, n_words - w32);
+        for (uint32_t v = 0; v < here; v += 4u) {
+            float4 x[4];
+            uint32_t j[4];
+            bool in[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                j[u] = __shfl_sync(0xffffffffu, wj, (int)(v + u)) + lane;
+                in[u] = lane < __shfl_sync(0xffffffffu, wn, (int)(v + u));
+                x[u] = in[u] ? __ldg(pos + j[u]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const float ux = x[u].x - ox, uy = x[u].y - oy, uz = x[u].z - oz;
+                const float ex = fmaxf(fmaxf(bx0 - ux, ux - bx1), 0.0f), ey = fmaxf(fmaxf(by0 - uy, uy - by1), 0.0f),
+                            ez = fmaxf(fmaxf(bz0 - uz, uz - bz1), 0.0f);
+                in[u] = in[u] && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= keep2;
+                const uint32_t kept = __ballot_sync(0xffffffffu, in[u]);
+                const int n_kept = __popc(kept);
+                if (128 * f.blocks + f.pending + n_kept > 128 * kTileBlocks) {
+                    tile_filter(S, f, R);
+                    consume(f.blocks);
+                    f.blocks = 0;
+                }
+                if (in[u]) {
+                    const int k = 128 * f.blocks + f.pending + __popc(kept & ((1u << lane) - 1u));
+                    const float tx = to_tf32(ux), ty = to_tf32(uy), tz = to_tf32(uz);
+                    x[u].w = to_tf32(fmaf(tx, tx, fmaf(ty, ty, tz * tz)));
+                    S.t.cand[k + 2 * (k >> 5)] = x[u];
+                    S.t.id[k + 2 * (k >> 5)] = j[u];
+                }
+                f.pending += n_kept;
+            }
+        }
+    }
+    tile_filter(S, f, R);
     return true;
 }
 
+// The groups of a warp's particles (lanes in `todo`, at cells cx, cy, cz of scene sc): calls
+// group(mask of its lanes, leader lane, lowest and highest x cell) for each, one row of cells from
+// its lowest x cell up. Returns false, with nothing called, when there are more than kTileGroups
+// (sparse or scattered particles).
+template <typename Group>
+__device__ __forceinline__ bool for_each_tile_group(uint32_t todo, uint32_t cx, uint32_t cy, uint32_t cz,
+                                                    uint32_t sc, Group&& group) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (int pass = 0; pass < 2; pass++) {
+        int k = 0;
+        for (uint32_t left = todo; left; k++) {
+            if (k == kTileGroups) return false;  // in the counting pass
+            const int lead = __ffs((int)left) - 1;
+            const uint32_t ly = __shfl_sync(0xffffffffu, cy, lead), lz = __shfl_sync(0xffffffffu, cz, lead);
+            const uint32_t ls = __shfl_sync(0xffffffffu, sc, lead);
+            const bool row = ((left >> lane) & 1u) && cy == ly && cz == lz && sc == ls;
+            // Lowest cell of the row (as signed cells) and the lanes within kTileCells of it.
+            const int lo = __reduce_min_sync(0xffffffffu, row ? (int)cx : INT_MAX);
+            const bool in = row && cx - (uint32_t)lo < kTileCells;
+            const uint32_t grp = __ballot_sync(0xffffffffu, in);
+            left &= ~grp;
+            if (pass == 0) continue;
+            const int hi = __reduce_max_sync(0xffffffffu, in ? (int)cx : INT_MIN);
+            group(grp, lead, (uint32_t)lo, (uint32_t)hi, ly, lz);
+        }
+    }
+    return true;
+}
+
+// The per-thread state of a density walk: particle i at xi, its sum and list so far.
+struct WalkState {
+    uint32_t i;
+    float4 xi;
+    DensitySum d;
+};
+
+// The walk's sums over the filled blocks: every lane goes through its mask words in order and
+// tests, sums and lists the candidates with in_range2 and DensitySum, as the per-thread walk does:
+// the same in-range candidates in the same order, so the densities and lists are the same bit
+// for bit. The next candidate's load runs ahead of the current one's arithmetic.
+__device__ __forceinline__ void tile_sum(const TileSmem& S, int blocks, const SceneParams& p,
+                                         uint32_t total, WalkState& w) {
+    __syncwarp();
+    const uint32_t* m = tile_masks(S);
+    const float h2 = p.h2, inv_h = p.inv_h;
+    const uint32_t nbr_cap = p.nbr_cap;
+    uint32_t nz = 0u;  // words with a bit set, first word highest
+    for (int k = 0; k < 4 * blocks; k += 4) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) nz |= m[33 * k + u] ? 0x80000000u >> (k + u) : 0u;
+    }
+    uint32_t bits = 0u, at = 0u, j = 0u;
+    float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    auto next = [&]() {
+        if (!bits) {
+            if (!nz) return false;
+            const uint32_t k = (uint32_t)__clz((int)nz);
+            nz ^= 0x80000000u >> k;
+            bits = m[(k >> 2) * kTileMaskStride + (k & 3u)];
+            at = k * kTileWordStride;
+        }
+        const uint32_t b = (uint32_t)__clz((int)bits);
+        bits ^= 0x80000000u >> b;
+        x = S.t.cand[at + b];
+        j = S.t.id[at + b];
+        return true;
+    };
+    bool more = next();
+    while (more) {
+        const float r2 = in_range2(w.xi, x);
+        const uint32_t cj = j;
+        more = next();
+        w.d.add_r2(w.i, cj, r2, r2 <= h2, inv_h, nbr_cap, total);
+    }
+    __syncwarp();
+}
+static_assert(kTileMaskStride == 33 * 4, "tile_sum steps 33 words per mask word of a block");
+
+// The lists of the last build are summed this substep (a scene that is stale and may rebuild has
+// just rebuilt them).
+__device__ __forceinline__ bool lists_in_use(const SkinLists& sk, uint32_t sc) {
+    return sk.stale[sc] ? sk.ctl[sc * kSkinCtl + kCtlAllow] != 0u : true;
+}
+
+// The same for a single scene's passes, where a scene whose last build left most lists unusable is
+// walked in index order until its next build.
+__device__ __forceinline__ bool sums_lists(const SkinLists& sk) {
+    return sk.stale[0] ? sk.ctl[kCtlAllow] != 0u : sk.ctl[kCtlPoor] == 0u;
+}
+
+// The list build: for every particle of a scene that is stale and may rebuild, the candidates
+// within h (1 + skin) (and a few just beyond: the filter's margin), in visiting order, under its
+// sorted index of this substep, which becomes its build index; its position; and its current
+// position and sorted index for the list pass of this substep. A particle whose group is no tile
+// or that has more than sk.cap candidates gets no usable list. Other scenes are left alone, and
+// the launch returns at its top when no build is due.
+template <bool kBatch>
+__global__ void __launch_bounds__(kTileWarps * 32, 4)
+    k_skin_build(StepLaunch L, const float4* __restrict__ pos, const uint32_t* __restrict__ scan, SkinLists sk) {
+    static_assert(kSkinCap * 32 * sizeof(uint16_t) <= sizeof(float4) * kTileBlocks * 4 * kTileWordStride,
+                  "the lists of a fill take the staged positions' place");
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    TileSmem& S = reinterpret_cast<TileSmem*>(s_raw)[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t slot_of = (lane >> 2) + 8u * (lane & 3u);  // lane 4 g + q owns slot g + 8 q of a run
+    if (sk.wcount[1] == 0u) return;  // no scene's build is due
+    const uint32_t runs = (L.total + 31u) / 32u;
+    for (uint32_t run = blockIdx.x * (uint32_t)kTileWarps + (threadIdx.x >> 5); run < runs;
+         run += gridDim.x * (uint32_t)kTileWarps) {
+        const uint32_t i = min(run * 32u + slot_of, L.total - 1u);
+        bool act = run * 32u + slot_of < L.total;
+        const uint32_t sc = kBatch ? (uint32_t)__ldg(L.scene_of + i) : 0u;
+        if (kBatch) act = act && sk.stale[sc] != 0u && sk.ctl[sc * kSkinCtl + kCtlAllow] != 0u;
+        const uint32_t todo = __ballot_sync(0xffffffffu, act);
+        if (todo == 0u) continue;
+        const SceneParams& p = scene_params<kBatch>(L, i);
+        const float4 xi = __ldg(pos + i);
+        const uint32_t cx = cell_coord(xi.x, p.h), cy = cell_coord(xi.y, p.h), cz = cell_coord(xi.z, p.h);
+        uint32_t c = 0u;  // candidates listed so far
+        TileFill f;
+        uint32_t refused = 0u;
+        auto list = [&](int blocks) {
+            __syncwarp();
+            const uint32_t* m = tile_masks(S);
+            uint16_t* at = reinterpret_cast<uint16_t*>(S.t.cand) + lane;  // slot-major, 32 lanes a slot
+            uint32_t n = 0u;
+            for (int k = 0; k < 4 * blocks; k++) {
+                uint32_t bits = m[(k >> 2) * kTileMaskStride + (k & 3)];
+                while (bits) {
+                    const uint32_t b = (uint32_t)__clz((int)bits);
+                    bits ^= 0x80000000u >> b;
+                    if (n < kSkinCap) at[32u * n] = (uint16_t)(k * kTileWordStride + (int)b);
+                    n++;
+                }
+            }
+            // A slot at a time, so that a warp's lanes store nearby words.
+            const uint32_t room = c < kSkinCap ? kSkinCap - c : 0u, stored = min(n, room);
+            uint32_t* out = sk.list + (size_t)c * L.total + i;
+            for (uint32_t k = 0; k < stored; k++, out += L.total) *out = S.t.id[at[32u * k]];
+            c += n;
+            __syncwarp();
+        };
+        if (for_each_tile_group(todo, cx, cy, cz, sc, [&](uint32_t grp, int lead, uint32_t lo, uint32_t hi,
+                                                          uint32_t ly, uint32_t lz) {
+                const uint32_t li = __shfl_sync(0xffffffffu, i, lead);
+                const SceneParams& pl = scene_params<kBatch>(L, li);
+                if (!tile_group<2>(S, f, grp, pl, scan, pos, xi, lo, hi, ly, lz, pl.skin_r2, list)) refused |= grp;
+            })) {
+            if (f.blocks) list(f.blocks);
+        } else {
+            refused = todo;
+        }
+        if (act) {
+            const bool usable = !((refused >> lane) & 1u) && c <= kSkinCap;
+            sk.x_build[i] = xi;
+            sk.b_of_id[__float_as_uint(xi.w)] = i;
+            sk.xcur[i] = make_float4(xi.x, xi.y, xi.z, __uint_as_float(i));
+            sk.count[i] = usable ? c | kSkinUsable : 0u;
+            // The scene's usable lists, one atomic per warp and scene.
+            const uint32_t gm = __match_any_sync(__activemask(), sc);
+            const uint32_t u = __ballot_sync(gm, usable);
+            if (lane == (uint32_t)(__ffs((int)gm) - 1) && u)
+                atomicAdd(sk.ctl + sc * kSkinCtl + kCtlUsable, (uint32_t)__popc(u));
+        }
+        __syncwarp();
+    }
+}
+
+// The walk of one particle by a whole warp (a single scene's few particles without a usable list),
+// so that its ~280 candidates are tested 32 at a time instead of in one thread's chain of dependent
+// loads. Lane r < 27 holds candidate segment r of the walk (row r / 3, part r % 3 of the rows of
+// for_each_candidate: the same buckets, the same pruning), the segments' candidates are numbered in
+// visiting order and taken in chunks of 32, and the in-range ones are summed in visiting order
+// (every lane adds them one by one through shuffles) and listed in visiting order: exactly the sum
+// and the list of the per-thread walk.
+__device__ __forceinline__ void walk_by_warp(const SceneParams& p, uint32_t i, uint32_t total_n,
+                                             const float4* __restrict__ pos, const float4* __restrict__ vel,
+                                             float4* __restrict__ rec, const uint32_t* __restrict__ scan,
+                                             float4* __restrict__ aux, float4* __restrict__ bnd,
+                                             uint32_t* __restrict__ nbr, uint32_t* __restrict__ nbr_count,
+                                             float* __restrict__ host_dens, bool defer_vel) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t* sc = scan + p.off;
+    const float4 xi = __ldg(pos + i);
+    const uint32_t cx = cell_coord(xi.x, p.h), cy = cell_coord(xi.y, p.h),
+                   cz = cell_coord(xi.z, p.h);
+    const bool distinct = distinct_keys(p, cx, cy, cz);
+    // Segment r of the walk: [b, b + len).
+    uint32_t b = 0u, len = 0u;
+    if (lane < 27) {
+        const float lim = distinct ? kPruneLimit : 1e30f;
+        const float fx = fmaf(-(float)(int)cx, p.h, xi.x) * p.inv_h;
+        const float fy = fmaf(-(float)(int)cy, p.h, xi.y) * p.inv_h;
+        const float fz = fmaf(-(float)(int)cz, p.h, xi.z) * p.inv_h;
+        const int t = lane / 3, part = lane % 3;
+        const uint32_t dy = (uint32_t)(t % 3) - 1u, dz = (uint32_t)(t / 3) - 1u;
+        const float dyz = face_dist2(dy, fy) + face_dist2(dz, fz);
+        if (dyz <= lim) {
+            const bool skip_l = dyz + face_dist2(0xFFFFFFFFu, fx) > lim;
+            const bool skip_r = dyz + face_dist2(1u, fx) > lim;
+            const uint32_t ry = cy + dy, rz = cz + dz;
+            const uint32_t hA = hash_cell(cx - 1u, ry, rz);
+            const uint32_t kA = key_mod(hA, p.mod_magic, p.n);
+            const bool same_block = (cx + 24u) / 50u == (cx + 26u) / 50u && hA <= 0xFFFFFFFDu;
+            uint32_t e = 0u;
+            if (same_block && kA + 2u < p.n) {
+                if (part == 0) {
+                    b = __ldg(sc + kA + (skip_l ? 1u : 0u));
+                    e = __ldg(sc + kA + (skip_r ? 2u : 3u));
+                }
+            } else if (part == 0) {
+                b = __ldg(sc + kA);
+                e = skip_l ? b : __ldg(sc + kA + 1u);
+            } else if (part == 1) {
+                const uint32_t kB = key_mod(hash_cell(cx, ry, rz), p.mod_magic, p.n);
+                b = __ldg(sc + kB);
+                e = __ldg(sc + kB + 1u);
+            } else if (!skip_r) {
+                const uint32_t kC = key_mod(hash_cell(cx + 1u, ry, rz), p.mod_magic, p.n);
+                b = __ldg(sc + kC);
+                e = __ldg(sc + kC + 1u);
+            }
+            len = e > b ? e - b : 0u;
+        }
+    }
+    // Exclusive prefix of the segment lengths: the visiting-order number of each segment's
+    // first candidate.
+    uint32_t incl = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    const uint32_t start = incl - len;
+    float rho = 0.0f;
+    uint32_t listed = 0u;
+    for (uint32_t base = 0; base < total; base += 32u) {
+        const uint32_t f = base + (uint32_t)lane;
+        // The segment holding candidate f: the last one starting at or before f.
+        int r = 0;
+#pragma unroll
+        for (int step = 16; step >= 1; step >>= 1) {
+            const uint32_t s_probe = __shfl_sync(0xffffffffu, start, (r + step) & 31);
+            if (r + step < 27 && s_probe <= f) r += step;
+        }
+        const uint32_t rb = __shfl_sync(0xffffffffu, b, r);
+        const uint32_t rs = __shfl_sync(0xffffffffu, start, r);
+        const bool valid = f < total;
+        const uint32_t j = rb + (f - rs);
+        float4 xj = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (valid) xj = __ldg(pos + j);
+        const float r2 = in_range2(xi, xj);
+        const bool inr = valid && r2 <= p.h2;
+        const float wv = inr ? w_over_sigma_r2(r2, p.inv_h) : 0.0f;
+        uint32_t mask = __ballot_sync(0xffffffffu, inr);
+        const uint32_t listm = __ballot_sync(0xffffffffu, inr && j != i);
+        if (inr && j != i) {
+            const uint32_t slot = listed + (uint32_t)__popc(listm & lt);
+            if (slot < p.nbr_cap) nbr[(size_t)slot * total_n + i] = j;
+        }
+        listed += (uint32_t)__popc(listm);
+        while (mask) {
+            const int l = __ffs(mask) - 1;
+            rho = __fadd_rn(rho, __shfl_sync(0xffffffffu, wv, l));
+            mask &= mask - 1u;
+        }
+    }
+    if (lane == 0) {
+        DensitySum d;
+        d.rho = rho;
+        d.listed = listed;
+        density_finish(p, i, xi, vel, cx, cy, cz, distinct, d, rec, aux, bnd, nbr_count, host_dens,
+                   defer_vel);
+    }
+}
+
+// The walk of the particles k_density_list queued in a single scene (no usable list this substep): a
+// crowd (kWalkerCrowd) in runs of 32, a smaller queue a warp per particle (walk_by_warp). One
+// resident wave whose warps claim the runs. A warp walks its particles as tiles (tile_group) where they qualify and per
+// thread (for_each_candidate) where not. In a crowd dense enough to overflow the skin lists the
+// tiles pay most: the filter's cost per candidate is a seventh of a thread's own test (419,000
+// particles with ~900 neighbours each: 3.1 ms against 7.5 ms a warp per particle and 8.7 ms a thread
+// per particle).
+__global__ void __launch_bounds__(kTileWarps * 32, 5)
+    k_walk_queue(StepLaunch L, const float4* __restrict__ pos, const float4* __restrict__ vel,
+                 float4* __restrict__ rec, const uint32_t* __restrict__ scan,
+                 float4* __restrict__ aux, float4* __restrict__ bnd, uint32_t* __restrict__ nbr,
+                 uint32_t* __restrict__ nbr_count, SkinLists sk, uint32_t* __restrict__ sched, bool tiles) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    TileSmem& S = reinterpret_cast<TileSmem*>(s_raw)[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t slot_of = (lane >> 2) + 8u * (lane & 3u);  // lane 4 g + q owns slot g + 8 q of a run
+    if (!sums_lists(sk)) return;  // k_walk walks every particle
+    const SceneParams& p = L.one;
+    const uint32_t slots = min(*sk.wcount, L.total);
+    if (slots < kWalkerCrowd || !tiles) {
+        for (uint32_t k = blockIdx.x * (uint32_t)kTileWarps + (threadIdx.x >> 5); k < slots;
+             k += gridDim.x * (uint32_t)kTileWarps)
+            walk_by_warp(p, __ldg(sk.queue + k), L.total, pos, vel, rec, scan, aux, bnd, nbr, nbr_count,
+                         L.host_dens, L.defer_vel);
+        return;
+    }
+    // Every warp takes runs of 32 slots: first the run of its own index, then runs claimed from
+    // the launch's counter (sched[0]), until none is left. Walks differ widely in length (dense and
+    // sparse regions), and a warp that finishes early takes the next run. No lane leaves a run
+    // before the warp's collective steps: inactive lanes carry act = false.
+    const uint32_t runs = (slots + 31u) / 32u;
+    const uint32_t warps = gridDim.x * (uint32_t)kTileWarps;
+    uint32_t run = blockIdx.x * (uint32_t)kTileWarps + (threadIdx.x >> 5);
+    for (; run < runs;) {
+        const uint32_t t = run * 32u + slot_of;
+        const bool act = t < slots;
+        WalkState w{};
+        w.i = act ? __ldg(sk.queue + t) : 0u;
+        // The next run, claimed now so that the counter's latency hides behind this one.
+        uint32_t next = 0u;
+        if (lane == 0u) next = warps + atomicAdd(sched, 1u);
+        next = __shfl_sync(0xffffffffu, next, 0);
+        const uint32_t todo = __ballot_sync(0xffffffffu, act);
+        w.xi = act ? __ldg(pos + w.i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        w.d.out = nbr + w.i;
+        const uint32_t cx = cell_coord(w.xi.x, p.h), cy = cell_coord(w.xi.y, p.h), cz = cell_coord(w.xi.z, p.h);
+        uint32_t single = 0u;  // lanes that walk per thread
+        TileFill f;
+        auto sum = [&](int blocks) { tile_sum(S, blocks, p, L.total, w); };
+        if (for_each_tile_group(todo, cx, cy, cz, 0u, [&](uint32_t grp, int, uint32_t lo, uint32_t hi,
+                                                                   uint32_t ly, uint32_t lz) {
+                if (!tile_group<1>(S, f, grp, p, scan, pos, w.xi, lo, hi, ly, lz, p.h2, sum)) single |= grp;
+            })) {
+            if (f.blocks) sum(f.blocks);
+        } else {
+            single = todo;
+        }
+        if ((single >> lane) & 1u) {
+            // The per-thread walk. Scene constants used per candidate, in registers.
+            const float s_inv_h = p.inv_h, h2 = p.h2;
+            const uint32_t s_nbr_cap = p.nbr_cap;
+            uint32_t s_end = lane;  // word one past the last kept candidate (stride 32)
+            auto drain = [&]() {
+#pragma unroll 2
+                for (uint32_t o = lane; o < s_end; o += 32u) {
+                    const uint32_t j = S.j[o];
+                    w.d.add(w.i, w.xi, j, __ldg(pos + j), s_inv_h, s_nbr_cap, L.total);
+                }
+                s_end = lane;
+            };
+            // Branch-free append: every candidate is stored at the list's end and kept only when
+            // in range (the next one overwrites it otherwise). Lists are drained above kDrainAt,
+            // so the slot index stays below kListCap.
+            for_each_candidate(p, scan, pos, w.xi, cx, cy, cz, [&](uint32_t j, const float4& xj) {
+                S.j[s_end] = j;
+                s_end += in_range2(w.xi, xj) <= h2 ? 32u : 0u;
+            }, [&]() {
+                if (s_end > lane + kDrainAt * 32u) drain();
+            });
+            drain();
+        }
+        run = next;
+        if (act)
+            density_finish(p, w.i, w.xi, vel, cx, cy, cz, distinct_keys(p, cx, cy, cz), w.d, rec, aux, bnd,
+                           nbr_count, L.host_dens, L.defer_vel);
+        __syncwarp();
+    }
+    // The last warp out puts the counter back to zero for the next launch (every other warp has
+    // made its last claim before it counts itself out).
+    if (lane == 0u) {
+        __threadfence();
+        if (atomicAdd(sched + 1, 1u) == warps - 1u) {
+            atomicExch(sched, 0u);
+            atomicExch(sched + 1, 0u);
+        }
+    }
+}
+
 // CalculateBoundaryVolume + CalculateDensities + the per-particle part of PressureFromDensityEOS
-// (wcsph_with_boundary_model.slang:102-203), by the bucket walk. Besides the density products it
-// writes particle i's neighbour list: every in-range j except i itself, in visiting order,
-// slot-major (nbr[s * n + i], so a warp's lanes store and later load consecutive words), and its
-// length in nbr_count[i] (a length above nbr_cap means the list overflowed and was truncated).
-// Positions do not change before the force pass, so that list is exactly the force pass's
-// neighbour set. Without skin lists every particle is walked, one per thread. With them, a
-// batch's walkers are the queue k_density_list leaves (each list block's walkers in index order,
-// so a stale scene is walked in index order); a single scene is walked here only when it is stale
-// or its lists are mostly unusable (in index order; otherwise k_density_walkers takes its few
-// walkers and this launch returns at its top). In a stale scene whose build policy allows it,
-// every particle also builds its skin list. The launch is one resident wave whose warps claim
-// runs of 32 slots. A warp whose particles share a row of cells walks the staged rows of
-// warp_row_union; any other warp walks per thread (for_each_candidate).
-template <bool kBatch, int kNbrBlock, int kMinBlocks, bool kStaging>
+// (wcsph_with_boundary_model.slang:102-203), by a walk of the neighbour cells, one thread per
+// particle. Besides the density products it writes particle i's neighbour list: every in-range j
+// except i itself, in visiting order, slot-major (nbr[s * n + i], so a warp's lanes store and later
+// load consecutive words), and its length in nbr_count[i] (a length above nbr_cap means the list
+// overflowed and was truncated). Positions do not change before the force pass, so that list is
+// exactly the force pass's neighbour set. It walks whole scenes in index order (no skin lists; a
+// single scene that is stale and may not rebuild, or whose lists are mostly unusable) and a batch's
+// queue. A single scene whose lists are summed returns at the kernel's top. One
+// resident wave whose warps claim runs of 32 slots. The tiles above are no faster for a fluid's ~43
+// neighbours: 515 us against 450 us for 1M particles (their sum phase runs at 16 warps per SM, this
+// kernel at 24, and it tests only ~200 candidates per particle after pruning).
+template <bool kBatch, int kNbrBlock, int kMinBlocks>
 __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
-    k_density(StepLaunch L, const float4* __restrict__ pos, const float4* __restrict__ vel,
-              float4* __restrict__ rec, const uint32_t* __restrict__ scan,
-              float4* __restrict__ aux, float4* __restrict__ bnd, uint32_t* __restrict__ nbr,
-              uint32_t* __restrict__ nbr_count, SkinLists sk, uint32_t* __restrict__ sched) {
-    static_assert(kSkinCap <= (uint32_t)kListCap, "a list build is staged in the shared list");
+    k_walk(StepLaunch L, const float4* __restrict__ pos, const float4* __restrict__ vel,
+           float4* __restrict__ rec, const uint32_t* __restrict__ scan,
+           float4* __restrict__ aux, float4* __restrict__ bnd, uint32_t* __restrict__ nbr,
+           uint32_t* __restrict__ nbr_count, SkinLists sk, uint32_t* __restrict__ sched) {
     static_assert(kNbrBlock % 32 == 0, "whole warps");
-    static_assert(kListBlock % 32 == 0, "a warp's 32 slots lie in one list block");
     __shared__ uint32_t s_j[kListCap * kNbrBlock];
-    // Each warp's 32 staged candidates (one placeholder element without staging, so that the
-    // shared memory the per-thread walk does not use stays L1 for its candidate loads).
-    __shared__ float4 s_stage[kStaging ? kNbrBlock : 1];
     const int tid = threadIdx.x;
     const uint32_t lane = (uint32_t)(tid & 31);
-    // A single scene whose lists are current and mostly usable: k_density_list and
-    // k_density_walkers cover every particle, and the whole launch returns here.
-    if (!kBatch && sk.list && sk.stale[0] == 0u && sk.ctl[kCtlPoor] == 0u) return;
+    if (!kBatch && sk.list && sums_lists(sk)) return;
     // Every warp takes runs of 32 slots: first the run of its own index, then runs claimed from
     // the launch's counter (sched[0]), until none is left. Walks differ widely in length (the
-    // queued walkers of a batch, the list builds of a stale scene), and a warp that finishes early
-    // takes the next run. No lane leaves a run before the warp's collective steps: inactive lanes
-    // carry act = false.
+    // queued walkers of a batch, dense and sparse regions), and a warp that finishes early takes
+    // the next run.
     const uint32_t runs = (L.total + 31u) / 32u;
     const uint32_t warps = gridDim.x * (uint32_t)(kNbrBlock / 32);
     uint32_t run = blockIdx.x * (uint32_t)(kNbrBlock / 32) + (uint32_t)(tid >> 5);
     for (; run < runs;) {
         const uint32_t t = run * 32u + lane;
         bool act = t < L.total;
-        uint32_t i = act ? t : 0u, sc = 0u;
-        bool rebuild = false;
-        if (act && sk.list) {
-            if (kBatch) {
-                // Slot t of the queue: valid below its list block's count of walkers.
-                if (t % kListBlock >= __ldg(sk.seg_n + t / kListBlock)) {
-                    act = false;
-                } else {
-                    i = __ldg(sk.queue + t);
-                    sc = (uint32_t)__ldg(L.scene_of + i);
-                }
-            } else if (sk.stale[0] == 0u && sk.ctl[kCtlPoor] == 0u) {
-                act = false;  // k_density_walkers walks the single scene's queued particles
-            }  // else a single scene that is stale or whose lists are mostly unusable: every
-               // particle, in index order (no queue)
-            rebuild = act && sk.stale[sc] != 0u && sk.ctl[sc * kSkinCtl + kCtlAllow] != 0u;
+        uint32_t i = act ? t : 0u;
+        if (kBatch && act && sk.list) {
+            // Slot t of the queue: valid below its list block's count of walkers.
+            if (t % kListBlock >= __ldg(sk.seg_n + t / kListBlock))
+                act = false;
+            else
+                i = __ldg(sk.queue + t);
         }
         // The next run, claimed now so that the counter's latency hides behind this one.
         uint32_t next = 0u;
         if (lane == 0u) next = warps + atomicAdd(sched, 1u);
-        next = __shfl_sync(0xffffffffu, next, 0);
-        if (__ballot_sync(0xffffffffu, act) == 0u) {  // the whole warp is idle
-            run = next;
-            continue;
-        }
+        run = __shfl_sync(0xffffffffu, next, 0);
+        if (!act) continue;
         const SceneParams& p = scene_params<kBatch>(L, i);
-        const float4 xi = act ? __ldg(pos + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 xi = __ldg(pos + i);
         const uint32_t cx = cell_coord(xi.x, p.h), cy = cell_coord(xi.y, p.h), cz = cell_coord(xi.z, p.h);
         DensitySum d;
         d.out = nbr + i;
         uint32_t s_end = tid;  // shared-memory word one past the last kept candidate (stride kNbrBlock)
         // Scene constants used per candidate, in registers (a batched launch reads its scene's
         // parameters from a device table).
-        const float s_inv_h = p.inv_h;
+        const float s_inv_h = p.inv_h, h2 = p.h2;
         const uint32_t s_nbr_cap = p.nbr_cap;
         auto drain = [&]() {
 #pragma unroll 2
@@ -1095,82 +1577,18 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
             }
             s_end = tid;
         };
-        const bool distinct = distinct_keys(p, cx, cy, cz);
-        const float h2 = p.h2;
-        uint32_t c = 0;
-        bool usable = false;
-        uint32_t key_lo = 0u, width = 0u;
-        if (kStaging && warp_row_union(p, act, !rebuild, cx, cy, cz, sc, key_lo, width)) {
-            // The staged walk: branch-free append as below, candidates read from shared memory.
-            // key_lo indexes the cell scan directly (the warp's scene offset included).
-            float4* stage = s_stage + (tid & ~31);
-#pragma unroll 1
-            for (uint32_t r = 0; r < 9u; r++) {
-                const uint32_t kA = key_lo + 50u * (r % 3u) + 2500u * (r / 3u);
-                const uint32_t b = __ldg(scan + kA), e = __ldg(scan + kA + width);
-#pragma unroll 1
-                for (uint32_t jb = b; jb < e; jb += 32u) {
-                    const uint32_t jl = jb + lane;
-                    if (jl < e) stage[lane] = __ldg(pos + jl);
-                    __syncwarp();
-                    const uint32_t cnt = min(32u, e - jb);
-#pragma unroll 4
-                    for (uint32_t k = 0; k < cnt; k++) {
-                        const float4 xj = stage[k];
-                        s_j[s_end] = jb + k;
-                        s_end += act && in_range2(xi, xj) <= h2 ? kNbrBlock : 0u;
-                        if ((k & 3u) == 3u && s_end > tid + kDrainAt * kNbrBlock) drain();
-                    }
-                    if (s_end > tid + kDrainAt * kNbrBlock) drain();
-                    __syncwarp();  // the next chunk overwrites the stage
-                }
-            }
-            drain();
-        } else if (act) {
-            if (rebuild && skin_keys_distinct(p, cx, cy, cz)) {
-                // A list build, staged in this thread's column of the shared list.
-                c = skin_walk(p, scan, pos, xi, cx, cy, cz, s_j + tid, (size_t)kNbrBlock, sk.cap);
-                usable = c <= sk.cap;
-            }
-            if (usable) {
-                // The density from the staged list (its in-range members, in the visiting order),
-                // then the list written out a slot at a time (a warp's lanes store consecutive words).
-#pragma unroll 1
-                for (uint32_t k = 0; k < c; k++) {
-                    const uint32_t j = s_j[k * kNbrBlock + tid];
-                    const float r2 = in_range2(xi, __ldg(pos + j));
-                    if (r2 <= h2) d.add_r2(i, j, r2, s_inv_h, s_nbr_cap, L.total);
-                }
-#pragma unroll 1
-                for (uint32_t k = 0; k < c; k++) sk.list[(size_t)k * L.total + i] = s_j[k * kNbrBlock + tid];
-            } else {
-                // Branch-free append: every candidate is stored at the list's end and kept only when
-                // in range (the next one overwrites it otherwise). Lists are drained above kDrainAt,
-                // so the slot index stays below kListCap.
-                for_each_candidate(p, scan, pos, xi, cx, cy, cz, [&](uint32_t j, const float4& xj) {
-                    s_j[s_end] = j;
-                    s_end += in_range2(xi, xj) <= h2 ? kNbrBlock : 0u;
-                }, [&]() {
-                    if (s_end > tid + kDrainAt * kNbrBlock) drain();
-                });
-                drain();
-            }
-        }
-        run = next;
-        if (!act) continue;
-        if (rebuild) {
-            // This substep's sorted index becomes the particle's build index.
-            sk.x_build[i] = xi;
-            sk.b_of_id[__float_as_uint(xi.w)] = i;
-            sk.count[i] = min(c, sk.cap) | (usable ? kSkinUsable : 0u);
-            // The scene's usable lists, one atomic per warp and scene.
-            const uint32_t g = __match_any_sync(__activemask(), sc);
-            const uint32_t u = __ballot_sync(g, usable);
-            if ((uint32_t)(tid & 31) == (uint32_t)(__ffs(g) - 1) && u)
-                atomicAdd(sk.ctl + sc * kSkinCtl + kCtlUsable, (uint32_t)__popc(u));
-        }
-        density_finish(p, i, xi, vel, cx, cy, cz, distinct, d, rec, aux, bnd, nbr_count, L.host_dens,
-                       L.defer_vel);
+        // Branch-free append: every candidate is stored at the list's end and kept only when in
+        // range (the next one overwrites it otherwise). Lists are drained above kDrainAt, so the
+        // slot index stays below kListCap.
+        for_each_candidate(p, scan, pos, xi, cx, cy, cz, [&](uint32_t j, const float4& xj) {
+            s_j[s_end] = j;
+            s_end += in_range2(xi, xj) <= h2 ? kNbrBlock : 0u;
+        }, [&]() {
+            if (s_end > tid + kDrainAt * kNbrBlock) drain();
+        });
+        drain();
+        density_finish(p, i, xi, vel, cx, cy, cz, distinct_keys(p, cx, cy, cz), d, rec, aux, bnd, nbr_count,
+                       L.host_dens, L.defer_vel);
     }
     // The last warp out puts the counter back to zero for the next launch (every other warp has
     // made its last claim before it counts itself out).
@@ -1187,7 +1605,8 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
 // usable, sums the in-range members of its list (the same in-range set as the walk: every
 // pair within h was within h (1 + skin) at the build; each once: the particle has moved less than
 // h / 4 since the build, so its 27 cells lie in the build's 5x5x5 block, whose keys were
-// distinct), in the list's order. Every other particle goes to the queue for k_density.
+// distinct), in the list's order. Every other particle goes to the queue for k_walk_queue (a
+// batch's: k_walk).
 // No shared memory: the pass is bound by its chains of dependent loads, so it runs at the
 // occupancy its registers allow.
 template <bool kBatch>
@@ -1196,18 +1615,20 @@ __global__ void __launch_bounds__(kListBlock, 10)
                    float4* __restrict__ rec, float4* __restrict__ aux, float4* __restrict__ bnd,
                    uint32_t* __restrict__ nbr, uint32_t* __restrict__ nbr_count, SkinLists sk) {
     const uint32_t i = blockIdx.x * kListBlock + threadIdx.x;
-    // A single scene that is stale, or whose last build left most lists unusable: k_density walks
+    // A single scene that is stale and waits, or whose last build left most lists unusable: k_walk walks
     // it in index order.
-    if (!kBatch && (sk.stale[0] != 0u || sk.ctl[kCtlPoor] != 0u)) return;
+    if (!kBatch && !sums_lists(sk)) return;
     bool walk = false;
     if (i < L.total) {
         const SceneParams& p = scene_params<kBatch>(L, i);
         uint32_t c = 0u, row = 0u;
-        walk = sk.stale[kBatch ? (uint32_t)__ldg(L.scene_of + i) : 0u] != 0u;
+        const uint32_t scene = kBatch ? (uint32_t)__ldg(L.scene_of + i) : 0u;
+        const bool built = sk.stale[scene] != 0u;  // this substep, unless the scene is walked
+        walk = !lists_in_use(sk, scene);
         // A particle of a stale scene only joins the queue: its position is not read.
         const float4 xi = walk ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : __ldg(pos + i);
         if (!walk) {
-            row = __ldg(sk.b_of_id + __float_as_uint(xi.w));
+            row = built ? i : __ldg(sk.b_of_id + __float_as_uint(xi.w));
             c = __ldg(sk.count + row);
             walk = (c & kSkinUsable) == 0u;
         }
@@ -1243,22 +1664,22 @@ __global__ void __launch_bounds__(kListBlock, 10)
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     const float r2 = in_range2(xi, xj[u]);
-                    if (r2 <= h2) d.add_r2(i, __float_as_uint(xj[u].w), r2, s_inv_h, s_nbr_cap, L.total);
+                    if (r2 <= h2) d.add_r2(i, __float_as_uint(xj[u].w), r2, true, s_inv_h, s_nbr_cap, L.total);
                 }
             }
 #pragma unroll 1
             for (; k < n_list; k++, q += stride) {
                 const float4 xj = __ldg(sk.xcur + __ldg(q));
                 const float r2 = in_range2(xi, xj);
-                if (r2 <= h2) d.add_r2(i, __float_as_uint(xj.w), r2, s_inv_h, s_nbr_cap, L.total);
+                if (r2 <= h2) d.add_r2(i, __float_as_uint(xj.w), r2, true, s_inv_h, s_nbr_cap, L.total);
             }
             density_finish(p, i, xi, vel, cx, cy, cz, distinct_keys(p, cx, cy, cz), d, rec, aux,
                            bnd, nbr_count, L.host_dens, L.defer_vel);
         }
     }
     // The walkers go to the queue in index order within the block: batched, to this block's
-    // segment (k_density takes slot t below its segment's count); a single scene, packed from 0
-    // in blocks claimed by one atomic each (k_density_walkers takes one walker per warp).
+    // segment (k_walk takes slot t below its segment's count); a single scene, packed from 0
+    // in blocks claimed by one atomic each (k_walk_queue's slots).
     __shared__ uint32_t s_cnt[kListBlock / 32];
     __shared__ uint32_t s_base;
     const uint32_t m = __ballot_sync(0xffffffffu, walk);
@@ -1282,144 +1703,12 @@ __global__ void __launch_bounds__(kListBlock, 10)
     if (walk) sk.queue[base + (uint32_t)__popc(m & ((1u << lane) - 1u))] = i;
 }
 
-// W(|x_j - x_i|) / sigma with the density drain's explicitly rounded arithmetic, from
-// r2 = in_range2(x_i, x_j).
-__device__ __forceinline__ float w_over_sigma_r2(float r2, float inv_h) {
-    const float r = r2 > 0.0f ? __fmul_rn(r2, rsqrtf(r2)) : 0.0f;
-    const float q = __fmul_rn(r, inv_h);
-    const float t = __fsub_rn(1.0f, q);
-    const float w_out = __fmul_rn(__fmul_rn(__fmul_rn(t, t), t), 2.0f);
-    const float q2 = __fmul_rn(q, q);
-    const float w_in = __fmaf_rn(6.0f, __fmul_rn(q2, q), __fmaf_rn(-6.0f, q2, 1.0f));
-    return q <= 1.0f ? (q > 0.5f ? w_out : w_in) : 0.0f;
-}
-
-// Warps per block of k_density_walkers.
-constexpr int kWalkerWarps = 4;
-
-// The density pass of a single scene's walkers (the particles k_density_list queued: no usable
-// list this substep), one warp per walker, so a walker's ~280 candidates are tested 32 at a time
-// instead of in one thread's chain of dependent loads. Lane r < 27 holds candidate segment r of
-// the walk (row r / 3, part r % 3 of the rows of for_each_candidate: the same buckets, the same
-// pruning), the segments' candidates are numbered in visiting order and taken in chunks of 32,
-// and the in-range ones are summed in visiting order (every lane adds them one by one through
-// shuffles) and listed in visiting order: exactly the sum and the list of the one-thread walk.
-__global__ void __launch_bounds__(kWalkerWarps * 32)
-    k_density_walkers(StepLaunch L, const float4* __restrict__ pos, const float4* __restrict__ vel,
-                      float4* __restrict__ rec, const uint32_t* __restrict__ scan,
-                      float4* __restrict__ aux, float4* __restrict__ bnd, uint32_t* __restrict__ nbr,
-                      uint32_t* __restrict__ nbr_count, SkinLists sk) {
-    if (sk.stale[0] != 0u || sk.ctl[kCtlPoor] != 0u) return;  // k_density walks every particle
-    const uint32_t walkers = min(*sk.wcount, L.total);
-    const int lane = threadIdx.x & 31;
-    const uint32_t lt = (1u << lane) - 1u;
-    const SceneParams& p = L.one;
-    const uint32_t* sc = scan + p.off;
-    for (uint32_t w = blockIdx.x * kWalkerWarps + (threadIdx.x >> 5); w < walkers;
-         w += gridDim.x * kWalkerWarps) {
-        const uint32_t i = __ldg(sk.queue + w);
-        const float4 xi = __ldg(pos + i);
-        const uint32_t cx = cell_coord(xi.x, p.h), cy = cell_coord(xi.y, p.h),
-                       cz = cell_coord(xi.z, p.h);
-        const bool distinct = distinct_keys(p, cx, cy, cz);
-        // Segment r of the walk: [b, b + len).
-        uint32_t b = 0u, len = 0u;
-        if (lane < 27) {
-            const float lim = distinct ? kPruneLimit : 1e30f;
-            const float fx = fmaf(-(float)(int)cx, p.h, xi.x) * p.inv_h;
-            const float fy = fmaf(-(float)(int)cy, p.h, xi.y) * p.inv_h;
-            const float fz = fmaf(-(float)(int)cz, p.h, xi.z) * p.inv_h;
-            const int t = lane / 3, part = lane % 3;
-            const uint32_t dy = (uint32_t)(t % 3) - 1u, dz = (uint32_t)(t / 3) - 1u;
-            const float dyz = face_dist2(dy, fy) + face_dist2(dz, fz);
-            if (dyz <= lim) {
-                const bool skip_l = dyz + face_dist2(0xFFFFFFFFu, fx) > lim;
-                const bool skip_r = dyz + face_dist2(1u, fx) > lim;
-                const uint32_t ry = cy + dy, rz = cz + dz;
-                const uint32_t hA = hash_cell(cx - 1u, ry, rz);
-                const uint32_t kA = key_mod(hA, p.mod_magic, p.n);
-                const bool same_block = (cx + 24u) / 50u == (cx + 26u) / 50u && hA <= 0xFFFFFFFDu;
-                uint32_t e = 0u;
-                if (same_block && kA + 2u < p.n) {
-                    if (part == 0) {
-                        b = __ldg(sc + kA + (skip_l ? 1u : 0u));
-                        e = __ldg(sc + kA + (skip_r ? 2u : 3u));
-                    }
-                } else if (part == 0) {
-                    b = __ldg(sc + kA);
-                    e = skip_l ? b : __ldg(sc + kA + 1u);
-                } else if (part == 1) {
-                    const uint32_t kB = key_mod(hash_cell(cx, ry, rz), p.mod_magic, p.n);
-                    b = __ldg(sc + kB);
-                    e = __ldg(sc + kB + 1u);
-                } else if (!skip_r) {
-                    const uint32_t kC = key_mod(hash_cell(cx + 1u, ry, rz), p.mod_magic, p.n);
-                    b = __ldg(sc + kC);
-                    e = __ldg(sc + kC + 1u);
-                }
-                len = e > b ? e - b : 0u;
-            }
-        }
-        // Exclusive prefix of the segment lengths: the visiting-order number of each segment's
-        // first candidate.
-        uint32_t incl = len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        const uint32_t start = incl - len;
-        float rho = 0.0f;
-        uint32_t listed = 0u;
-        for (uint32_t base = 0; base < total; base += 32u) {
-            const uint32_t f = base + (uint32_t)lane;
-            // The segment holding candidate f: the last one starting at or before f.
-            int r = 0;
-#pragma unroll
-            for (int step = 16; step >= 1; step >>= 1) {
-                const uint32_t s_probe = __shfl_sync(0xffffffffu, start, (r + step) & 31);
-                if (r + step < 27 && s_probe <= f) r += step;
-            }
-            const uint32_t rb = __shfl_sync(0xffffffffu, b, r);
-            const uint32_t rs = __shfl_sync(0xffffffffu, start, r);
-            const bool valid = f < total;
-            const uint32_t j = rb + (f - rs);
-            float4 xj = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (valid) xj = __ldg(pos + j);
-            const float r2 = in_range2(xi, xj);
-            const bool inr = valid && r2 <= p.h2;
-            const float wv = inr ? w_over_sigma_r2(r2, p.inv_h) : 0.0f;
-            uint32_t mask = __ballot_sync(0xffffffffu, inr);
-            const uint32_t listm = __ballot_sync(0xffffffffu, inr && j != i);
-            if (inr && j != i) {
-                const uint32_t slot = listed + (uint32_t)__popc(listm & lt);
-                if (slot < p.nbr_cap) nbr[(size_t)slot * L.total + i] = j;
-            }
-            listed += (uint32_t)__popc(listm);
-            while (mask) {
-                const int l = __ffs(mask) - 1;
-                rho = __fadd_rn(rho, __shfl_sync(0xffffffffu, wv, l));
-                mask &= mask - 1u;
-            }
-        }
-        if (lane == 0) {
-            DensitySum d;
-            d.rho = rho;
-            d.listed = listed;
-            density_finish(p, i, xi, vel, cx, cy, cz, distinct, d, rec, aux, bnd, nbr_count, L.host_dens,
-                       L.defer_vel);
-        }
-    }
-}
-
-
 // Small models, where three lanes per particle still fit one wave of the GPU and one lane per
 // particle would leave the SMs waiting on each thread's chain of candidate loads: the density pass
 // with the 27-cell walk split over three lanes of one warp, lane r walking the rows of the z-plane
 // dz = r - 1 (rows 3r..3r+2). Each lane sums its plane in visiting order and the particle's density
 // is (plane 0 + plane 1) + plane 2, whatever the list capacity. The neighbour list is the planes'
-// entries one after the other, the reference's visiting order as in k_density, so the force pass
+// entries one after the other, the reference's visiting order as in k_walk, so the force pass
 // is the same in both modes. A plane whose shared list fills mid-walk keeps summing but its
 // entries are not listed (the list length is then reported above the capacity, and the force
 // pass walks the candidates again).
@@ -1627,25 +1916,36 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
             const uint32_t* __restrict__ scan, const uint32_t* __restrict__ nbr,
             const uint32_t* __restrict__ nbr_count, float4* __restrict__ pos_out,
             float4* __restrict__ vel_out, float4* __restrict__ acc_out,
-            uint32_t* __restrict__ skin_stale, uint32_t* __restrict__ skin_ctl, HostOut ho) {
+            uint32_t* __restrict__ skin_stale, uint32_t* __restrict__ skin_ctl,
+            uint32_t* __restrict__ skin_due, HostOut ho) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     // The density pass is done with the skin lists' flags: run each scene's build policy and clear
     // the flags for the next substep.
     if (skin_stale && blockIdx.x == 0) {
+        if (threadIdx.x == 0) *skin_due = 0u;
         for (uint32_t sc = threadIdx.x; sc < L.n_scenes; sc += blockDim.x) {
             uint32_t* c = skin_ctl + sc * kSkinCtl;
             const bool stale = skin_stale[sc] != 0u;
-            uint32_t age = c[kCtlAge], wait = c[kCtlWait], since = c[kCtlSince];
+            const uint32_t n = L.n_scenes > 1 ? L.scenes[sc].n : L.one.n;
+            const uint32_t min_life = n < kSkinSmallScene ? kSkinMinLifeSmall
+                                      : n < kSkinFullScene ? kSkinMinLife
+                                                           : kSkinMinLifeFull;
+            const uint32_t grace = n < kSkinFullScene ? 0u : kSkinGrace;
+            uint32_t age = c[kCtlAge], wait = c[kCtlWait], since = c[kCtlSince], young = c[kCtlYoung];
             if (stale && c[kCtlFresh]) {  // the last build's lists just went stale: were they worth it?
-                wait = age < kSkinMinLife || c[kCtlPoor] ? min(max(2u * wait, kSkinMinWait), kSkinMaxWait) : 0u;
+                if (age < min_life || c[kCtlPoor]) {
+                    young++;
+                    if (young > grace || c[kCtlPoor]) wait = min(max(2u * wait, kSkinMinWait), kSkinMaxWait);
+                } else {
+                    young = wait = 0u;
+                }
                 c[kCtlFresh] = 0u;
                 since = 0u;
             }
             if (stale && c[kCtlAllow]) {  // the density pass rebuilt
-                const uint32_t n = L.n_scenes > 1 ? L.scenes[sc].n : L.one.n;
                 c[kCtlBuilds]++;
                 c[kCtlFresh] = 1u;
-                c[kCtlPoor] = 2u * c[kCtlUsable] < n ? 1u : 0u;
+                c[kCtlPoor] = c[kCtlUsable] < n - n / kSkinPoorPart ? 1u : 0u;
                 c[kCtlUsable] = 0u;
                 age = 0u;
             } else {
@@ -1656,7 +1956,11 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
             c[kCtlAge] = age;
             c[kCtlWait] = wait;
             c[kCtlSince] = since;
-            c[kCtlAllow] = !c[kCtlFresh] && since >= wait ? 1u : 0u;
+            c[kCtlYoung] = young;
+            // Lists that have lived long enough are rebuilt in the very substep they go stale in
+            // (a small scene's, which walks beside the others of its batch, one substep later).
+            const bool at_once = n >= kSkinSmallScene && (age >= min_life || young < grace) && !c[kCtlPoor];
+            c[kCtlAllow] = (c[kCtlFresh] ? at_once : since >= wait) ? 1u : 0u;
         }
     }
     // The particle's new position and velocity and its density, for the host outputs.
@@ -2206,15 +2510,15 @@ cudaError_t launch_cells_reorder(const StepLaunch& L, uint32_t n, const uint32_t
     switch (kc.cell_block) {
         case 128:
             k_cells_reorder<128><<<(n + 128u) / 128u, 128, 0, s>>>(L, n, skeys, perm, cell_scan, pos_in,
-                                                                 vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl);
+                                                                 vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl, sk.wcount);
             break;
         case 512:
             k_cells_reorder<512><<<(n + 512u) / 512u, 512, 0, s>>>(L, n, skeys, perm, cell_scan, pos_in,
-                                                                 vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl);
+                                                                 vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl, sk.wcount);
             break;
         default:
             k_cells_reorder<256><<<(n + 256u) / 256u, 256, 0, s>>>(L, n, skeys, perm, cell_scan, pos_in,
-                                                                 vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl);
+                                                                 vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl, sk.wcount);
     }
     return cudaGetLastError();
 }
@@ -2232,18 +2536,65 @@ static int sm_count() {
     return n;
 }
 
+constexpr size_t kTileSmemBytes = kTileWarps * sizeof(TileSmem);
+
+// Blocks of one resident wave of a tile kernel over `total` particles (fewer when they cover them).
+// Residency per SM is asked of the occupancy calculator once per kernel and device.
+template <typename Kernel>
+cudaError_t tile_blocks(Kernel* kernel, std::atomic<int>* per_sm, uint32_t total, uint32_t& blocks) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    int r = dev < 16 ? per_sm[dev].load(std::memory_order_relaxed) : 0;
+    if (r == 0) {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmemBytes);
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kernel, kTileWarps * 32, kTileSmemBytes);
+        if (e != cudaSuccess) return e;
+        if (r < 1) r = 1;
+        if (dev < 16) per_sm[dev].store(r, std::memory_order_relaxed);
+    }
+    const int sms = sm_count();
+    blocks = (total + kTileWarps * 32 - 1) / (kTileWarps * 32);
+    if (sms > 0) blocks = min(blocks, (uint32_t)sms * (uint32_t)r);
+    return cudaSuccess;
+}
+
+template <bool kBatch>
+cudaError_t launch_build(const StepLaunch& L, const float4* pos, const uint32_t* cell_scan,
+                         const SkinLists& sk, cudaStream_t s) {
+    static std::atomic<int> per_sm[16];
+    uint32_t blocks = 0u;
+    const cudaError_t e = tile_blocks(k_skin_build<kBatch>, per_sm, L.total, blocks);
+    if (e != cudaSuccess) return e;
+    k_skin_build<kBatch><<<blocks, kTileWarps * 32, kTileSmemBytes, s>>>(L, pos, cell_scan, sk);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_walk_queue(const StepLaunch& L, const float4* pos, const float4* vel, float4* rec,
+                              const uint32_t* cell_scan, float4* aux, float4* bnd, uint32_t* nbr,
+                              uint32_t* nbr_count, const SkinLists& sk, uint32_t* sched, bool tiles,
+                              cudaStream_t s) {
+    static std::atomic<int> per_sm[16];
+    uint32_t blocks = 0u;
+    const cudaError_t e = tile_blocks(k_walk_queue, per_sm, L.total, blocks);
+    if (e != cudaSuccess) return e;
+    k_walk_queue<<<blocks, kTileWarps * 32, kTileSmemBytes, s>>>(L, pos, vel, rec, cell_scan, aux, bnd, nbr,
+                                                                 nbr_count, sk, sched, tiles);
+    return cudaGetLastError();
+}
+
 // One resident wave of the walk kernel: its blocks take runs of slots until none is left, so
 // more blocks would only start after the work is gone. Residency per SM is asked of the
 // occupancy calculator once per instantiation.
-template <bool kBatch, int B, int M, bool kStaging>
-void launch_walk(const StepLaunch& L, const float4* pos, const float4* vel, float4* rec,
-                 const uint32_t* cell_scan, float4* aux, float4* bnd, uint32_t* nbr,
-                 uint32_t* nbr_count, const SkinLists& sk, uint32_t* sched, cudaStream_t s) {
+template <bool kBatch, int B, int M>
+cudaError_t launch_walk(const StepLaunch& L, const float4* pos, const float4* vel, float4* rec,
+                        const uint32_t* cell_scan, float4* aux, float4* bnd, uint32_t* nbr,
+                        uint32_t* nbr_count, const SkinLists& sk, uint32_t* sched, cudaStream_t s) {
     static std::atomic<int> per_sm{0};
     int r = per_sm.load(std::memory_order_relaxed);
     if (r == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_density<kBatch, B, M, kStaging>, B, 0) ==
-                cudaSuccess && r > 0)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_walk<kBatch, B, M>, B, 0) == cudaSuccess && r > 0)
             per_sm.store(r, std::memory_order_relaxed);
         else
             r = M;
@@ -2251,39 +2602,21 @@ void launch_walk(const StepLaunch& L, const float4* pos, const float4* vel, floa
     const int sms = sm_count();
     const uint32_t all_blocks = (L.total + B - 1) / B;
     const uint32_t blocks = sms > 0 ? min(all_blocks, (uint32_t)sms * (uint32_t)r) : all_blocks;
-    k_density<kBatch, B, M, kStaging><<<blocks, B, 0, s>>>(L, pos, vel, rec, cell_scan, aux, bnd, nbr,
-                                                           nbr_count, sk, sched);
+    k_walk<kBatch, B, M><<<blocks, B, 0, s>>>(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, sched);
+    return cudaGetLastError();
 }
 
-template <int B, int M>
-void density_shape(const StepLaunch& L, const float4* pos, const float4* vel, float4* rec,
-                   const uint32_t* cell_scan, float4* aux, float4* bnd, uint32_t* nbr,
-                   uint32_t* nbr_count, const SkinLists& sk, uint32_t* sched, bool staging,
-                   cudaStream_t s) {
-    if (sk.list) {
-        // Skin lists: the list pass first; the walk passes then take the queue it leaves.
-        const uint32_t lb = (L.total + kListBlock - 1) / kListBlock;
-        if (L.n_scenes > 1) {
-            k_density_list<true><<<lb, kListBlock, 0, s>>>(L, pos, vel, rec, aux, bnd, nbr, nbr_count, sk);
-        } else {
-            cudaMemsetAsync(sk.wcount, 0, sizeof(uint32_t), s);
-            k_density_list<false><<<lb, kListBlock, 0, s>>>(L, pos, vel, rec, aux, bnd, nbr, nbr_count, sk);
-            const int sms = sm_count();
-            const uint32_t wb = (uint32_t)(sms > 0 ? sms : 148) * 8u;  // 32 warps per SM
-            k_density_walkers<<<wb, kWalkerWarps * 32, 0, s>>>(L, pos, vel, rec, cell_scan, aux, bnd,
-                                                               nbr, nbr_count, sk);
-        }
-    }
-    if (L.n_scenes > 1) {
-        if (staging)
-            launch_walk<true, B, M, true>(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, sched, s);
-        else
-            launch_walk<true, B, M, false>(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, sched, s);
-    } else {
-        if (staging)
-            launch_walk<false, B, M, true>(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, sched, s);
-        else
-            launch_walk<false, B, M, false>(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, sched, s);
+// The walk in the density pass's launch shape.
+template <bool kBatch>
+cudaError_t launch_walk_shaped(int shape, const StepLaunch& L, const float4* pos, const float4* vel,
+                               float4* rec, const uint32_t* cell_scan, float4* aux, float4* bnd,
+                               uint32_t* nbr, uint32_t* nbr_count, const SkinLists& sk, uint32_t* sched,
+                               cudaStream_t s) {
+    switch (shape) {
+        case kNbr128x8: return launch_walk<kBatch, 128, 8>(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, sched, s);
+        case kNbr96x8: return launch_walk<kBatch, 96, 8>(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, sched, s);
+        case kNbr64x12: return launch_walk<kBatch, 64, 12>(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, sched, s);
+        default: return launch_walk<kBatch, 128, 6>(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, sched, s);
     }
 }
 
@@ -2295,11 +2628,12 @@ void force_shape(const StepLaunch& L, const float4* pos, const float4* vel, cons
     const uint32_t blocks = (L.total + B - 1) / B;
     if (L.n_scenes > 1)
         k_force<true, B, M><<<blocks, B, 0, s>>>(L, pos, vel, aux, rec, bnd, cell_scan, nbr, nbr_count,
-                                                 pos_out, vel_out, acc_out, sk.stale, sk.ctl, HostOut{});
+                                                 pos_out, vel_out, acc_out, sk.stale, sk.ctl,
+                                                 sk.wcount + 1, HostOut{});
     else  // shared memory only for host outputs: without them the whole on-chip memory stays L1
         k_force<false, B, M><<<blocks, B, ho.any() ? 7 * B * sizeof(float) : 0, s>>>(
             L, pos, vel, aux, rec, bnd, cell_scan, nbr, nbr_count, pos_out, vel_out, acc_out,
-            sk.stale, sk.ctl, ho);
+            sk.stale, sk.ctl, sk.wcount + 1, ho);
 }
 
 bool planes_mode(uint32_t total) {
@@ -2322,14 +2656,24 @@ cudaError_t launch_density(const StepLaunch& L, const float4* pos, const float4*
                                                                    nbr, nbr_count);
         return cudaGetLastError();
     }
-    const bool st = kc.walk_staging != 0;
-    switch (kc.nbr_shape) {
-        case kNbr128x8: density_shape<128, 8>(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, walk_sched, st, s); break;
-        case kNbr96x8: density_shape<96, 8>(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, walk_sched, st, s); break;
-        case kNbr64x12: density_shape<64, 12>(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, walk_sched, st, s); break;
-        default: density_shape<128, 6>(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, walk_sched, st, s);
+    const bool batch = L.n_scenes > 1;
+    if (sk.list) {
+        // Skin lists: the build where it is due, then the list pass, then the walk of the queue it
+        // leaves (a batch's below).
+        cudaError_t e = batch ? launch_build<true>(L, pos, cell_scan, sk, s) : launch_build<false>(L, pos, cell_scan, sk, s);
+        if (e != cudaSuccess) return e;
+        const uint32_t lb = (L.total + kListBlock - 1) / kListBlock;
+        if (batch) {
+            k_density_list<true><<<lb, kListBlock, 0, s>>>(L, pos, vel, rec, aux, bnd, nbr, nbr_count, sk);
+        } else {
+            k_density_list<false><<<lb, kListBlock, 0, s>>>(L, pos, vel, rec, aux, bnd, nbr, nbr_count, sk);
+            e = launch_walk_queue(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, walk_sched,
+                                  kc.walk_staging != 0, s);
+            if (e != cudaSuccess) return e;
+        }
     }
-    return cudaGetLastError();
+    return batch ? launch_walk_shaped<true>(kc.nbr_shape, L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, walk_sched, s)
+                 : launch_walk_shaped<false>(kc.nbr_shape, L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, walk_sched, s);
 }
 
 cudaError_t launch_force(const StepLaunch& L, const float4* pos, const float4* vel,

@@ -489,7 +489,7 @@ class WCSPHWithBoundaryModel:
         check(self._lib.vfs_model_set_skin(self._h, skin))
 
     def set_walk_staging(self, enable: bool) -> None:
-        """Block-per-cell staging of the density walk (on by default; bit-identical results)."""
+        """Block-per-cell staging of a crowd's density walk (on by default; bit-identical results)."""
         check(self._lib.vfs_model_set_walk_staging(self._h, int(bool(enable))))
 
     def skin_builds(self) -> int:
