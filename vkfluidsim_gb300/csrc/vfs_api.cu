@@ -395,11 +395,17 @@ int Model::enqueue_substep(cudaEvent_t* ev) {
     if (ev) VFS_CUDA_TRY(cudaEventRecord(ev[0], s));
     // The sort scratch is zero here: zeroed when allocated and by every substep's cell pass.
     if (ev) VFS_CUDA_TRY(cudaEventRecord(ev[1], s));
-    // Incremental stable sort: keys + the particles whose key changed (compacted into keys/vals),
-    // a sort of those alone (count on the device), a merge with the rest.
+    // A small model sorts in one launch. Otherwise an incremental stable sort: keys + the particles
+    // whose key changed (compacted into keys/vals), a sort of those alone (count on the device), a
+    // merge with the rest.
     const SkinLists sk = active_skin();
-    VFS_CUDA_TRY(launch_keys_delta(launch, pos[c], pkeys, keys, vals, moved, sc, sort_scratch, s,
-                                   host_pos, pos[c], aux, skin.b_of_id, host_b_next));
+    const bool small = small_sort(n);
+    if (small)
+        VFS_CUDA_TRY(launch_sort_small(launch, pos[c], sk_buf, sp_buf, cell_scan, s, host_pos, pos[c], aux,
+                                       skin.b_of_id, host_b_next));
+    else
+        VFS_CUDA_TRY(launch_keys_delta(launch, pos[c], pkeys, keys, vals, moved, sc, sort_scratch, s,
+                                       host_pos, pos[c], aux, skin.b_of_id, host_b_next));
     if (host_pos) {
         int rc = move_build_indices(host_b_next, 0, n);
         if (rc) return rc;
@@ -407,10 +413,12 @@ int Model::enqueue_substep(cudaEvent_t* ev) {
         if (rc) return rc;
     }
     if (ev) VFS_CUDA_TRY(cudaEventRecord(ev[2], s));
-    uint32_t *mk = nullptr, *mi = nullptr;
-    VFS_CUDA_TRY(launch_sort(n, sc, sort_scratch, keys, keys_alt, vals, vals_alt, &mk, &mi, s,
-                             /*vals_given=*/true, sort_scratch.mcount));
-    VFS_CUDA_TRY(launch_merge(n, pkeys, moved, sort_scratch.mcount, mk, mi, sk_buf, sp_buf, s));
+    if (!small) {
+        uint32_t *mk = nullptr, *mi = nullptr;
+        VFS_CUDA_TRY(launch_sort(n, sc, sort_scratch, keys, keys_alt, vals, vals_alt, &mk, &mi, s,
+                                 /*vals_given=*/true, sort_scratch.mcount));
+        VFS_CUDA_TRY(launch_merge(n, pkeys, moved, sort_scratch.mcount, mk, mi, sk_buf, sp_buf, s));
+    }
     skeys = sk_buf;
     sperm = sp_buf;
     if (ev) VFS_CUDA_TRY(cudaEventRecord(ev[3], s));
@@ -422,9 +430,12 @@ int Model::enqueue_substep(cudaEvent_t* ev) {
         ~DeferOff() { l.defer_vel = false; }
     } defer_off{launch};
     launch.defer_vel = cells_wait != nullptr;
-    VFS_CUDA_TRY(launch_cells_reorder(launch, n, skeys, sperm, cell_scan, pos[c], vel[c], pos[o], vel[o],
-                                      scratch, (uint32_t)sort_scratch_words(sc), pkeys, cell_guess,
-                                      sk, kc, s));
+    if (small)
+        VFS_CUDA_TRY(launch_reorder(launch, n, sperm, pos[c], vel[c], pos[o], vel[o], sk, s));
+    else
+        VFS_CUDA_TRY(launch_cells_reorder(launch, n, skeys, sperm, cell_scan, pos[c], vel[c], pos[o], vel[o],
+                                          scratch, (uint32_t)sort_scratch_words(sc), pkeys, cell_guess,
+                                          sk, kc, s));
     if (ev) VFS_CUDA_TRY(cudaEventRecord(ev[4], s));
     VFS_CUDA_TRY(launch_density(launch, pos[o], vel[o], rec, cell_scan, aux, bnd, nbr, nbr_count, sk,
                                 walk_sched, kc, s));

@@ -214,6 +214,17 @@ cudaError_t launch_keys_delta(const StepLaunch& L, const float4* pos, const uint
                               const float* host3 = nullptr, float4* pos_out = nullptr,
                               float4* aux = nullptr, const uint32_t* b_of_id = nullptr,
                               uint32_t* b_next = nullptr);
+// Models of up to 65,536 particles in all: keys, stable sort and cell starts in one launch
+// (launch_sort_small, in place of the incremental sort and launch_cells_reorder's cell starts; the
+// host arguments as in launch_keys_delta), then the gather alone (launch_reorder).
+bool small_sort(uint32_t total);
+cudaError_t launch_sort_small(const StepLaunch& L, const float4* pos, uint32_t* skeys, uint32_t* perm,
+                              uint32_t* cell_scan, cudaStream_t s, const float* host3 = nullptr,
+                              float4* pos_out = nullptr, float4* aux = nullptr,
+                              const uint32_t* b_of_id = nullptr, uint32_t* b_next = nullptr);
+cudaError_t launch_reorder(const StepLaunch& L, uint32_t n, const uint32_t* perm, const float4* pos_in,
+                           const float4* vel_in, float4* pos_out, float4* vel_out, const SkinLists& sk,
+                           cudaStream_t s);
 // Incremental sort, last pass: merge of the unmoved particles with the sorted moved ones into the
 // stable sort of all (key, index) pairs.
 cudaError_t launch_merge(uint32_t n, const uint32_t* pkeys, const uint32_t* bits,

@@ -18,6 +18,7 @@
 // array, so the three buckets are one contiguous range [scan[kA], scan[kA+3]). When the three
 // keys are not consecutive, each bucket is walked on its own. Duplicate keys among the 27 are
 // walked as often as they occur, like wcsph_with_boundary_model.slang:166-190.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -519,6 +520,60 @@ __device__ __forceinline__ uint32_t lower_bound_near(const uint32_t* __restrict_
     return lo;
 }
 
+// The gather of particle i (every thread of the block calls it, i >= n too): position and velocity
+// by the sort's permutation; with skin lists (xcur set), the position and sorted index under the
+// particle's build index and its displacement since the build, flagging its scene.
+__device__ __forceinline__ void reorder_particle(
+    const StepLaunch& L, uint32_t i, uint32_t n, const uint32_t* __restrict__ perm,
+    const float4* __restrict__ pos_in, const float4* __restrict__ vel_in, float4* __restrict__ pos_out,
+    float4* __restrict__ vel_out, const uint32_t* __restrict__ b_of_id, float4* __restrict__ xcur,
+    const float4* __restrict__ x_build, uint32_t* __restrict__ stale, const uint32_t* __restrict__ ctl,
+    uint32_t* __restrict__ wcount) {
+    bool exceed = false;  // skin lists: the particle moved past h skin / 2 since its list build
+    uint32_t exceed_sc = 0u;
+    if (i < n) {
+        uint32_t src = perm[i];
+        if (src >= n) src = i;  // only after a reported sort failure
+        const float4 x = __ldg(pos_in + src);
+        pos_out[i] = x;
+        if (!L.defer_vel) vel_out[i] = __ldg(vel_in + src);
+        if (xcur) {
+            const uint32_t sc = L.n_scenes > 1 ? (uint32_t)__ldg(L.scene_of + i) : 0u;
+            exceed_sc = sc;
+            if (ctl[sc * kSkinCtl + kCtlFresh] == 0u) {
+                // No build yet, or the last build's lists have gone stale: they stay unusable
+                // until the next build, so the scene is stale without a displacement check, and
+                // nothing reads its positions by build index.
+                exceed = true;
+            } else {
+                // Skin lists: the particle's current position and sorted index under its build
+                // index (the list pass gathers both with one load), and its displacement since
+                // the build.
+                const uint32_t id = __float_as_uint(x.w);
+                const uint32_t bi = id < n ? __ldg(b_of_id + id) : n;
+                if (bi < n) {
+                    xcur[bi] = make_float4(x.x, x.y, x.z, __uint_as_float(i));
+                    const float4 b = __ldg(x_build + bi);
+                    const float dx = x.x - b.x, dy = x.y - b.y, dz = x.z - b.z;
+                    const float lim = L.n_scenes > 1 ? L.scenes[sc].skin_half2 : L.one.skin_half2;
+                    exceed = !(dx * dx + dy * dy + dz * dz <= lim);
+                }
+            }
+        }
+    }
+    // Stale scenes, one atomic per warp and scene at most (most particles of a fast scene exceed).
+    if (xcur) {
+        const uint32_t m = __ballot_sync(0xffffffffu, exceed);
+        if (exceed) {
+            const uint32_t g = __match_any_sync(m, exceed_sc);
+            if ((threadIdx.x & 31u) == (uint32_t)(__ffs(g) - 1) && ld_volatile(stale + exceed_sc) == 0u) {
+                atomicOr(stale + exceed_sc, 1u);
+                if (ctl[exceed_sc * kSkinCtl + kCtlAllow]) wcount[1] = 1u;  // a build is due
+            }
+        }
+    }
+}
+
 template <uint32_t kCellBlock>
 __global__ void __launch_bounds__(kCellBlock)
     k_cells_reorder(StepLaunch L, uint32_t n, const uint32_t* __restrict__ skeys,
@@ -551,50 +606,8 @@ __global__ void __launch_bounds__(kCellBlock)
         s_hi = guess ? lower_bound_near(skeys, n, c1, ((volatile uint32_t*)guess)[blockIdx.x + 1])
                      : lower_bound_keys(skeys, n, c1);
     const uint32_t i = c0 + tid;
-    bool exceed = false;  // skin lists: the particle moved past h skin / 2 since its list build
-    uint32_t exceed_sc = 0u;
-    if (i < n) {
-        uint32_t src = perm[i];
-        if (src >= n) src = i;  // only after a reported sort failure
-        const float4 x = __ldg(pos_in + src);
-        pos_out[i] = x;
-        if (!L.defer_vel) vel_out[i] = __ldg(vel_in + src);
-        if (xcur) {
-            const uint32_t sc = L.n_scenes > 1 ? (uint32_t)__ldg(L.scene_of + i) : 0u;
-            exceed_sc = sc;
-            if (ctl[sc * kSkinCtl + kCtlFresh] == 0u) {
-                // No build yet, or the last build's lists have gone stale: they stay unusable
-                // until the next build, so the scene is stale without a displacement check, and
-                // nothing reads its positions by build index.
-                exceed = true;
-            } else {
-                // Skin lists: the particle's current position and sorted index under its build
-                // index (the list pass gathers both with one load), and its displacement since
-                // the build.
-                const uint32_t id = __float_as_uint(x.w);
-                const uint32_t bi = id < n ? __ldg(b_of_id + id) : n;
-                if (bi < n) {
-                    xcur[bi] = make_float4(x.x, x.y, x.z, __uint_as_float(i));
-                    const float4 b = __ldg(x_build + bi);
-                    const float dx = x.x - b.x, dy = x.y - b.y, dz = x.z - b.z;
-                    const float lim = L.n_scenes > 1 ? L.scenes[sc].skin_half2 : L.one.skin_half2;
-                    exceed = !(dx * dx + dy * dy + dz * dz <= lim);
-                }
-            }
-        }
-        if (pkeys_out) pkeys_out[i] = skeys[i];
-    }
-    // Stale scenes, one atomic per warp and scene at most (most particles of a fast scene exceed).
-    if (xcur) {
-        const uint32_t m = __ballot_sync(0xffffffffu, exceed);
-        if (exceed) {
-            const uint32_t g = __match_any_sync(m, exceed_sc);
-            if ((tid & 31u) == (uint32_t)(__ffs(g) - 1) && ld_volatile(stale + exceed_sc) == 0u) {
-                atomicOr(stale + exceed_sc, 1u);
-                if (ctl[exceed_sc * kSkinCtl + kCtlAllow]) wcount[1] = 1u;  // a build is due
-            }
-        }
-    }
+    reorder_particle(L, i, n, perm, pos_in, vel_in, pos_out, vel_out, b_of_id, xcur, x_build, stale, ctl, wcount);
+    if (i < n && pkeys_out) pkeys_out[i] = skeys[i];
     __syncthreads();
     const uint32_t lo = s_lo, hi = max(s_lo, s_hi);
     if (lo == hi) {
@@ -609,6 +622,18 @@ __global__ void __launch_bounds__(kCellBlock)
     }
     const uint32_t last = max(min(skeys[hi - 1u], c1 - 1u) + 1u, c0);
     for (uint32_t c = last + tid; c < c1; c += kCellBlock) scan[c] = hi;
+}
+
+// The gather alone, for models whose sort writes the cell starts (k_sort_small).
+__global__ void __launch_bounds__(128)
+    k_reorder(StepLaunch L, uint32_t n, const uint32_t* __restrict__ perm, const float4* __restrict__ pos_in,
+              const float4* __restrict__ vel_in, float4* __restrict__ pos_out, float4* __restrict__ vel_out,
+              const uint32_t* __restrict__ b_of_id, float4* __restrict__ xcur,
+              const float4* __restrict__ x_build, uint32_t* __restrict__ stale,
+              const uint32_t* __restrict__ ctl, uint32_t* __restrict__ wcount) {
+    if (wcount && blockIdx.x == 0 && threadIdx.x == 0) wcount[0] = 0u;  // the list pass's queue
+    reorder_particle(L, blockIdx.x * 128u + threadIdx.x, n, perm, pos_in, vel_in, pos_out, vel_out, b_of_id,
+                     xcur, x_build, stale, ctl, wcount);
 }
 
 __global__ void __launch_bounds__(256)
@@ -2334,6 +2359,206 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// ---------------------------------------------------------------- small models: one kernel
+// Keys, stable sort and cell starts of a model of up to kSmallSort particles in one cluster of 8 or
+// 16 blocks, everything in (distributed) shared memory: a key and an index, 16 bits each, in one
+// word. The incremental sort and the cell starts cost such a model six launches and 39 to 44 us under
+// ncu, nearly all of it launch and dependent-load latency (8 bytes a particle take under a
+// microsecond to move); this kernel and the gather take 15 us at 5,000 particles, 26 at 47,000 (30
+// with eight blocks), 28 at 65,536: block barriers, cluster barriers (seven) and the ranking of up to
+// four items per thread. More than 65,536 particles would need two words an item.
+// Block c holds positions [c S, c S + S) of the array being sorted, S = ceil(n / blocks / 32) 32. Each of one
+// or two LSD passes ranks its items as k_onesweep does (per-warp histograms, match.any), exchanges
+// the blocks' digit counts, and stores every item straight into its place in the owner's shared
+// memory. The heads of equal keys are then stored into a table over the keys, and a suffix minimum
+// over it gives every key's first position.
+constexpr uint32_t kSmallSort = 65536;
+
+template <bool kBatch, bool kHostIn, int kBlocks, int ITEMS>
+__global__ void __launch_bounds__(1024, 1)
+    k_sort_small(StepLaunch L, const float4* __restrict__ pos, int digit_bits, int passes,
+                 uint32_t* __restrict__ skeys, uint32_t* __restrict__ perm, uint32_t* __restrict__ scan,
+                 const float* __restrict__ host3, float4* __restrict__ pos_out, float4* __restrict__ aux,
+                 const uint32_t* __restrict__ b_of_id, uint32_t* __restrict__ b_next) {
+    namespace cg = cooperative_groups;
+    constexpr uint32_t kSeg = 1024u * ITEMS;
+    extern __shared__ uint32_t s_mem[];
+    uint32_t* const s_buf = s_mem;                      // [2][kSeg] key << 16 | index
+    uint32_t* const s_head = s_mem + 2 * kSeg;          // [kSeg] first position of each key of this block's
+    uint32_t* const s_whist = s_mem + 3 * kSeg;         // [32][256] per-warp digit counts, then prefixes
+    __shared__ uint32_t s_cnt[256], s_base[256], s_warp[32], s_min;
+    __shared__ float s_p[kHostIn ? 3072 : 1];
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t n = L.total, c = cluster.block_rank();
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    constexpr uint32_t kUnit = 32u * kBlocks;
+    const uint32_t S = ((n + kUnit - 1u) / kUnit) * 32u;
+    const uint32_t magic = 0xFFFFFFFFu / S + 1u;  // pos / S = umulhi(pos, magic) for pos < 2^16
+    const uint32_t first = c * S, mine = first < n ? min(S, n - first) : 0u;
+    const uint32_t lt = (1u << lane) - 1u;
+    // Keys of the block's particles, in index order.
+    for (uint32_t t0 = 0; t0 < mine; t0 += 1024u) {
+        const uint32_t t = t0 + tid, i = first + t;
+        float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (kHostIn) {
+            // Page-locked positions of a host round trip, stored as the state upload stores them
+            // (see k_keys_flags): coalesced through shared memory.
+            const uint32_t m3 = 3u * min(1024u, mine - t0);
+            const float* src = host3 + 3 * (size_t)(first + t0);
+            __syncthreads();
+            for (uint32_t k = tid; k < m3; k += 1024u) s_p[k] = src[k];
+            __syncthreads();
+            if (t < mine) {
+                x = make_float4(s_p[3u * tid], s_p[3u * tid + 1u], s_p[3u * tid + 2u], __uint_as_float(i));
+                if (b_next) {
+                    const uint32_t old = __float_as_uint(pos_out[i].w);
+                    b_next[i] = old < n ? b_of_id[old] : 0u;
+                }
+                pos_out[i] = x;
+                aux[i].z = 0.0f;
+            }
+        } else if (t < mine) {
+            x = __ldg(pos + i);
+        }
+        if (t < mine) s_buf[t] = particle_key<kBatch>(L, i, x) << 16 | i;
+    }
+    for (uint32_t k = tid; k < S; k += 1024u) s_head[k] = 0xFFFFFFFFu;
+    const uint32_t bins = 1u << digit_bits, mask = bins - 1u;
+    uint32_t* cur = s_buf;
+    uint32_t* nxt = s_buf + kSeg;
+    for (int ps = 0; ps < passes; ps++) {
+        const int shift = 16 + ps * digit_bits;
+        for (uint32_t k = tid; k < 32u * bins; k += 1024u) s_whist[k] = 0u;
+        __syncthreads();
+        uint32_t v[ITEMS], r[ITEMS];
+#pragma unroll
+        for (int it = 0; it < ITEMS; it++) {
+            const uint32_t t = (warp * ITEMS + it) * 32u + lane;
+            const bool valid = t < mine;
+            v[it] = valid ? cur[t] : 0u;
+            const uint32_t d = valid ? (v[it] >> shift) & mask : bins;
+            const uint32_t peers = __match_any_sync(0xffffffffu, d);
+            const uint32_t pre = (uint32_t)__popc(peers & lt);
+            uint32_t prev = 0u;
+            if (valid) prev = s_whist[warp * bins + d];
+            __syncwarp();
+            if (valid && pre == 0u) s_whist[warp * bins + d] = prev + (uint32_t)__popc(peers);
+            __syncwarp();
+            r[it] = prev + pre;
+        }
+        __syncthreads();
+        // Per digit, the prefix over the warps: four threads a digit, eight warps each.
+        if (tid < 4u * bins) {
+            const uint32_t d = tid >> 2, w0 = 8u * (tid & 3u);
+            uint32_t sum = 0u;
+#pragma unroll
+            for (uint32_t w = 0; w < 8u; w++) sum += s_whist[(w0 + w) * bins + d];
+            uint32_t incl = sum;
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o, 4);
+                if ((int)(tid & 3u) >= o) incl += t;
+            }
+            uint32_t run = incl - sum;
+#pragma unroll
+            for (uint32_t w = 0; w < 8u; w++) {
+                const uint32_t t = s_whist[(w0 + w) * bins + d];
+                s_whist[(w0 + w) * bins + d] = run;
+                run += t;
+            }
+            if ((tid & 3u) == 3u) s_cnt[d] = run;
+        }
+        cluster.sync();
+        // A digit's first position: all blocks' smaller digits, then the earlier blocks' same digit.
+        uint32_t lower = 0u, total = 0u;
+        if (tid < bins) {
+#pragma unroll
+            for (uint32_t b = 0; b < (uint32_t)kBlocks; b++) {
+                const uint32_t k = cluster.map_shared_rank(s_cnt, b)[tid];
+                lower += b < c ? k : 0u;
+                total += k;
+            }
+        }
+        uint32_t incl = total;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+            if ((int)lane >= o) incl += t;
+        }
+        if (lane == 31u) s_warp[warp] = incl;
+        __syncthreads();
+        if (tid < bins) {
+            uint32_t before = 0u;
+            for (uint32_t w = 0; w < warp; w++) before += s_warp[w];  // at most 7
+            s_base[tid] = before + incl - total + lower;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int it = 0; it < ITEMS; it++) {
+            if ((warp * ITEMS + it) * 32u + lane < mine) {
+                const uint32_t d = (v[it] >> shift) & mask;
+                const uint32_t to = s_base[d] + s_whist[warp * bins + d] + r[it];
+                const uint32_t b = __umulhi(to, magic);
+                cluster.map_shared_rank(nxt, b)[to - b * S] = v[it];
+            }
+        }
+        cluster.sync();
+        uint32_t* const t = cur;
+        cur = nxt;
+        nxt = t;
+    }
+    // The sorted arrays, and the heads of equal keys into the table of their keys' owner (owner b
+    // holds keys [b S, b S + S)).
+    for (uint32_t t = tid; t < mine; t += 1024u) {
+        const uint32_t i = first + t, key = cur[t] >> 16;
+        skeys[i] = key;
+        perm[i] = cur[t] & 0xFFFFu;
+        uint32_t before = 0xFFFFFFFFu;
+        if (t) before = cur[t - 1u] >> 16;
+        else if (i) before = cluster.map_shared_rank(cur, c - 1u)[S - 1u] >> 16;
+        if (key != before) {
+            const uint32_t b = __umulhi(key, magic);
+            cluster.map_shared_rank(s_head, b)[key - b * S] = i;
+        }
+    }
+    cluster.sync();
+    // scan[k] = the smallest head of the keys >= k (n when none): a suffix minimum, ITEMS keys a thread.
+    uint32_t h[ITEMS];
+    uint32_t low = 0xFFFFFFFFu;
+#pragma unroll
+    for (int it = ITEMS - 1; it >= 0; it--) {
+        const uint32_t k = tid * ITEMS + it;
+        if (k < S) low = min(low, s_head[k]);
+        h[it] = low;
+    }
+    uint32_t after = low;  // over this thread and the later ones of its warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_down_sync(0xffffffffu, after, o);
+        if (lane + (uint32_t)o < 32u) after = min(after, t);
+    }
+    if (lane == 0u) s_warp[warp] = after;
+    __syncthreads();
+    if (tid == 0u) {
+        uint32_t m = 0xFFFFFFFFu;
+        for (uint32_t w = 0; w < 32u; w++) m = min(m, s_warp[w]);
+        s_min = m;
+    }
+    cluster.sync();
+    uint32_t rest = n;
+    for (uint32_t b = c + 1u; b < (uint32_t)kBlocks; b++) rest = min(rest, *cluster.map_shared_rank(&s_min, b));
+    for (uint32_t w = warp + 1u; w < 32u; w++) rest = min(rest, s_warp[w]);
+    const uint32_t later = __shfl_down_sync(0xffffffffu, after, 1);
+    if (lane < 31u) rest = min(rest, later);
+#pragma unroll
+    for (int it = 0; it < ITEMS; it++) {
+        const uint32_t k = tid * ITEMS + it;
+        if (k < S && first + k < n) scan[first + k] = min(h[it], rest);
+    }
+    if (c == 0u && tid == 0u) scan[n] = n;
+    cluster.sync();  // no block leaves while another may read its shared memory
+}
+
 constexpr int kSortBlock = 256;
 
 template <int ITEMS>
@@ -2428,6 +2653,84 @@ cudaError_t launch_keys_delta(const StepLaunch& L, const float4* pos, const uint
         k_moved_compact<true, false><<<tiles, 256, 0, s>>>(L, pos, bits, scr.dstatus, mkeys, midx, scr.mcount);
     else
         k_moved_compact<false, false><<<tiles, 256, 0, s>>>(L, pos, bits, scr.dstatus, mkeys, midx, scr.mcount);
+    return cudaGetLastError();
+}
+
+bool small_sort(uint32_t total) { return total <= kSmallSort; }
+
+namespace {
+// A cluster of 16 blocks is more than every device need schedule: asked once per device.
+template <bool kBatch, bool kHostIn, int kBlocks, int ITEMS>
+cudaError_t sort_small_items(const StepLaunch& L, const float4* pos, int bits, int passes, uint32_t* skeys,
+                             uint32_t* perm, uint32_t* scan, const float* host3, float4* pos_out, float4* aux,
+                             const uint32_t* b_of_id, uint32_t* b_next, cudaStream_t s) {
+    auto* const kernel = k_sort_small<kBatch, kHostIn, kBlocks, ITEMS>;
+    cudaLaunchAttribute cluster{};
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim = {kBlocks, 1, 1};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kBlocks);
+    cfg.blockDim = dim3(1024);
+    cfg.dynamicSmemBytes = (3u * 1024u * ITEMS + 32u * 256u) * sizeof(uint32_t);
+    cfg.stream = s;
+    cfg.attrs = &cluster;
+    cfg.numAttrs = 1;
+    static std::atomic<int> state[16];  // 0: not asked, 1: this cluster size, 2: eight blocks instead
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    int st = dev < 16 ? state[dev].load(std::memory_order_relaxed) : 0;
+    if (st == 0) {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+        if (e != cudaSuccess) return e;
+        st = 1;
+        if (kBlocks > 8) {
+            int clusters = 0;
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+                cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
+                cudaGetLastError();
+                st = 2;
+            }
+        }
+        if (dev < 16) state[dev].store(st, std::memory_order_relaxed);
+    }
+    if constexpr (kBlocks > 8) {
+        if (st == 2)
+            return sort_small_items<kBatch, kHostIn, 8, 2 * ITEMS>(L, pos, bits, passes, skeys, perm, scan, host3,
+                                                                   pos_out, aux, b_of_id, b_next, s);
+    }
+    return cudaLaunchKernelEx(&cfg, kernel, L, pos, bits, passes, skeys, perm, scan, host3, pos_out, aux, b_of_id, b_next);
+}
+
+template <bool kBatch, bool kHostIn>
+cudaError_t sort_small(const StepLaunch& L, const float4* pos, uint32_t* skeys, uint32_t* perm, uint32_t* scan,
+                       const float* host3, float4* pos_out, float4* aux, const uint32_t* b_of_id,
+                       uint32_t* b_next, cudaStream_t s) {
+    // At least 3 bits a digit: the kernel's four threads a digit then fill whole warps.
+    const int key_bits = key_bits_for(L.total - 1u), passes = (key_bits + 7) / 8;
+    const int bits = std::max(3, (key_bits + passes - 1) / passes);
+    if (L.total <= 8192u) return sort_small_items<kBatch, kHostIn, 8, 1>(L, pos, bits, passes, skeys, perm, scan, host3, pos_out, aux, b_of_id, b_next, s);
+    if (L.total <= 16384u) return sort_small_items<kBatch, kHostIn, 16, 1>(L, pos, bits, passes, skeys, perm, scan, host3, pos_out, aux, b_of_id, b_next, s);
+    if (L.total <= 32768u) return sort_small_items<kBatch, kHostIn, 16, 2>(L, pos, bits, passes, skeys, perm, scan, host3, pos_out, aux, b_of_id, b_next, s);
+    return sort_small_items<kBatch, kHostIn, 16, 4>(L, pos, bits, passes, skeys, perm, scan, host3, pos_out, aux, b_of_id, b_next, s);
+}
+}  // namespace
+
+cudaError_t launch_sort_small(const StepLaunch& L, const float4* pos, uint32_t* skeys, uint32_t* perm,
+                              uint32_t* cell_scan, cudaStream_t s, const float* host3, float4* pos_out,
+                              float4* aux, const uint32_t* b_of_id, uint32_t* b_next) {
+    if (L.total == 0) return cudaSuccess;
+    if (L.n_scenes > 1) return sort_small<true, false>(L, pos, skeys, perm, cell_scan, nullptr, nullptr, nullptr, nullptr, nullptr, s);
+    if (host3) return sort_small<false, true>(L, pos, skeys, perm, cell_scan, host3, pos_out, aux, b_of_id, b_next, s);
+    return sort_small<false, false>(L, pos, skeys, perm, cell_scan, nullptr, nullptr, nullptr, nullptr, nullptr, s);
+}
+
+cudaError_t launch_reorder(const StepLaunch& L, uint32_t n, const uint32_t* perm, const float4* pos_in,
+                           const float4* vel_in, float4* pos_out, float4* vel_out, const SkinLists& sk,
+                           cudaStream_t s) {
+    if (n == 0) return cudaSuccess;
+    k_reorder<<<(n + 127u) / 128u, 128, 0, s>>>(L, n, perm, pos_in, vel_in, pos_out, vel_out, sk.b_of_id, sk.xcur,
+                                                sk.x_build, sk.stale, sk.ctl, sk.wcount);
     return cudaGetLastError();
 }
 
