@@ -237,6 +237,10 @@ cudaError_t launch_sort(uint32_t n, const SortConfig& sc, const SortScratch& scr
                         uint32_t* keys, uint32_t* keys_alt, uint32_t* vals, uint32_t* vals_alt,
                         uint32_t** sorted_keys, uint32_t** sorted_perm, cudaStream_t s,
                         bool vals_given = false, const uint32_t* n_dev = nullptr);
+// One of its passes, from (kin, vin) into (kout, vout); vin NULL: the values are the indices.
+cudaError_t launch_sort_pass(uint32_t n, const SortConfig& sc, const SortScratch& scratch, int pass,
+                             const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout,
+                             const uint32_t* n_dev, cudaStream_t s);
 // cell_scan[k] = first sorted index with key >= k (k in [0, n]); gathers pos/vel by perm; zeroes
 // zero[0, zero_words) (the sort scratch, for the next substep); copies skeys to pkeys_out (the next
 // substep's previous sorted keys) when pkeys_out is not NULL. guess (n / 128 + 2 words, any
@@ -288,11 +292,14 @@ cudaError_t launch_force(const StepLaunch& L, const float4* pos, const float4* v
                          const uint32_t* nbr, const uint32_t* nbr_count, float4* pos_out,
                          float4* vel_out, float4* acc_out, const SkinLists& sk,
                          const KernelConfig& kc, cudaStream_t s, const HostOut& ho = HostOut{});
-// Stable in-place sort of (keys, items) with caller-provided temporaries (n words each) and
-// sort scratch (sort_scratch_words(sc) + 1 words, zeroed here); items become the permutation.
+// Stable in-place sort of (keys, items) with caller-provided temporaries (n words each; the second
+// pair, which spares an odd number of passes the copies back, may be NULL) and sort scratch
+// (sort_scratch_words(sc) words, zeroed here); items become the permutation. Error bits go to *err.
 int enqueue_sort_pairs(uint32_t* items, uint32_t* keys, uint32_t n, const SortConfig& sc,
-                       uint32_t* tmp_keys, uint32_t* tmp_items, uint32_t* scratch,
-                       cudaStream_t s);
+                       uint32_t* tmp_keys, uint32_t* tmp_items, uint32_t* tmp2_keys, uint32_t* tmp2_items,
+                       uint32_t* scratch, uint32_t* err, cudaStream_t s);
+// Device address, on the current device, of the error word that every pair sort reports through.
+int sort_status_address(uint32_t** out);
 // Scene-local spatial_offsets[k] = cell start - off, or n for empty keys (reference layout), for
 // the scene owning keys [off, off + n).
 cudaError_t launch_offsets(uint32_t n, uint32_t off, const uint32_t* cell_scan, uint32_t* offsets,

@@ -316,31 +316,47 @@ __device__ __forceinline__ uint32_t block_excl_scan256(uint32_t v, uint32_t* s_w
 constexpr uint32_t kLookbackSpinLimit = 1u << 20;
 
 // Decoupled look-back of tile `tile` for digit `bin`: sums the predecessors' published counts,
-// walking back until a tile with an inclusive prefix. A predecessor that has published nothing is
-// polled at most spin_limit times; then kErrLookbackTimeout is set in *err and the partial sum is
-// returned (the caller's scatter is guarded, and the host reports the error word).
+// walking back until a tile with an inclusive prefix. kLookbackWide predecessors are read at a
+// time: tiles that start together all begin with aggregates, and one word per L2 round trip makes
+// tile t wait about t / 2 of them (a 1M-pair sort with its offsets and reorders: 152 us reading one
+// at a time, 146 four, 148 eight, 159 sixteen). A predecessor that has published nothing is polled
+// at most spin_limit times; then kErrLookbackTimeout is set in *err and the partial sum is returned
+// (the caller's scatter is guarded, and the host reports the error word).
+constexpr int kLookbackWide = 4;
 __device__ __forceinline__ uint32_t lookback_exclusive(const uint32_t* status, int bins,
                                                        uint32_t tile, int bin, uint32_t spin_limit,
                                                        uint32_t* err) {
     uint32_t excl = 0u;
-    uint32_t t = tile - 1u;
+    uint32_t t = tile;  // predecessors below t are still to be summed
     uint32_t spins = 0u;
     while (true) {
-        const uint32_t s = ld_volatile(status + (size_t)t * bins + bin);
-        const uint32_t flag = s & ~kCountMask;
-        if (flag == 0u) {
+        uint32_t w[kLookbackWide];
+#pragma unroll
+        for (int u = 0; u < kLookbackWide; u++)
+            w[u] = (uint32_t)u < t ? ld_volatile(status + (size_t)(t - 1u - (uint32_t)u) * bins + bin) : 0u;
+        bool waiting = false;
+        uint32_t seen = 0u;
+#pragma unroll
+        for (int u = 0; u < kLookbackWide; u++) {
+            const uint32_t flag = w[u] & ~kCountMask;
+            if (waiting || (uint32_t)u >= t) continue;
+            if (flag == 0u) {
+                waiting = true;
+                continue;
+            }
+            excl += w[u] & kCountMask;
+            seen++;
+            if (flag == kFlagPrefix || (uint32_t)u + 1u == t) return excl;
+        }
+        t -= seen;
+        if (waiting) {
             if (++spins > spin_limit) {
                 atomicOr(err, kErrLookbackTimeout);
-                break;
+                return excl;
             }
-            __nanosleep(32);
-            continue;
+            if (seen == 0u) __nanosleep(32);
         }
-        excl += s & kCountMask;
-        if (flag == kFlagPrefix || t == 0u) break;
-        t--;
     }
-    return excl;
 }
 
 // Failure-detection self-test of the look-back wait: thread b plays tile 1 of digit b over a
@@ -379,6 +395,7 @@ __global__ void __launch_bounds__(BLOCK)
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const uint32_t mask = (uint32_t)bins - 1u;
+    const int bits = 32 - __clz((int)mask);
     if (tid == 0) s_tile = atomicAdd(counter, 1u);
     for (int e = tid; e < WARPS * kMaxSortBins; e += BLOCK) (&s_whist[0][0])[e] = 0u;
     // Global exclusive digit offsets of this pass.
@@ -402,7 +419,14 @@ __global__ void __launch_bounds__(BLOCK)
         const uint32_t idx = base + it * 32u + lane;
         const bool valid = idx < n;
         const uint32_t d = valid ? ((k[it] >> shift) & mask) : (uint32_t)bins;
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        // Lanes with the same digit, a ballot per bit (one more than a digit's: the invalid lanes'):
+        // eight independent votes take less than a match.any (4M pairs: 309 against 336 us).
+        uint32_t peers = 0xffffffffu;
+        for (int b = 0; b <= bits; b++) {
+            const bool bit = (d >> b) & 1u;
+            const uint32_t vote = __ballot_sync(0xffffffffu, bit);
+            peers &= bit ? vote : ~vote;
+        }
         const uint32_t pre = __popc(peers & lt_mask);
         uint32_t prev = 0u;
         if (valid) prev = s_whist[warp][d];
@@ -2747,10 +2771,21 @@ cudaError_t launch_merge(uint32_t n, const uint32_t* pkeys, const uint32_t* bits
 cudaError_t launch_digit_hist(const uint32_t* keys, uint32_t n, const SortConfig& sc,
                               uint32_t* ghist, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    uint32_t blocks = (n + 255u) / 256u;
-    if (blocks > 152u * 8u) blocks = 152u * 8u;
+    // Few blocks: each adds its passes x bins counters to the global ones with atomics (1M keys: 15 us
+    // with 1,216 blocks, 6 with 304).
+    uint32_t blocks = (n + 1023u) / 1024u;
+    if (blocks > 152u * 2u) blocks = 152u * 2u;
     k_digit_hist<<<blocks, 256, 0, s>>>(keys, n, sc.passes, sc.digit_bits, ghist);
     return cudaGetLastError();
+}
+
+cudaError_t launch_sort_pass(uint32_t n, const SortConfig& sc, const SortScratch& scr, int pass,
+                             const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout,
+                             const uint32_t* n_dev, cudaStream_t s) {
+    const int items = sc.tile / kSortBlock;
+    if (items == 8) return launch_onesweep_t<8>(n, sc, scr, pass, kin, vin, kout, vout, n_dev, s);
+    if (items == 12) return launch_onesweep_t<12>(n, sc, scr, pass, kin, vin, kout, vout, n_dev, s);
+    return launch_onesweep_t<16>(n, sc, scr, pass, kin, vin, kout, vout, n_dev, s);
 }
 
 cudaError_t launch_sort(uint32_t n, const SortConfig& sc, const SortScratch& scr, uint32_t* keys,
@@ -2762,14 +2797,7 @@ cudaError_t launch_sort(uint32_t n, const SortConfig& sc, const SortScratch& scr
     uint32_t* kout = keys_alt;
     uint32_t* vout = vals_alt;
     for (int pass = 0; pass < sc.passes; pass++) {
-        cudaError_t e;
-        const int items = sc.tile / kSortBlock;
-        if (items == 8)
-            e = launch_onesweep_t<8>(n, sc, scr, pass, kin, vin, kout, vout, n_dev, s);
-        else if (items == 12)
-            e = launch_onesweep_t<12>(n, sc, scr, pass, kin, vin, kout, vout, n_dev, s);
-        else
-            e = launch_onesweep_t<16>(n, sc, scr, pass, kin, vin, kout, vout, n_dev, s);
+        const cudaError_t e = launch_sort_pass(n, sc, scr, pass, kin, vin, kout, vout, n_dev, s);
         if (e != cudaSuccess) return e;
         kin = kout;
         vin = vout;

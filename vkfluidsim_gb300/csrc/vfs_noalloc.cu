@@ -19,7 +19,7 @@ constexpr uint32_t kNoAllocPairs = VFS_SORT_NOALLOC_MAX_PAIRS;
 constexpr uint32_t kNoAllocTile = 256u * 16u;  // onesweep tile of make_sort_config(.., 8, 16, ..)
 constexpr uint32_t kNoAllocTiles = (kNoAllocPairs + kNoAllocTile - 1u) / kNoAllocTile;
 // Digit histograms + tile counters + look-back status words + the key pass's words
-// (unused by a pair sort, but part of sort_scratch_words) + the error word, for any key width.
+// (unused by a pair sort, but part of sort_scratch_words), for any key width (one word more than used).
 constexpr size_t kNoAllocSortWords = (size_t)kMaxSortPasses * kMaxSortBins + kMaxSortPasses +
                                      (size_t)kMaxSortPasses * kNoAllocTiles * kMaxSortBins + 2 +
                                      (kNoAllocPairs + 1023u) / 1024u + 1;
@@ -65,12 +65,15 @@ extern "C" int vfs_sort_pairs_noalloc(uint32_t* items, uint32_t* keys, uint32_t 
                                           std::to_string(kNoAllocPairs) + " pairs (got " +
                                           std::to_string(n) + ")");
     const SortConfig sc = make_sort_config(n, 8, 16, key_bits_for(max_value));
-    if (sort_scratch_words(sc) + 1 > kNoAllocSortWords)
+    if (sort_scratch_words(sc) > kNoAllocSortWords)
         return fail(VFS_ERR_CAPACITY, "sort configuration exceeds the static scratch");
     uint32_t* base = nullptr;
     const int rc = scratch_address(&base);
     if (rc) return rc;
-    // enqueue_sort_pairs zeroes the histogram / status / error words the previous call left.
-    return enqueue_sort_pairs(items, keys, n, sc, base, base + kNoAllocPairs,
-                              base + 2 * (size_t)kNoAllocPairs, (cudaStream_t)stream);
+    uint32_t* err = nullptr;
+    const int rs = sort_status_address(&err);
+    if (rs) return rs;
+    // enqueue_sort_pairs zeroes the histogram / status words the previous call left.
+    return enqueue_sort_pairs(items, keys, n, sc, base, base + kNoAllocPairs, nullptr, nullptr,
+                              base + 2 * (size_t)kNoAllocPairs, err, (cudaStream_t)stream);
 }

@@ -5,6 +5,7 @@
 // They run on the caller's stream and return without synchronising it.
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <string>
 
 #include "vfs_cuda.h"
@@ -48,38 +49,68 @@ __global__ void k_reorder_float3(const uint32_t* __restrict__ idx, const float* 
     dst[3 * (size_t)i + 2] = src[3 * (size_t)s + 2];
 }
 
-// Error bits of every pair sort on this device since the last vfs_sort_pairs_status: each sort's
-// own error word (its look-back timeouts) is OR-ed in after its passes. A fixed device word, so
-// the no-allocation sort can report through it too.
+// Error bits of every pair sort on this device since the last vfs_sort_pairs_status (look-back
+// timeouts). A fixed device word, so the no-allocation sort can report through it too.
 __device__ uint32_t g_sort_status;
 
-__global__ void k_sort_status_accumulate(const uint32_t* __restrict__ err) {
-    const uint32_t e = *err;
-    if (e) atomicOr(&g_sort_status, e);
-}
+constexpr int kMaxDevices = 64;
+std::mutex g_status_mu;
+uint32_t* g_status_addr[kMaxDevices] = {};
 
 }  // namespace
 
-// Enqueues a stable sort of (keys, index) with caller-provided scratch: tmp_keys / tmp_items
-// (n words each) and `scratch` of sort_scratch_words(sc) words plus one error word.
+int sort_status_address(uint32_t** out) {
+    int dev = 0;
+    VFS_PRIM_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kMaxDevices) return fail(VFS_ERR_CAPACITY, "device ordinal beyond 63");
+    std::lock_guard<std::mutex> lock(g_status_mu);
+    if (!g_status_addr[dev]) {
+        void* p = nullptr;
+        VFS_PRIM_TRY(cudaGetSymbolAddress(&p, g_sort_status));
+        g_status_addr[dev] = static_cast<uint32_t*>(p);
+    }
+    *out = g_status_addr[dev];
+    return VFS_OK;
+}
+
 int enqueue_sort_pairs(uint32_t* items, uint32_t* keys, uint32_t n, const SortConfig& sc,
-                       uint32_t* tmp_keys, uint32_t* tmp_items, uint32_t* scratch,
-                       cudaStream_t s) {
-    SortScratch scr;
+                       uint32_t* tmp_keys, uint32_t* tmp_items, uint32_t* tmp2_keys, uint32_t* tmp2_items,
+                       uint32_t* scratch, uint32_t* err, cudaStream_t s) {
+    SortScratch scr{};
     scr.ghist = scratch;
     scr.counters = scratch + (size_t)sc.passes * sc.bins;
     scr.status = scr.counters + sc.passes;
-    scr.err = scratch + sort_scratch_words(sc);
-    VFS_PRIM_TRY(cudaMemsetAsync(scratch, 0, (sort_scratch_words(sc) + 1) * sizeof(uint32_t), s));
+    scr.err = err;
+    VFS_PRIM_TRY(cudaMemsetAsync(scratch, 0, sort_scratch_words(sc) * sizeof(uint32_t), s));
     VFS_PRIM_TRY(launch_digit_hist(keys, n, sc, scr.ghist, s));
-    uint32_t* sk = nullptr;
-    uint32_t* sp = nullptr;
-    VFS_PRIM_TRY(launch_sort(n, sc, scr, keys, tmp_keys, items, tmp_items, &sk, &sp, s));
-    if (sk != keys) VFS_PRIM_TRY(cudaMemcpyAsync(keys, sk, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
-    if (sp != items)
-        VFS_PRIM_TRY(cudaMemcpyAsync(items, sp, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
-    k_sort_status_accumulate<<<1, 1, 0, s>>>(scr.err);
-    VFS_PRIM_TRY(cudaGetLastError());
+    // The passes go from the caller's arrays through the temporaries and back; an odd number of them
+    // through both pairs, or, without a second one, out of the temporaries by copies.
+    const uint32_t *kin = keys, *vin = nullptr;  // the first pass's values are the indices
+    const bool two = tmp2_keys != nullptr;
+    for (int pass = 0; pass < sc.passes; pass++) {
+        const int left = sc.passes - 1 - pass;  // passes after this one
+        uint32_t *kout, *vout;
+        if (left == 0 && kin != keys) {
+            kout = keys;
+            vout = items;
+        } else if (two && kin == tmp_keys) {
+            kout = tmp2_keys;
+            vout = tmp2_items;
+        } else if (!two && kin == tmp_keys) {
+            kout = keys;
+            vout = items;
+        } else {
+            kout = tmp_keys;
+            vout = tmp_items;
+        }
+        VFS_PRIM_TRY(launch_sort_pass(n, sc, scr, pass, kin, vin, kout, vout, nullptr, s));
+        kin = kout;
+        vin = vout;
+    }
+    if (kin != keys) {
+        VFS_PRIM_TRY(cudaMemcpyAsync(keys, kin, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
+        VFS_PRIM_TRY(cudaMemcpyAsync(items, vin, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
+    }
     return VFS_OK;
 }
 
@@ -95,15 +126,17 @@ int vfs_sort_pairs(uint32_t* items, uint32_t* keys, uint32_t n, uint32_t max_val
     if (n > vfs::kMaxParticles) return fail(VFS_ERR_CAPACITY, "n must be <= 2^30");
     cudaStream_t s = (cudaStream_t)stream;
     const vfs::SortConfig sc = vfs::make_sort_config(n, 8, 16, vfs::key_bits_for(max_value));
-    const size_t words = vfs::sort_scratch_words(sc) + 1;
-    uint32_t *tk = nullptr, *ti = nullptr, *scratch = nullptr;
-    VFS_PRIM_TRY(cudaMallocAsync(&tk, (size_t)n * 4, s));
-    VFS_PRIM_TRY(cudaMallocAsync(&ti, (size_t)n * 4, s));
-    VFS_PRIM_TRY(cudaMallocAsync(&scratch, words * 4, s));
-    const int rc = vfs::enqueue_sort_pairs(items, keys, n, sc, tk, ti, scratch, s);
-    cudaFreeAsync(tk, s);
-    cudaFreeAsync(ti, s);
-    cudaFreeAsync(scratch, s);
+    uint32_t* err = nullptr;
+    int rc = vfs::sort_status_address(&err);
+    if (rc) return rc;
+    // One allocation: the temporaries (two pairs from three passes on), then the sort scratch.
+    const size_t pairs = sc.passes > 2 ? 2 : 1, stride = ((size_t)n + 63) & ~(size_t)63;
+    uint32_t* mem = nullptr;
+    VFS_PRIM_TRY(cudaMallocAsync(&mem, (2 * pairs * stride + vfs::sort_scratch_words(sc)) * 4, s));
+    uint32_t* const two = pairs > 1 ? mem + 2 * stride : nullptr;
+    rc = vfs::enqueue_sort_pairs(items, keys, n, sc, mem, mem + stride, two, two ? two + stride : nullptr,
+                                 mem + 2 * pairs * stride, err, s);
+    cudaFreeAsync(mem, s);
     return rc;
 }
 
