@@ -28,7 +28,7 @@ namespace vfs {
 namespace {
 
 constexpr uint32_t kErrAdjointOverflow = 2u;  // a neighbour list longer than its capacity
-constexpr int kAdjLanes = 4;                     // lanes sharing one particle's neighbour list
+constexpr int kDensBatch = 4;  // neighbours a lane of k_adj_density gathers at a time
 
 __device__ __forceinline__ float3 f3(const float4& a) { return make_float3(a.x, a.y, a.z); }
 __device__ __forceinline__ float dot3(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
@@ -185,17 +185,17 @@ __device__ float3 boundary_adjoint(const SceneParams& p, float3 x, float psi_bar
 
 struct AdjBuffers {
     const float4* pos;   // x' (sorted positions of the substep)
-    const float4* vel;   // v'
+    const float4* rec;   // 2 per particle: (x', p/rho^2), (v', m/max(rho, 1e-6)), the force pass's records
     const float4* aux;   // (pd, mr, rho, pb)
     const float4* bnd;   // (G, Psi)
     const uint32_t* nbr;
     const uint32_t* nbr_count;
     float4* xbar;        // accumulates d L / d x' (sorted order)
     float4* vbar;        // accumulates d L / d v'
-    float4* abar;        // d L / d a
+    float4* abar;        // d L / d a, and the neighbour word (nbr_count) in w
     float2* pmbar;       // (d L / d pd, d L / d mr)
     float* pbbar;
-    float* rhobar;
+    float4* xr;          // x' and d L / d rho
     float4* gbar;        // d L / d G
     double* dparams;     // [d nu, d k]
     uint32_t* err;
@@ -210,7 +210,7 @@ __global__ void k_adj_integrate(SceneParams p, uint32_t n, const float4* __restr
     const float vx = vo.x + p.dt * xo.x, vy = vo.y + p.dt * xo.y, vz = vo.z + p.dt * xo.z;
     B.xbar[i] = make_float4(xo.x, xo.y, xo.z, 0.f);
     B.vbar[i] = make_float4(vx, vy, vz, 0.f);
-    B.abar[i] = make_float4(p.dt * vx, p.dt * vy, p.dt * vz, 0.f);
+    B.abar[i] = make_float4(p.dt * vx, p.dt * vy, p.dt * vz, __uint_as_float(__ldg(B.nbr_count + i)));
     B.pmbar[i] = make_float2(0.f, 0.f);
 }
 
@@ -244,6 +244,15 @@ __device__ __forceinline__ float3 group_sum3(float3 v) {
     return make_float3(group_sum<kLanes>(v.x), group_sum<kLanes>(v.y), group_sum<kLanes>(v.z));
 }
 
+// A 32-byte force record in one 256-bit load, as the force pass reads it.
+__device__ __forceinline__ void load_record(const float4* __restrict__ rec, uint32_t j, float4& a,
+                                            float4& b) {
+    const float4* q = rec + 2 * (size_t)j;
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(q));
+}
+
 // Adjoint of the force pass: pressure, viscosity, boundary pressure and wall terms.
 //
 // Pair (j, i) of j's force, with x = x_j - x_i, v = v_j - v_i, n = x / r, c_j = d L / d a_j:
@@ -255,6 +264,11 @@ __device__ __forceinline__ float3 group_sum3(float3 v) {
 // of pair (i, j) that falls on j, which is the own-pair expression evaluated at c_j - c_i (pressure)
 // and s_i c_j - s_j c_i (viscosity). Otherwise i's part is left to i, which scatters its own
 // pair's reverse to j with atomics (c_i counted as zero here).
+// Bound by the gathers, each the latency of an L2 hit, of which a neighbour once cost five (position,
+// velocity, pressures, word, adjoint). The force pass's own record holds the first three and the
+// adjoint's spare component the word, so it is two now, and the next index is fetched under them:
+// 38.0 -> 28.6 us at 65,536 particles (batches of two and three neighbours: 31.6 and 30.9 against
+// 31.3 for one, all with four lanes).
 template <int kLanes>
 __global__ void __launch_bounds__(128) k_adj_force(SceneParams p, uint32_t n, AdjBuffers B) {
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -264,29 +278,41 @@ __global__ void __launch_bounds__(128) k_adj_force(SceneParams p, uint32_t n, Ad
     float3 xj = xb, cj = xb;
     float pdj = 0.f, pbj = 0.f;
     if (j < n) {
-        xj = f3(B.pos[j]);
-        const float3 vj = f3(B.vel[j]);
-        const float4 aj = B.aux[j];
-        cj = f3(B.abar[j]);
-        pdj = aj.x;
-        pbj = aj.w;
-        const float s_j = p.visc_scale * aj.y;
-        const uint32_t cnt = B.nbr_count[j];
+        float4 r0, r1;
+        load_record(B.rec, j, r0, r1);
+        xj = f3(r0);
+        const float3 vj = f3(r1);
+        const float4 c4 = B.abar[j];
+        cj = f3(c4);
+        pdj = r0.w;
+        pbj = B.aux[j].w;
+        const float s_j = p.visc_scale * r1.w;
+        const uint32_t cnt = __float_as_uint(c4.w);
         const bool dj = (cnt & kNbrDistinct) != 0u;
         if (lane == 0 && (cnt & kNbrCountMask) > p.nbr_cap) atomicOr(B.err, kErrAdjointOverflow);
         const uint32_t listed = min(cnt & kNbrCountMask, p.nbr_cap);
+        // Two gathers a neighbour (its 32-byte force record, and its adjoint with its word), the
+        // next neighbour's index a round ahead.
+        const uint32_t* nl = B.nbr + j + (size_t)lane * n;
+        const size_t step = (size_t)kLanes * n;
+        uint32_t next = lane < listed ? __ldg(nl) : 0u;
         for (uint32_t k = lane; k < listed; k += kLanes) {
-            const uint32_t i = B.nbr[(size_t)k * n + j];
-            const float3 x = xj - f3(B.pos[i]);
+            const uint32_t i = next;
+            float4 q0, q1;
+            load_record(B.rec, i, q0, q1);
+            const float4 c4 = B.abar[i];
+            nl += step;
+            if (k + kLanes < listed) next = __ldg(nl);
+            const float3 x = xj - f3(q0);
             const float r2 = dot3(x, x);
             if (!(r2 > 1e-18f)) continue;
             const float inv_r = rsqrtf(r2);
             const float r = r2 * inv_r;
-            const float3 v = vj - f3(B.vel[i]);
-            const float2 ai = *reinterpret_cast<const float2*>(B.aux + i);  // (pd_i, mr_i)
-            const uint32_t ci_word = B.nbr_count[i];
+            const float3 v = vj - f3(q1);
+            const float2 ai = make_float2(q0.w, q1.w);  // (pd_i, mr_i)
+            const uint32_t ci_word = __float_as_uint(c4.w);
             const bool gather = dj && (ci_word & kNbrDistinct) != 0u && nbr_cells_adjacent(cnt, ci_word);
-            const float3 ci = gather ? f3(B.abar[i]) : make_float3(0.f, 0.f, 0.f);
+            const float3 ci = gather ? f3(c4) : make_float3(0.f, 0.f, 0.f);
             float gw, dgw;
             gw_and_deriv(p, r, gw, dgw);
             const float inv_den = 1.0f / (r2 + p.visc_eps);
@@ -359,7 +385,8 @@ __global__ void k_adj_eos(SceneParams p, uint32_t n, AdjBuffers B) {
         float rb = pdb * (dp - 2.0f * pr * inv_rho) * inv_rho * inv_rho;
         rb += pbb * dp * inv_rho0 * inv_rho0;
         if (rho > 1e-6f) rb -= mrb * p.mass * inv_rho * inv_rho;
-        B.rhobar[i] = rb;
+        const float4 x = B.pos[i];
+        B.xr[i] = make_float4(x.x, x.y, x.z, rb);
         dk = (pdb * inv_rho * inv_rho + pbb * inv_rho0 * inv_rho0) * f;
     }
     block_add_double((double)dk, &B.dparams[1]);
@@ -367,6 +394,8 @@ __global__ void k_adj_eos(SceneParams p, uint32_t n, AdjBuffers B) {
 
 // Adjoint of the density sum and of the volume-map terms, the list split over kLanes lanes as in
 // k_adj_force; the reverse half of each pair is gathered or scattered under the same rule.
+// Position and d L / d rho travel together in one gather; four neighbours' gathers are in flight a
+// lane (27.4 -> 12.6 us at 65,536 particles; with four lanes 15.7 for two in flight, 13.9 for four).
 template <int kLanes>
 __global__ void __launch_bounds__(128) k_adj_density(SceneParams p, uint32_t n, AdjBuffers B) {
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -374,26 +403,49 @@ __global__ void __launch_bounds__(128) k_adj_density(SceneParams p, uint32_t n, 
     float3 xb = make_float3(0.f, 0.f, 0.f), xj = xb;
     float rbj = 0.0f;
     if (j < n) {
-        xj = f3(B.pos[j]);
-        rbj = B.rhobar[j];
+        const float4 xr = B.xr[j];
+        xj = f3(xr);
+        rbj = xr.w;
         const uint32_t cnt = B.nbr_count[j];
         const bool dj = (cnt & kNbrDistinct) != 0u;
         const uint32_t listed = min(cnt & kNbrCountMask, p.nbr_cap);
-        for (uint32_t k = lane; k < listed; k += kLanes) {
-            const uint32_t i = B.nbr[(size_t)k * n + j];
-            const float3 x = xj - f3(B.pos[i]);
-            const float r2 = dot3(x, x);
-            if (!(r2 > 1e-18f)) continue;
-            const float inv_r = rsqrtf(r2);
-            const float w = p.mass * dW_dr(p, r2 * inv_r) * inv_r;
-            const uint32_t ci_word = B.nbr_count[i];
-            const bool gather = dj && (ci_word & kNbrDistinct) != 0u && nbr_cells_adjacent(cnt, ci_word);
-            // Own pair: d rho_j / d x_j = m W'(r) n, d rho_j / d x_i = -m W'(r) n.
-            if (gather)
-                xb = xb + ((rbj + B.rhobar[i]) * w) * x;  // with i's pair (i, j): d rho_i / d x_j
-            else {
-                xb = xb + (rbj * w) * x;
-                if (rbj != 0.0f) atomic_add3(&B.xbar[i], (-rbj * w) * x);
+        // kDensBatch neighbours' gathers in flight, and the next batch's indices.
+        const uint32_t* nl = B.nbr + j + (size_t)lane * n;
+        const size_t step = (size_t)kLanes * n;
+        uint32_t in[kDensBatch];
+#pragma unroll
+        for (int u = 0; u < kDensBatch; u++) in[u] = lane + u * kLanes < listed ? __ldg(nl + u * step) : j;
+        for (uint32_t k0 = lane; k0 < listed; k0 += kDensBatch * kLanes) {
+            nl += kDensBatch * step;
+            float4 xis[kDensBatch];
+            uint32_t words[kDensBatch], is[kDensBatch];
+#pragma unroll
+            for (int u = 0; u < kDensBatch; u++) {
+                is[u] = in[u];
+                xis[u] = B.xr[is[u]];
+                words[u] = B.nbr_count[is[u]];
+            }
+#pragma unroll
+            for (int u = 0; u < kDensBatch; u++)
+                in[u] = k0 + (kDensBatch + u) * kLanes < listed ? __ldg(nl + u * step) : j;
+#pragma unroll
+            for (int u = 0; u < kDensBatch; u++) {
+                const uint32_t i = is[u];  // (j itself past the list's end: r2 is 0)
+                const float4 xi = xis[u];
+                const float3 x = xj - f3(xi);
+                const float r2 = dot3(x, x);
+                if (!(r2 > 1e-18f)) continue;
+                const float inv_r = rsqrtf(r2);
+                const float w = p.mass * dW_dr(p, r2 * inv_r) * inv_r;
+                const uint32_t ci_word = words[u];
+                const bool gather = dj && (ci_word & kNbrDistinct) != 0u && nbr_cells_adjacent(cnt, ci_word);
+                // Own pair: d rho_j / d x_j = m W'(r) n, d rho_j / d x_i = -m W'(r) n.
+                if (gather)
+                    xb = xb + ((rbj + xi.w) * w) * x;  // with i's pair (i, j): d rho_i / d x_j
+                else {
+                    xb = xb + (rbj * w) * x;
+                    if (rbj != 0.0f) atomic_add3(&B.xbar[i], (-rbj * w) * x);
+                }
             }
         }
     }
@@ -457,11 +509,11 @@ struct Rollout {
     std::vector<float4*> ck_pos, ck_vel;  // state before steps 0, every, 2 every, ...
     float4 *fin_pos = nullptr, *fin_vel = nullptr;  // state after the last step
     // One segment of per-substep records.
-    std::vector<float4*> s_pos, s_vel, s_aux, s_bnd;
+    std::vector<float4*> s_pos, s_vel, s_aux, s_bnd, s_rec;
     std::vector<uint32_t*> s_perm, s_nbr, s_cnt;
-    float4 *xbar = nullptr, *vbar = nullptr, *xs = nullptr, *vs = nullptr, *abar = nullptr, *gbar = nullptr;
+    float4 *xbar = nullptr, *vbar = nullptr, *xs = nullptr, *vs = nullptr, *abar = nullptr, *gbar = nullptr, *xr = nullptr;
     float2* pmbar = nullptr;
-    float *pbbar = nullptr, *rhobar = nullptr;
+    float* pbbar = nullptr;
     float* host_io = nullptr;  // 3N floats on the device for host transfers
     double* dparams = nullptr;
     bool forward_done = false;
@@ -477,6 +529,7 @@ struct Rollout {
         for (auto* p : s_vel) cudaFree(p);
         for (auto* p : s_aux) cudaFree(p);
         for (auto* p : s_bnd) cudaFree(p);
+        for (auto* p : s_rec) cudaFree(p);
         for (auto* p : s_perm) cudaFree(p);
         for (auto* p : s_nbr) cudaFree(p);
         for (auto* p : s_cnt) cudaFree(p);
@@ -490,7 +543,7 @@ struct Rollout {
         cudaFree(gbar);
         cudaFree(pmbar);
         cudaFree(pbbar);
-        cudaFree(rhobar);
+        cudaFree(xr);
         cudaFree(host_io);
         cudaFree(dparams);
     }
@@ -513,6 +566,7 @@ struct Rollout {
         s_vel.resize(seg, nullptr);
         s_aux.resize(seg, nullptr);
         s_bnd.resize(seg, nullptr);
+        s_rec.resize(seg, nullptr);
         s_perm.resize(seg, nullptr);
         s_nbr.resize(seg, nullptr);
         s_cnt.resize(seg, nullptr);
@@ -521,13 +575,14 @@ struct Rollout {
             VFS_ADJ_TRY(cudaMalloc(&s_vel[t], N * sizeof(float4)));
             VFS_ADJ_TRY(cudaMalloc(&s_aux[t], N * sizeof(float4)));
             VFS_ADJ_TRY(cudaMalloc(&s_bnd[t], N * sizeof(float4)));
+            VFS_ADJ_TRY(cudaMalloc(&s_rec[t], 2 * N * sizeof(float4)));
             VFS_ADJ_TRY(cudaMalloc(&s_perm[t], N * 4));
             VFS_ADJ_TRY(cudaMalloc(&s_nbr[t], N * (size_t)cap * 4));
             VFS_ADJ_TRY(cudaMalloc(&s_cnt[t], N * 4));
         }
-        for (float4** b : {&fin_pos, &fin_vel, &xbar, &vbar, &xs, &vs, &abar, &gbar})
+        for (float4** b : {&fin_pos, &fin_vel, &xbar, &vbar, &xs, &vs, &abar, &gbar, &xr})
             VFS_ADJ_TRY(cudaMalloc(b, N * sizeof(float4)));
-        for (float** b : {&pbbar, &rhobar}) VFS_ADJ_TRY(cudaMalloc(b, N * 4));
+        VFS_ADJ_TRY(cudaMalloc(&pbbar, N * 4));
         VFS_ADJ_TRY(cudaMalloc(&pmbar, N * sizeof(float2)));
         VFS_ADJ_TRY(cudaMalloc(&host_io, N * 12));
         VFS_ADJ_TRY(cudaMalloc(&dparams, 2 * sizeof(double)));
@@ -583,6 +638,7 @@ struct Rollout {
             return fail(VFS_ERR_INVALID_ARGUMENT, "the model's neighbour capacity changed after the rollout was created");
         float4* own_aux = m->aux;
         float4* own_bnd = m->bnd;
+        float4* own_rec = m->rec;
         uint32_t* own_nbr = m->nbr;
         uint32_t* own_cnt = m->nbr_count;
         const int o = 1 - m->cur;
@@ -592,6 +648,7 @@ struct Rollout {
         for (int t = 0; t < len && rc == VFS_OK; t++) {
             m->aux = s_aux[t];
             m->bnd = s_bnd[t];
+            m->rec = s_rec[t];
             m->nbr = s_nbr[t];
             m->nbr_count = s_cnt[t];
             m->pos[o] = s_pos[t];
@@ -605,6 +662,7 @@ struct Rollout {
         }
         m->aux = own_aux;
         m->bnd = own_bnd;
+        m->rec = own_rec;
         m->nbr = own_nbr;
         m->nbr_count = own_cnt;
         m->pos[o] = own_pos;
@@ -651,7 +709,7 @@ struct Rollout {
         cudaStream_t s = m->stream;
         AdjBuffers B;
         B.pos = s_pos[t];
-        B.vel = s_vel[t];
+        B.rec = s_rec[t];
         B.aux = s_aux[t];
         B.bnd = s_bnd[t];
         B.nbr = s_nbr[t];
@@ -661,16 +719,27 @@ struct Rollout {
         B.abar = abar;
         B.pmbar = pmbar;
         B.pbbar = pbbar;
-        B.rhobar = rhobar;
+        B.xr = xr;
         B.gbar = gbar;
         B.dparams = dparams;
         B.err = m->err;
         const unsigned g256 = (n + 255) / 256;
         k_adj_integrate<<<g256, 256, 0, s>>>(p, n, xbar, vbar, B);
-        const unsigned gl = (unsigned)(((size_t)n * kAdjLanes + 127) / 128);
-        k_adj_force<kAdjLanes><<<gl, 128, 0, s>>>(p, n, B);
+        // Lanes sharing one particle's list: two where that fills the GPU (65,536 particles: force 28.6
+        // us, density 12.6; four 31.3 and 13.9, eight 35.6 and 17.2), four below, where each lane's
+        // chain of gathers is the time (24-substep gradients, four against two lanes: 4,000 particles
+        // 2.58 ms against 2.76, 32,000 3.78 against 3.92, 48,000 4.14 against 4.05).
+        const bool wide = n < 40960u;
+        const unsigned gl = (unsigned)(((size_t)n * (wide ? 4 : 2) + 127) / 128);
+        if (wide)
+            k_adj_force<4><<<gl, 128, 0, s>>>(p, n, B);
+        else
+            k_adj_force<2><<<gl, 128, 0, s>>>(p, n, B);
         k_adj_eos<<<g256, 256, 0, s>>>(p, n, B);
-        k_adj_density<kAdjLanes><<<gl, 128, 0, s>>>(p, n, B);
+        if (wide)
+            k_adj_density<4><<<gl, 128, 0, s>>>(p, n, B);
+        else
+            k_adj_density<2><<<gl, 128, 0, s>>>(p, n, B);
         k_adj_unsort<<<g256, 256, 0, s>>>(n, s_perm[t], xs, vs, xbar, vbar);
         VFS_ADJ_TRY(cudaGetLastError());
         return VFS_OK;
