@@ -184,7 +184,6 @@ __device__ float3 boundary_adjoint(const SceneParams& p, float3 x, float psi_bar
 // ---- the reverse substep, one thread per sorted particle ----
 
 struct AdjBuffers {
-    const float4* pos;   // x' (sorted positions of the substep)
     const float4* rec;   // 2 per particle: (x', p/rho^2), (v', m/max(rho, 1e-6)), the force pass's records
     const float4* aux;   // (pd, mr, rho, pb)
     const float4* bnd;   // (G, Psi)
@@ -289,20 +288,18 @@ __global__ void __launch_bounds__(128) k_adj_force(SceneParams p, uint32_t n, Ad
         const float s_j = p.visc_scale * r1.w;
         const uint32_t cnt = __float_as_uint(c4.w);
         const bool dj = (cnt & kNbrDistinct) != 0u;
-        if (lane == 0 && (cnt & kNbrCountMask) > p.nbr_cap) atomicOr(B.err, kErrAdjointOverflow);
-        const uint32_t listed = min(cnt & kNbrCountMask, p.nbr_cap);
+        // (An overflowed list is truncated, or in part never written: an error, and not read.)
+        const uint32_t all = cnt & kNbrCountMask, listed = all > p.nbr_cap ? 0u : all;
+        if (lane == 0 && all > p.nbr_cap) atomicOr(B.err, kErrAdjointOverflow);
         // Two gathers a neighbour (its 32-byte force record, and its adjoint with its word), the
         // next neighbour's index a round ahead.
-        const uint32_t* nl = B.nbr + j + (size_t)lane * n;
-        const size_t step = (size_t)kLanes * n;
-        uint32_t next = lane < listed ? __ldg(nl) : 0u;
+        uint32_t next = lane < listed ? __ldg(B.nbr + nbr_word_at(lane, n, j)) : 0u;
         for (uint32_t k = lane; k < listed; k += kLanes) {
             const uint32_t i = next;
             float4 q0, q1;
             load_record(B.rec, i, q0, q1);
             const float4 c4 = B.abar[i];
-            nl += step;
-            if (k + kLanes < listed) next = __ldg(nl);
+            if (k + kLanes < listed) next = __ldg(B.nbr + nbr_word_at(k + kLanes, n, j));
             const float3 x = xj - f3(q0);
             const float r2 = dot3(x, x);
             if (!(r2 > 1e-18f)) continue;
@@ -385,7 +382,7 @@ __global__ void k_adj_eos(SceneParams p, uint32_t n, AdjBuffers B) {
         float rb = pdb * (dp - 2.0f * pr * inv_rho) * inv_rho * inv_rho;
         rb += pbb * dp * inv_rho0 * inv_rho0;
         if (rho > 1e-6f) rb -= mrb * p.mass * inv_rho * inv_rho;
-        const float4 x = B.pos[i];
+        const float4 x = B.rec[2 * (size_t)i];
         B.xr[i] = make_float4(x.x, x.y, x.z, rb);
         dk = (pdb * inv_rho * inv_rho + pbb * inv_rho0 * inv_rho0) * f;
     }
@@ -408,15 +405,13 @@ __global__ void __launch_bounds__(128) k_adj_density(SceneParams p, uint32_t n, 
         rbj = xr.w;
         const uint32_t cnt = B.nbr_count[j];
         const bool dj = (cnt & kNbrDistinct) != 0u;
-        const uint32_t listed = min(cnt & kNbrCountMask, p.nbr_cap);
+        const uint32_t all = cnt & kNbrCountMask, listed = all > p.nbr_cap ? 0u : all;
         // kDensBatch neighbours' gathers in flight, and the next batch's indices.
-        const uint32_t* nl = B.nbr + j + (size_t)lane * n;
-        const size_t step = (size_t)kLanes * n;
         uint32_t in[kDensBatch];
 #pragma unroll
-        for (int u = 0; u < kDensBatch; u++) in[u] = lane + u * kLanes < listed ? __ldg(nl + u * step) : j;
+        for (int u = 0; u < kDensBatch; u++)
+            in[u] = lane + u * kLanes < listed ? __ldg(B.nbr + nbr_word_at(lane + u * kLanes, n, j)) : j;
         for (uint32_t k0 = lane; k0 < listed; k0 += kDensBatch * kLanes) {
-            nl += kDensBatch * step;
             float4 xis[kDensBatch];
             uint32_t words[kDensBatch], is[kDensBatch];
 #pragma unroll
@@ -426,8 +421,10 @@ __global__ void __launch_bounds__(128) k_adj_density(SceneParams p, uint32_t n, 
                 words[u] = B.nbr_count[is[u]];
             }
 #pragma unroll
-            for (int u = 0; u < kDensBatch; u++)
-                in[u] = k0 + (kDensBatch + u) * kLanes < listed ? __ldg(nl + u * step) : j;
+            for (int u = 0; u < kDensBatch; u++) {
+                const uint32_t k = k0 + (kDensBatch + u) * kLanes;
+                in[u] = k < listed ? __ldg(B.nbr + nbr_word_at(k, n, j)) : j;
+            }
 #pragma unroll
             for (int u = 0; u < kDensBatch; u++) {
                 const uint32_t i = is[u];  // (j itself past the list's end: r2 is 0)
@@ -509,7 +506,7 @@ struct Rollout {
     std::vector<float4*> ck_pos, ck_vel;  // state before steps 0, every, 2 every, ...
     float4 *fin_pos = nullptr, *fin_vel = nullptr;  // state after the last step
     // One segment of per-substep records.
-    std::vector<float4*> s_pos, s_vel, s_aux, s_bnd, s_rec;
+    std::vector<float4*> s_aux, s_bnd, s_rec;
     std::vector<uint32_t*> s_perm, s_nbr, s_cnt;
     float4 *xbar = nullptr, *vbar = nullptr, *xs = nullptr, *vs = nullptr, *abar = nullptr, *gbar = nullptr, *xr = nullptr;
     float2* pmbar = nullptr;
@@ -525,8 +522,6 @@ struct Rollout {
         if (seg_graph) cudaGraphExecDestroy(seg_graph);
         for (auto* p : ck_pos) cudaFree(p);
         for (auto* p : ck_vel) cudaFree(p);
-        for (auto* p : s_pos) cudaFree(p);
-        for (auto* p : s_vel) cudaFree(p);
         for (auto* p : s_aux) cudaFree(p);
         for (auto* p : s_bnd) cudaFree(p);
         for (auto* p : s_rec) cudaFree(p);
@@ -562,8 +557,6 @@ struct Rollout {
             VFS_ADJ_TRY(cudaMalloc(&ck_vel[c], N * sizeof(float4)));
         }
         const int seg = every < steps ? every : steps;
-        s_pos.resize(seg, nullptr);
-        s_vel.resize(seg, nullptr);
         s_aux.resize(seg, nullptr);
         s_bnd.resize(seg, nullptr);
         s_rec.resize(seg, nullptr);
@@ -571,13 +564,11 @@ struct Rollout {
         s_nbr.resize(seg, nullptr);
         s_cnt.resize(seg, nullptr);
         for (int t = 0; t < seg; t++) {
-            VFS_ADJ_TRY(cudaMalloc(&s_pos[t], N * sizeof(float4)));
-            VFS_ADJ_TRY(cudaMalloc(&s_vel[t], N * sizeof(float4)));
             VFS_ADJ_TRY(cudaMalloc(&s_aux[t], N * sizeof(float4)));
             VFS_ADJ_TRY(cudaMalloc(&s_bnd[t], N * sizeof(float4)));
             VFS_ADJ_TRY(cudaMalloc(&s_rec[t], 2 * N * sizeof(float4)));
             VFS_ADJ_TRY(cudaMalloc(&s_perm[t], N * 4));
-            VFS_ADJ_TRY(cudaMalloc(&s_nbr[t], N * (size_t)cap * 4));
+            VFS_ADJ_TRY(cudaMalloc(&s_nbr[t], N * (size_t)nbr_row(cap) * 4));
             VFS_ADJ_TRY(cudaMalloc(&s_cnt[t], N * 4));
         }
         for (float4** b : {&fin_pos, &fin_vel, &xbar, &vbar, &xs, &vs, &abar, &gbar, &xr})
@@ -630,8 +621,8 @@ struct Rollout {
         return VFS_OK;
     }
 
-    // Recomputes `len` substeps from the state in the model, keeping each substep's sorted inputs,
-    // permutation, density products and neighbour lists: the model's buffers for those are pointed
+    // Recomputes `len` substeps from the state in the model, keeping each substep's permutation,
+    // force records (the sorted inputs among them), density products and neighbour lists: the model's buffers for those are pointed
     // at the segment's per-substep records, so the passes write them in place.
     int record_segment(int len) {
         if (m->nbr_cap != cap)
@@ -641,9 +632,6 @@ struct Rollout {
         float4* own_rec = m->rec;
         uint32_t* own_nbr = m->nbr;
         uint32_t* own_cnt = m->nbr_count;
-        const int o = 1 - m->cur;
-        float4* own_pos = m->pos[o];
-        float4* own_vel = m->vel[o];
         int rc = VFS_OK;
         for (int t = 0; t < len && rc == VFS_OK; t++) {
             m->aux = s_aux[t];
@@ -651,8 +639,6 @@ struct Rollout {
             m->rec = s_rec[t];
             m->nbr = s_nbr[t];
             m->nbr_count = s_cnt[t];
-            m->pos[o] = s_pos[t];
-            m->vel[o] = s_vel[t];
             rc = m->enqueue_substep(nullptr);
             if (rc == VFS_OK) {
                 const cudaError_t e = cudaMemcpyAsync(s_perm[t], m->sperm, (size_t)m->n * 4,
@@ -665,8 +651,6 @@ struct Rollout {
         m->rec = own_rec;
         m->nbr = own_nbr;
         m->nbr_count = own_cnt;
-        m->pos[o] = own_pos;
-        m->vel[o] = own_vel;
         return rc;
     }
 
@@ -708,7 +692,6 @@ struct Rollout {
         const SceneParams& p = m->scenes[0].params;
         cudaStream_t s = m->stream;
         AdjBuffers B;
-        B.pos = s_pos[t];
         B.rec = s_rec[t];
         B.aux = s_aux[t];
         B.bnd = s_bnd[t];

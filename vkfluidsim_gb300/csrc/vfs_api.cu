@@ -581,7 +581,7 @@ int Model::init() {
     VFS_CUDA_TRY(cudaMalloc(&bnd, N * sizeof(float4)));
     VFS_CUDA_TRY(cudaMalloc(&acc, N * sizeof(float4)));
     VFS_CUDA_TRY(cudaMalloc(&stage, N * 32));
-    VFS_CUDA_TRY(cudaMalloc(&nbr, N * nbr_cap * sizeof(uint32_t)));
+    VFS_CUDA_TRY(cudaMalloc(&nbr, N * (size_t)nbr_row(nbr_cap) * sizeof(uint32_t)));
     VFS_CUDA_TRY(cudaMalloc(&nbr_count, N * sizeof(uint32_t)));
     VFS_CUDA_TRY(cudaMalloc(&err, 4));
     VFS_CUDA_TRY(cudaMemset(err, 0, 4));
@@ -1260,7 +1260,7 @@ int set_neighbor_capacity(Model& m, int32_t slots) {
     VFS_CUDA_TRY(cudaStreamSynchronize(m.stream));
     const size_t N = m.n ? m.n : 1;
     uint32_t* fresh = nullptr;
-    VFS_CUDA_TRY(cudaMalloc(&fresh, N * (size_t)slots * sizeof(uint32_t)));
+    VFS_CUDA_TRY(cudaMalloc(&fresh, N * (size_t)nbr_row((uint32_t)slots) * sizeof(uint32_t)));
     cudaFree(m.nbr);
     m.nbr = fresh;
     m.nbr_cap = (uint32_t)slots;

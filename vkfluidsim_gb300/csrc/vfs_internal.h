@@ -29,6 +29,16 @@ __host__ __device__ inline uint32_t nbr_word(uint32_t listed, uint32_t cx, uint3
            (distinct ? kNbrDistinct : 0u);
 }
 
+// The neighbour lists are in quads: word k & 3 of quad (k >> 2) * n + i is entry k of particle i's
+// list, so a thread stores and reloads four entries with one 16-byte access and a warp's are
+// consecutive. A list has room for nbr_row(cap) words, its capacity in whole quads. (One
+// word per slot, each entry's store from whichever lanes found one, took 13 sectors a store: 1M
+// falling particles, density over lists 117 us, force 104; in quads 104 and 98.)
+__host__ __device__ inline uint32_t nbr_row(uint32_t cap) { return (cap + 3u) & ~3u; }
+__host__ __device__ inline size_t nbr_word_at(uint32_t k, size_t n, uint32_t i) {
+    return (((size_t)(k >> 2) * n + i) << 2) | (k & 3u);
+}
+
 // For two particles within h of each other (cells at most 2 apart per axis): are their cells
 // adjacent (at most 1 apart on every axis)? Decided from the cell residues of their words.
 __host__ __device__ inline bool nbr_cells_adjacent(uint32_t a, uint32_t b) {
@@ -140,7 +150,7 @@ enum NbrShape : int { kNbr128x6 = 0, kNbr128x8 = 1, kNbr96x8 = 2, kNbr64x12 = 3,
 // (small scenes: in the next). A single scene whose last build left too many lists unusable is
 // walked in index order, as a stale one that waits is, until its next build.
 struct SkinLists {
-    uint32_t* list = nullptr;     // slot-major: list[k * total + b] = build index of candidate k of b
+    uint32_t* list = nullptr;     // in quads (nbr_word_at): the build indices of b's candidates
     uint32_t* count = nullptr;    // per build index: list length, kSkinUsable when it can be summed
     float4* x_build = nullptr;    // per build index: position at the last build
     uint32_t* b_of_id = nullptr;  // per id: build index

@@ -821,7 +821,8 @@ __device__ __forceinline__ float w_over_sigma_r2(float r2, float inv_h) {
 struct DensitySum {
     float rho = 0.0f;
     uint32_t listed = 0;
-    uint32_t* out;  // slot `listed` of i's list (slot-major, stride = particles)
+    uint4* out;  // the next quad of i's list (stride = particles)
+    uint32_t q0 = 0, q1 = 0, q2 = 0;  // the last entries, not yet stored
     __device__ __forceinline__ void add(uint32_t i, const float4& xi, uint32_t j, const float4& xj,
                                         float inv_h, uint32_t cap, uint32_t stride) {
         add_r2(i, j, in_range2(xi, xj), true, inv_h, cap, stride);
@@ -832,12 +833,20 @@ struct DensitySum {
                                            uint32_t cap, uint32_t stride) {
         rho = __fadd_rn(rho, in ? w_over_sigma_r2(r2, inv_h) : 0.0f);
         if (in && j != i) {
-            if (listed < cap) {
-                *out = j;
+            if ((listed & 3u) == 3u && listed < nbr_row(cap)) {
+                *out = make_uint4(q0, q1, q2, j);
                 out += stride;
             }
+            q0 = q1;
+            q1 = q2;
+            q2 = j;
             listed++;
         }
+    }
+    // Stores the last quad when it is not full (its other words are never read).
+    __device__ __forceinline__ void flush(uint32_t cap) {
+        const uint32_t m = listed & 3u;
+        if (m && listed < nbr_row(cap)) *out = m == 1u ? make_uint4(q2, 0u, 0u, 0u) : m == 2u ? make_uint4(q1, q2, 0u, 0u) : make_uint4(q0, q1, q2, 0u);
     }
 };
 
@@ -1321,10 +1330,16 @@ __global__ void __launch_bounds__(kTileWarps * 32, 4)
                     n++;
                 }
             }
-            // A slot at a time, so that a warp's lanes store nearby words.
+            // A quad at a time (a fill that begins inside one: its words first), so that a warp's
+            // lanes store nearby sectors.
             const uint32_t room = c < kSkinCap ? kSkinCap - c : 0u, stored = min(n, room);
-            uint32_t* out = sk.list + (size_t)c * L.total + i;
-            for (uint32_t k = 0; k < stored; k++, out += L.total) *out = S.t.id[at[32u * k]];
+            uint32_t k = 0u;
+            for (; k < stored && ((c + k) & 3u); k++) sk.list[nbr_word_at(c + k, L.total, i)] = S.t.id[at[32u * k]];
+            uint4* out = reinterpret_cast<uint4*>(sk.list) + (size_t)((c + k) >> 2) * L.total + i;
+            for (; k + 4u <= stored; k += 4u, out += L.total)
+                *out = make_uint4(S.t.id[at[32u * k]], S.t.id[at[32u * (k + 1u)]], S.t.id[at[32u * (k + 2u)]],
+                                  S.t.id[at[32u * (k + 3u)]]);
+            for (; k < stored; k++) sk.list[nbr_word_at(c + k, L.total, i)] = S.t.id[at[32u * k]];
             c += n;
             __syncwarp();
         };
@@ -1446,7 +1461,7 @@ __device__ __forceinline__ void walk_by_warp(const SceneParams& p, uint32_t i, u
         const uint32_t listm = __ballot_sync(0xffffffffu, inr && j != i);
         if (inr && j != i) {
             const uint32_t slot = listed + (uint32_t)__popc(listm & lt);
-            if (slot < p.nbr_cap) nbr[(size_t)slot * total_n + i] = j;
+            if (slot < p.nbr_cap) nbr[nbr_word_at(slot, total_n, i)] = j;
         }
         listed += (uint32_t)__popc(listm);
         while (mask) {
@@ -1508,7 +1523,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 5)
         next = __shfl_sync(0xffffffffu, next, 0);
         const uint32_t todo = __ballot_sync(0xffffffffu, act);
         w.xi = act ? __ldg(pos + w.i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        w.d.out = nbr + w.i;
+        w.d.out = reinterpret_cast<uint4*>(nbr) + w.i;
         const uint32_t cx = cell_coord(w.xi.x, p.h), cy = cell_coord(w.xi.y, p.h), cz = cell_coord(w.xi.z, p.h);
         uint32_t single = 0u;  // lanes that walk per thread
         TileFill f;
@@ -1546,9 +1561,11 @@ __global__ void __launch_bounds__(kTileWarps * 32, 5)
             drain();
         }
         run = next;
-        if (act)
+        if (act) {
+            w.d.flush(p.nbr_cap);
             density_finish(p, w.i, w.xi, vel, cx, cy, cz, distinct_keys(p, cx, cy, cz), w.d, rec, aux, bnd,
                            nbr_count, L.host_dens, L.defer_vel);
+        }
         __syncwarp();
     }
     // The last warp out puts the counter back to zero for the next launch (every other warp has
@@ -1565,8 +1582,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 5)
 // CalculateBoundaryVolume + CalculateDensities + the per-particle part of PressureFromDensityEOS
 // (wcsph_with_boundary_model.slang:102-203), by a walk of the neighbour cells, one thread per
 // particle. Besides the density products it writes particle i's neighbour list: every in-range j
-// except i itself, in visiting order, slot-major (nbr[s * n + i], so a warp's lanes store and later
-// load consecutive words), and its length in nbr_count[i] (a length above nbr_cap means the list
+// except i itself, in visiting order, in quads (nbr_word_at), and its length in nbr_count[i] (a length above nbr_cap means the list
 // overflowed and was truncated). Positions do not change before the force pass, so that list is
 // exactly the force pass's neighbour set. It walks whole scenes in index order (no skin lists; a
 // single scene that is stale and may not rebuild, or whose lists are mostly unusable) and a batch's
@@ -1612,7 +1628,7 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
         const float4 xi = __ldg(pos + i);
         const uint32_t cx = cell_coord(xi.x, p.h), cy = cell_coord(xi.y, p.h), cz = cell_coord(xi.z, p.h);
         DensitySum d;
-        d.out = nbr + i;
+        d.out = reinterpret_cast<uint4*>(nbr) + i;
         uint32_t s_end = tid;  // shared-memory word one past the last kept candidate (stride kNbrBlock)
         // Scene constants used per candidate, in registers (a batched launch reads its scene's
         // parameters from a device table).
@@ -1636,6 +1652,7 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
             if (s_end > tid + kDrainAt * kNbrBlock) drain();
         });
         drain();
+        d.flush(s_nbr_cap);
         density_finish(p, i, xi, vel, cx, cy, cz, distinct_keys(p, cx, cy, cz), d, rec, aux, bnd, nbr_count,
                        L.host_dens, L.defer_vel);
     }
@@ -1656,13 +1673,17 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
 // h / 4 since the build, so its 27 cells lie in the build's 5x5x5 block, whose keys were
 // distinct), in the list's order. Every other particle goes to the queue for k_walk_queue (a
 // batch's: k_walk).
-// No shared memory: the pass is bound by its chains of dependent loads, so it runs at the
-// occupancy its registers allow.
+// Bound by the chains of dependent loads and by L1: the gathers' and the list stores' wavefronts. The
+// in-range indices wait in a ring of two quads per thread in shared memory and leave as whole quads,
+// at most one per four candidates: 1M falling particles 117 -> 104 us (quads gathered in registers
+// and stored as they fill: 109 to 116). Nine blocks an SM: ten spill (112 us), eight have fewer loads
+// in flight (108).
 template <bool kBatch>
-__global__ void __launch_bounds__(kListBlock, 10)
+__global__ void __launch_bounds__(kListBlock, 9)
     k_density_list(StepLaunch L, const float4* __restrict__ pos, const float4* __restrict__ vel,
                    float4* __restrict__ rec, float4* __restrict__ aux, float4* __restrict__ bnd,
                    uint32_t* __restrict__ nbr, uint32_t* __restrict__ nbr_count, SkinLists sk) {
+    __shared__ uint32_t s_ring[8 * kListBlock];
     const uint32_t i = blockIdx.x * kListBlock + threadIdx.x;
     // A single scene that is stale and waits, or whose last build left most lists unusable: k_walk walks
     // it in index order.
@@ -1688,40 +1709,56 @@ __global__ void __launch_bounds__(kListBlock, 10)
             const float h2 = p.h2, s_inv_h = p.inv_h;
             const uint32_t s_nbr_cap = p.nbr_cap;
             DensitySum d;
-            d.out = nbr + i;
+            d.out = reinterpret_cast<uint4*>(nbr) + i;
             const size_t stride = L.total;
-            const uint32_t* q = sk.list + row;
+            const uint4* q = reinterpret_cast<const uint4*>(sk.list) + row;
+            uint32_t quads = 0u;
+            uint32_t* ring = s_ring + threadIdx.x;
+            auto add = [&](uint32_t jj, float r2, bool in) {
+                d.rho = __fadd_rn(d.rho, in ? w_over_sigma_r2(r2, s_inv_h) : 0.0f);
+                ring[(d.listed & 7u) * kListBlock] = jj;
+                d.listed += in && jj != i ? 1u : 0u;
+            };
+            auto put = [&]() {
+                const uint32_t* r = ring + (quads & 1u) * (4u * kListBlock);
+                if (4u * quads < nbr_row(s_nbr_cap))
+                    *d.out = make_uint4(r[0], r[kListBlock], r[2 * kListBlock], r[3 * kListBlock]);
+                d.out += L.total;
+                quads++;
+            };
+            // The next quad of build indices loads while the current one is resolved and summed.
+            uint4 next = make_uint4(0u, 0u, 0u, 0u);
+            if (n_list) next = __ldg(q);
             uint32_t k = 0;
-            // The next batch's build indices load while the current batch is resolved and summed.
-            uint32_t jn[4];
-            if (n_list >= 4u) {
-#pragma unroll
-                for (int u = 0; u < 4; u++) jn[u] = __ldg(q + u * stride);
-            }
 #pragma unroll 1
-            for (; k + 4u <= n_list; k += 4u, q += 4 * stride) {
-                uint32_t j[4];
+            for (; k + 4u <= n_list; k += 4u) {
+                const uint32_t j[4] = {next.x, next.y, next.z, next.w};
+                q += stride;
+                if (k + 4u < n_list) next = __ldg(q);
                 float4 xj[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) j[u] = jn[u];
-                if (k + 8u <= n_list) {
-#pragma unroll
-                    for (int u = 0; u < 4; u++) jn[u] = __ldg(q + (4 + u) * stride);
-                }
 #pragma unroll
                 for (int u = 0; u < 4; u++) xj[u] = __ldg(sk.xcur + j[u]);  // position, sorted index
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     const float r2 = in_range2(xi, xj[u]);
-                    if (r2 <= h2) d.add_r2(i, __float_as_uint(xj[u].w), r2, true, s_inv_h, s_nbr_cap, L.total);
+                    add(__float_as_uint(xj[u].w), r2, r2 <= h2);
+                }
+                if ((d.listed >> 2) != quads) put();
+            }
+            if (k < n_list) {
+                const uint32_t m = n_list - k;  // 1 to 3
+                const uint32_t j[3] = {next.x, m > 1u ? next.y : next.x, m > 2u ? next.z : next.x};
+                float4 xj[3];
+#pragma unroll
+                for (int u = 0; u < 3; u++) xj[u] = __ldg(sk.xcur + j[u]);
+#pragma unroll
+                for (int u = 0; u < 3; u++) {
+                    const float r2 = in_range2(xi, xj[u]);
+                    add(__float_as_uint(xj[u].w), r2, (uint32_t)u < m && r2 <= h2);
                 }
             }
-#pragma unroll 1
-            for (; k < n_list; k++, q += stride) {
-                const float4 xj = __ldg(sk.xcur + __ldg(q));
-                const float r2 = in_range2(xi, xj);
-                if (r2 <= h2) d.add_r2(i, __float_as_uint(xj.w), r2, true, s_inv_h, s_nbr_cap, L.total);
-            }
+            if ((d.listed >> 2) != quads) put();
+            if (d.listed & 3u) put();
             density_finish(p, i, xi, vel, cx, cy, cz, distinct_keys(p, cx, cy, cz), d, rec, aux,
                            bnd, nbr_count, L.host_dens, L.defer_vel);
         }
@@ -1825,7 +1862,7 @@ __global__ void __launch_bounds__(kPlaneBlock)
         for (uint32_t o = tid; o < s_end; o += kPlaneBlock) {
             const uint32_t j = s_j[o];
             if (j == i) continue;
-            if (k < p.nbr_cap) nbr[(size_t)k * L.total + i] = j;
+            if (k < p.nbr_cap) nbr[nbr_word_at(k, L.total, i)] = j;
             k++;
         }
     }
@@ -2026,33 +2063,34 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
         const uint32_t listed = nbr_count[i] & kNbrCountMask;
         if (listed <= p.nbr_cap) {
             // The density pass's list: the in-range neighbours in the reference's visiting order.
-            uint32_t k = 0;
-            const uint32_t* nl = nbr + i;  // slot k of particle i's list
+            // A quad of indices is one load, made under the previous quad's gathers, so each quad
+            // waits on one dependent load (the records) instead of two, the last, partial one too.
+            const uint4* nl = reinterpret_cast<const uint4*>(nbr) + i;
             const size_t stride = L.total;
-            // The next batch's indices load while the current batch is gathered and summed, so
-            // each batch waits on one dependent load (the records) instead of two.
-            uint32_t jn[4];
-            if (listed >= 4u) {
-#pragma unroll
-                for (int u = 0; u < 4; u++) jn[u] = __ldg(nl + u * stride);
-            }
+            uint4 next = make_uint4(0u, 0u, 0u, 0u);
+            if (listed) next = __ldg(nl);
+            uint32_t k = 0;
 #pragma unroll 1
-            for (; k + 4u <= listed; k += 4u, nl += 4 * stride) {
-                uint32_t j[4];
+            for (; k + 4u <= listed; k += 4u) {
+                const uint32_t j[4] = {next.x, next.y, next.z, next.w};
+                nl += stride;
+                if (k + 4u < listed) next = __ldg(nl);
                 float4 a[4], b[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) j[u] = jn[u];
-                if (k + 8u <= listed) {
-#pragma unroll
-                    for (int u = 0; u < 4; u++) jn[u] = __ldg(nl + (4 + u) * stride);
-                }
 #pragma unroll
                 for (int u = 0; u < 4; u++) load_record(rec, j[u], a[u], b[u]);
 #pragma unroll
                 for (int u = 0; u < 4; u++) force_term(p, xi, vi, pdi, a[u], make_float2(a[u].w, b[u].w), b[u], f);
             }
-#pragma unroll 1
-            for (; k < listed; k++, nl += stride) force_term_rec(p, xi, vi, pdi, rec, __ldg(nl), f);
+            if (k < listed) {
+                const uint32_t m = listed - k;  // 1 to 3
+                const uint32_t j[3] = {next.x, m > 1u ? next.y : next.x, m > 2u ? next.z : next.x};
+                float4 a[3], b[3];
+#pragma unroll
+                for (int u = 0; u < 3; u++) load_record(rec, j[u], a[u], b[u]);
+#pragma unroll
+                for (int u = 0; u < 3; u++)
+                    if ((uint32_t)u < m) force_term(p, xi, vi, pdi, a[u], make_float2(a[u].w, b[u].w), b[u], f);
+            }
         } else {
             // Overflowed list (very dense neighbourhood): walk the candidates again and add every
             // in-range one as it comes, in the same order. This path needs no shared memory, so

@@ -66,7 +66,7 @@ struct Model {
     float4* rec = nullptr;  // 2 float4 per particle: the force pass's neighbour records
     float4* bnd = nullptr;
     float4* acc = nullptr;
-    uint32_t* nbr = nullptr;        // nbr_cap slot-major neighbour lists
+    uint32_t* nbr = nullptr;        // neighbour lists of nbr_row(nbr_cap) words, in quads
     uint32_t nbr_cap = kNbrCap;     // slots per particle (longer lists fall back to a walk)
     uint32_t* nbr_count = nullptr;  // list length per particle
     SkinLists skin{};               // candidate lists with a skin (absent in three-lane mode)
