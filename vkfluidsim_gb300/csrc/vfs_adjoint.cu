@@ -20,6 +20,7 @@
 #include <string>
 #include <vector>
 
+#include "vfs_chain.h"
 #include "vfs_cuda.h"
 #include "vfs_internal.h"
 #include "vfs_model.h"
@@ -203,6 +204,7 @@ struct AdjBuffers {
 // Symplectic Euler, reversed: x_out = x' + v_out dt, v_out = v' + a dt.
 __global__ void k_adj_integrate(SceneParams p, uint32_t n, const float4* __restrict__ xbar_out,
                                 const float4* __restrict__ vbar_out, AdjBuffers B) {
+    VFS_CHAINED();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 xo = xbar_out[i], vo = vbar_out[i];
@@ -270,6 +272,7 @@ __device__ __forceinline__ void load_record(const float4* __restrict__ rec, uint
 // 31.3 for one, all with four lanes).
 template <int kLanes>
 __global__ void __launch_bounds__(128) k_adj_force(SceneParams p, uint32_t n, AdjBuffers B) {
+    VFS_CHAINED();
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t j = (uint32_t)(t / kLanes), lane = (uint32_t)(t % kLanes);
     float3 xb = make_float3(0.f, 0.f, 0.f), vb = make_float3(0.f, 0.f, 0.f);
@@ -365,6 +368,7 @@ __global__ void __launch_bounds__(128) k_adj_force(SceneParams p, uint32_t n, Ad
 
 // Adjoint of the EOS epilogue: rho_bar from pd_bar, pb_bar, mr_bar; d L / d k.
 __global__ void k_adj_eos(SceneParams p, uint32_t n, AdjBuffers B) {
+    VFS_CHAINED();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     float dk = 0.0f;
     if (i < n) {
@@ -395,6 +399,7 @@ __global__ void k_adj_eos(SceneParams p, uint32_t n, AdjBuffers B) {
 // lane (27.4 -> 12.6 us at 65,536 particles; with four lanes 15.7 for two in flight, 13.9 for four).
 template <int kLanes>
 __global__ void __launch_bounds__(128) k_adj_density(SceneParams p, uint32_t n, AdjBuffers B) {
+    VFS_CHAINED();
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t j = (uint32_t)(t / kLanes), lane = (uint32_t)(t % kLanes);
     float3 xb = make_float3(0.f, 0.f, 0.f), xj = xb;
@@ -460,6 +465,7 @@ __global__ void __launch_bounds__(128) k_adj_density(SceneParams p, uint32_t n, 
 __global__ void k_adj_unsort(uint32_t n, const uint32_t* __restrict__ perm,
                              const float4* __restrict__ xs, const float4* __restrict__ vs,
                              float4* __restrict__ xprev, float4* __restrict__ vprev) {
+    VFS_CHAINED();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t src = perm[i];
@@ -707,7 +713,7 @@ struct Rollout {
         B.dparams = dparams;
         B.err = m->err;
         const unsigned g256 = (n + 255) / 256;
-        k_adj_integrate<<<g256, 256, 0, s>>>(p, n, xbar, vbar, B);
+        launch_chained(k_adj_integrate, g256, 256, 0, s, p, n, xbar, vbar, B);
         // Lanes sharing one particle's list: two where that fills the GPU (65,536 particles: force 28.6
         // us, density 12.6; four 31.3 and 13.9, eight 35.6 and 17.2), four below, where each lane's
         // chain of gathers is the time (24-substep gradients, four against two lanes: 4,000 particles
@@ -715,15 +721,15 @@ struct Rollout {
         const bool wide = n < 40960u;
         const unsigned gl = (unsigned)(((size_t)n * (wide ? 4 : 2) + 127) / 128);
         if (wide)
-            k_adj_force<4><<<gl, 128, 0, s>>>(p, n, B);
+            launch_chained(k_adj_force<4>, gl, 128, 0, s, p, n, B);
         else
-            k_adj_force<2><<<gl, 128, 0, s>>>(p, n, B);
-        k_adj_eos<<<g256, 256, 0, s>>>(p, n, B);
+            launch_chained(k_adj_force<2>, gl, 128, 0, s, p, n, B);
+        launch_chained(k_adj_eos, g256, 256, 0, s, p, n, B);
         if (wide)
-            k_adj_density<4><<<gl, 128, 0, s>>>(p, n, B);
+            launch_chained(k_adj_density<4>, gl, 128, 0, s, p, n, B);
         else
-            k_adj_density<2><<<gl, 128, 0, s>>>(p, n, B);
-        k_adj_unsort<<<g256, 256, 0, s>>>(n, s_perm[t], xs, vs, xbar, vbar);
+            launch_chained(k_adj_density<2>, gl, 128, 0, s, p, n, B);
+        launch_chained(k_adj_unsort, g256, 256, 0, s, n, s_perm[t], xs, vs, xbar, vbar);
         VFS_ADJ_TRY(cudaGetLastError());
         return VFS_OK;
     }

@@ -26,6 +26,7 @@
 #include <climits>
 #include <atomic>
 
+#include "vfs_chain.h"
 #include "vfs_internal.h"
 
 namespace vfs {
@@ -378,6 +379,7 @@ __global__ void __launch_bounds__(BLOCK)
                int shift, int bins, const uint32_t* __restrict__ ghist,
                uint32_t* __restrict__ counter, uint32_t* __restrict__ status,
                uint32_t* __restrict__ err, const uint32_t* __restrict__ n_dev) {
+    VFS_CHAINED();
     static_assert(BLOCK == 256, "block scan assumes 256 threads");
     constexpr int WARPS = BLOCK / 32;
     constexpr int TILE = BLOCK * ITEMS;
@@ -609,6 +611,7 @@ __global__ void __launch_bounds__(kCellBlock)
                     const uint32_t* __restrict__ b_of_id, float4* __restrict__ xcur,
                     const float4* __restrict__ x_build, uint32_t* __restrict__ stale,
                     const uint32_t* __restrict__ ctl, uint32_t* __restrict__ wcount) {
+    VFS_CHAINED();
     __shared__ uint32_t s_lo, s_hi;
     if (wcount && blockIdx.x == 0 && threadIdx.x == 0) wcount[0] = 0u;  // the list pass's queue
     // The sort is done with its scratch (histograms, tile counters, look-back status): clear it
@@ -655,6 +658,7 @@ __global__ void __launch_bounds__(128)
               const uint32_t* __restrict__ b_of_id, float4* __restrict__ xcur,
               const float4* __restrict__ x_build, uint32_t* __restrict__ stale,
               const uint32_t* __restrict__ ctl, uint32_t* __restrict__ wcount) {
+    VFS_CHAINED_LATE();
     if (wcount && blockIdx.x == 0 && threadIdx.x == 0) wcount[0] = 0u;  // the list pass's queue
     reorder_particle(L, blockIdx.x * 128u + threadIdx.x, n, perm, pos_in, vel_in, pos_out, vel_out, b_of_id,
                      xcur, x_build, stale, ctl, wcount);
@@ -1294,13 +1298,21 @@ __device__ __forceinline__ bool sums_lists(const SkinLists& sk) {
 template <bool kBatch>
 __global__ void __launch_bounds__(kTileWarps * 32, 4)
     k_skin_build(StepLaunch L, const float4* __restrict__ pos, const uint32_t* __restrict__ scan, SkinLists sk) {
+    VFS_CHAINED_LATE();
     static_assert(kSkinCap * 32 * sizeof(uint16_t) <= sizeof(float4) * kTileBlocks * 4 * kTileWordStride,
                   "the lists of a fill take the staged positions' place");
     extern __shared__ __align__(16) unsigned char s_raw[];
     TileSmem& S = reinterpret_cast<TileSmem*>(s_raw)[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t slot_of = (lane >> 2) + 8u * (lane & 3u);  // lane 4 g + q owns slot g + 8 q of a run
-    if (sk.wcount[1] == 0u) return;  // no scene's build is due
+    // The list pass's blocks beside a build's run with what on-chip memory its tiles leave as L1: let in
+    // at once only where a build is rarely due (1M flow, building every few substeps: 6.67 ms, let in
+    // always 6.74; 97,336 particles 66.1 us a substep, let in late 67.5).
+    if (!kBatch && L.total < kSkinFullScene) chained_release();
+    if (sk.wcount[1] == 0u) {  // no scene's build is due
+        chained_release();
+        return;
+    }
     const uint32_t runs = (L.total + 31u) / 32u;
     for (uint32_t run = blockIdx.x * (uint32_t)kTileWarps + (threadIdx.x >> 5); run < runs;
          run += gridDim.x * (uint32_t)kTileWarps) {
@@ -1491,6 +1503,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 5)
                  float4* __restrict__ rec, const uint32_t* __restrict__ scan,
                  float4* __restrict__ aux, float4* __restrict__ bnd, uint32_t* __restrict__ nbr,
                  uint32_t* __restrict__ nbr_count, SkinLists sk, uint32_t* __restrict__ sched, bool tiles) {
+    VFS_CHAINED();
     extern __shared__ __align__(16) unsigned char s_raw[];
     TileSmem& S = reinterpret_cast<TileSmem*>(s_raw)[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
@@ -1596,10 +1609,13 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
            float4* __restrict__ rec, const uint32_t* __restrict__ scan,
            float4* __restrict__ aux, float4* __restrict__ bnd, uint32_t* __restrict__ nbr,
            uint32_t* __restrict__ nbr_count, SkinLists sk, uint32_t* __restrict__ sched) {
+    VFS_CHAINED_LATE();
     static_assert(kNbrBlock % 32 == 0, "whole warps");
     __shared__ uint32_t s_j[kListCap * kNbrBlock];
     const int tid = threadIdx.x;
     const uint32_t lane = (uint32_t)(tid & 31);
+    // The force pass's blocks likewise: not beside a batch's walk (64 scenes: 27.1 ms, late 25.7).
+    if (!kBatch) chained_release();
     if (!kBatch && sk.list && sums_lists(sk)) return;
     // Every warp takes runs of 32 slots: first the run of its own index, then runs claimed from
     // the launch's counter (sched[0]), until none is left. Walks differ widely in length (the
@@ -1683,6 +1699,7 @@ __global__ void __launch_bounds__(kListBlock, 9)
     k_density_list(StepLaunch L, const float4* __restrict__ pos, const float4* __restrict__ vel,
                    float4* __restrict__ rec, float4* __restrict__ aux, float4* __restrict__ bnd,
                    uint32_t* __restrict__ nbr, uint32_t* __restrict__ nbr_count, SkinLists sk) {
+    VFS_CHAINED();
     __shared__ uint32_t s_ring[8 * kListBlock];
     const uint32_t i = blockIdx.x * kListBlock + threadIdx.x;
     // A single scene that is stale and waits, or whose last build left most lists unusable: k_walk walks
@@ -1806,6 +1823,7 @@ __global__ void __launch_bounds__(kPlaneBlock)
                      float4* __restrict__ rec, const uint32_t* __restrict__ scan,
                      float4* __restrict__ aux, float4* __restrict__ bnd,
                      uint32_t* __restrict__ nbr, uint32_t* __restrict__ nbr_count) {
+    VFS_CHAINED_LATE();
     __shared__ uint32_t s_j[kListCap * kPlaneBlock];
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31u, pw = lane / 3u, pl = lane - 3u * pw;
@@ -2004,6 +2022,7 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
             float4* __restrict__ vel_out, float4* __restrict__ acc_out,
             uint32_t* __restrict__ skin_stale, uint32_t* __restrict__ skin_ctl,
             uint32_t* __restrict__ skin_due, HostOut ho) {
+    VFS_CHAINED();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     // The density pass is done with the skin lists' flags: run each scene's build policy and clear
     // the flags for the next substep.
@@ -2177,6 +2196,7 @@ __global__ void __launch_bounds__(256)
                  const float* __restrict__ host3, float4* __restrict__ pos_out,
                  float4* __restrict__ aux, const uint32_t* __restrict__ b_of_id,
                  uint32_t* __restrict__ b_next) {
+    VFS_CHAINED();
     __shared__ uint32_t s_h[kMaxSortPasses * kMaxSortBins];
     __shared__ uint32_t s_n[8];
     __shared__ float s_p[kHostIn ? 3 * kDeltaTile : 1];
@@ -2249,6 +2269,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(1024)
     k_tile_scan(uint32_t tiles, uint32_t* __restrict__ tile_cnt, uint32_t* __restrict__ bits,
                 uint32_t W, uint32_t* __restrict__ mcount) {
+    VFS_CHAINED();
     __shared__ uint32_t s_w[32];
     __shared__ uint32_t s_carry;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -2299,6 +2320,7 @@ __global__ void __launch_bounds__(256)
     k_moved_compact(StepLaunch L, const float4* __restrict__ pos, uint32_t* __restrict__ bits,
                     const uint32_t* __restrict__ tile_cnt, uint32_t* __restrict__ mkeys,
                     uint32_t* __restrict__ midx, uint32_t* __restrict__ mcount) {
+    VFS_CHAINED();
     __shared__ uint32_t s_bits[32], s_off[32], s_sum[8];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t W = (L.total + 31u) >> 5;
@@ -2384,6 +2406,7 @@ __global__ void __launch_bounds__(256)
             const uint32_t* __restrict__ mcount, const uint32_t* __restrict__ mk,
             const uint32_t* __restrict__ mi, uint32_t* __restrict__ out_keys,
             uint32_t* __restrict__ out_perm) {
+    VFS_CHAINED();
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t m = min(*mcount, n);
     const uint32_t W = (n + 31u) >> 5;
@@ -2442,6 +2465,7 @@ __global__ void __launch_bounds__(1024, 1)
                  uint32_t* __restrict__ skeys, uint32_t* __restrict__ perm, uint32_t* __restrict__ scan,
                  const float* __restrict__ host3, float4* __restrict__ pos_out, float4* __restrict__ aux,
                  const uint32_t* __restrict__ b_of_id, uint32_t* __restrict__ b_next) {
+    VFS_CHAINED();
     namespace cg = cooperative_groups;
     constexpr uint32_t kSeg = 1024u * ITEMS;
     extern __shared__ uint32_t s_mem[];
@@ -2627,8 +2651,7 @@ template <int ITEMS>
 cudaError_t launch_onesweep_t(uint32_t n, const SortConfig& sc, const SortScratch& scr, int pass,
                               const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
                               uint32_t* vout, const uint32_t* n_dev, cudaStream_t s) {
-    k_onesweep<kSortBlock, ITEMS><<<sc.tiles, kSortBlock, 0, s>>>(
-        kin, vin, kout, vout, n, pass * sc.digit_bits, sc.bins, scr.ghist + pass * sc.bins,
+    launch_chained(k_onesweep<kSortBlock, ITEMS>, sc.tiles, kSortBlock, 0, s, kin, vin, kout, vout, n, pass * sc.digit_bits, sc.bins, scr.ghist + pass * sc.bins,
         scr.counters + pass, scr.status + (size_t)pass * sc.tiles * sc.bins, scr.err, n_dev);
     return cudaGetLastError();
 }
@@ -2692,29 +2715,29 @@ cudaError_t launch_keys_delta(const StepLaunch& L, const float4* pos, const uint
     if (L.total == 0) return cudaSuccess;
     const uint32_t tiles = sc.delta_blocks, W = (L.total + 31u) >> 5;
     if (L.n_scenes > 1)
-        k_keys_flags<true, false><<<tiles, 256, 0, s>>>(L, pos, pkeys, bits, sc.passes, sc.digit_bits,
+        launch_chained(k_keys_flags<true, false>, tiles, 256, 0, s, L, pos, pkeys, bits, sc.passes, sc.digit_bits,
                                                         scr.ghist, scr.dstatus, nullptr, nullptr, nullptr,
                                                         nullptr, nullptr);
     else if (host3)
-        k_keys_flags<false, true><<<tiles, 256, 0, s>>>(L, pos, pkeys, bits, sc.passes, sc.digit_bits,
+        launch_chained(k_keys_flags<false, true>, tiles, 256, 0, s, L, pos, pkeys, bits, sc.passes, sc.digit_bits,
                                                         scr.ghist, scr.dstatus, host3, pos_out, aux,
                                                         b_of_id, b_next);
     else
-        k_keys_flags<false, false><<<tiles, 256, 0, s>>>(L, pos, pkeys, bits, sc.passes, sc.digit_bits,
+        launch_chained(k_keys_flags<false, false>, tiles, 256, 0, s, L, pos, pkeys, bits, sc.passes, sc.digit_bits,
                                                          scr.ghist, scr.dstatus, nullptr, nullptr, nullptr,
                                                          nullptr, nullptr);
     if (tiles <= kFoldTiles) {
         if (L.n_scenes > 1)
-            k_moved_compact<true, true><<<tiles, 256, 0, s>>>(L, pos, bits, scr.dstatus, mkeys, midx, scr.mcount);
+            launch_chained(k_moved_compact<true, true>, tiles, 256, 0, s, L, pos, bits, scr.dstatus, mkeys, midx, scr.mcount);
         else
-            k_moved_compact<false, true><<<tiles, 256, 0, s>>>(L, pos, bits, scr.dstatus, mkeys, midx, scr.mcount);
+            launch_chained(k_moved_compact<false, true>, tiles, 256, 0, s, L, pos, bits, scr.dstatus, mkeys, midx, scr.mcount);
         return cudaGetLastError();
     }
-    k_tile_scan<<<1, 1024, 0, s>>>(tiles, scr.dstatus, bits, W, scr.mcount);
+    launch_chained(k_tile_scan, 1, 1024, 0, s, tiles, scr.dstatus, bits, W, scr.mcount);
     if (L.n_scenes > 1)
-        k_moved_compact<true, false><<<tiles, 256, 0, s>>>(L, pos, bits, scr.dstatus, mkeys, midx, scr.mcount);
+        launch_chained(k_moved_compact<true, false>, tiles, 256, 0, s, L, pos, bits, scr.dstatus, mkeys, midx, scr.mcount);
     else
-        k_moved_compact<false, false><<<tiles, 256, 0, s>>>(L, pos, bits, scr.dstatus, mkeys, midx, scr.mcount);
+        launch_chained(k_moved_compact<false, false>, tiles, 256, 0, s, L, pos, bits, scr.dstatus, mkeys, midx, scr.mcount);
     return cudaGetLastError();
 }
 
@@ -2727,15 +2750,17 @@ cudaError_t sort_small_items(const StepLaunch& L, const float4* pos, int bits, i
                              uint32_t* perm, uint32_t* scan, const float* host3, float4* pos_out, float4* aux,
                              const uint32_t* b_of_id, uint32_t* b_next, cudaStream_t s) {
     auto* const kernel = k_sort_small<kBatch, kHostIn, kBlocks, ITEMS>;
-    cudaLaunchAttribute cluster{};
-    cluster.id = cudaLaunchAttributeClusterDimension;
-    cluster.val.clusterDim = {kBlocks, 1, 1};
+    cudaLaunchAttribute attrs[2] = {};
+    attrs[0].id = cudaLaunchAttributeClusterDimension;
+    attrs[0].val.clusterDim = {kBlocks, 1, 1};
+    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see vfs_chain.h
+    attrs[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(kBlocks);
     cfg.blockDim = dim3(1024);
     cfg.dynamicSmemBytes = (3u * 1024u * ITEMS + 32u * 256u) * sizeof(uint32_t);
     cfg.stream = s;
-    cfg.attrs = &cluster;
+    cfg.attrs = attrs;
     cfg.numAttrs = 1;
     static std::atomic<int> state[16];  // 0: not asked, 1: this cluster size, 2: eight blocks instead
     int dev = 0;
@@ -2761,6 +2786,7 @@ cudaError_t sort_small_items(const StepLaunch& L, const float4* pos, int bits, i
             return sort_small_items<kBatch, kHostIn, 8, 2 * ITEMS>(L, pos, bits, passes, skeys, perm, scan, host3,
                                                                    pos_out, aux, b_of_id, b_next, s);
     }
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kernel, L, pos, bits, passes, skeys, perm, scan, host3, pos_out, aux, b_of_id, b_next);
 }
 
@@ -2791,7 +2817,7 @@ cudaError_t launch_reorder(const StepLaunch& L, uint32_t n, const uint32_t* perm
                            const float4* vel_in, float4* pos_out, float4* vel_out, const SkinLists& sk,
                            cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    k_reorder<<<(n + 127u) / 128u, 128, 0, s>>>(L, n, perm, pos_in, vel_in, pos_out, vel_out, sk.b_of_id, sk.xcur,
+    launch_chained(k_reorder, (n + 127u) / 128u, 128, 0, s, L, n, perm, pos_in, vel_in, pos_out, vel_out, sk.b_of_id, sk.xcur,
                                                 sk.x_build, sk.stale, sk.ctl, sk.wcount);
     return cudaGetLastError();
 }
@@ -2801,7 +2827,7 @@ cudaError_t launch_merge(uint32_t n, const uint32_t* pkeys, const uint32_t* bits
                          uint32_t* out_keys, uint32_t* out_perm, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     const uint64_t threads = 2ull * n;
-    k_merge<<<(unsigned)((threads + 255u) / 256u), 256, 0, s>>>(n, pkeys, bits, mcount, mk, mi,
+    launch_chained(k_merge, (unsigned)((threads + 255u) / 256u), 256, 0, s, n, pkeys, bits, mcount, mk, mi,
                                                                  out_keys, out_perm);
     return cudaGetLastError();
 }
@@ -2878,15 +2904,15 @@ cudaError_t launch_cells_reorder(const StepLaunch& L, uint32_t n, const uint32_t
     if (n == 0) return cudaSuccess;
     switch (kc.cell_block) {
         case 128:
-            k_cells_reorder<128><<<(n + 128u) / 128u, 128, 0, s>>>(L, n, skeys, perm, cell_scan, pos_in,
+            launch_chained(k_cells_reorder<128>, (n + 128u) / 128u, 128, 0, s, L, n, skeys, perm, cell_scan, pos_in,
                                                                  vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl, sk.wcount);
             break;
         case 512:
-            k_cells_reorder<512><<<(n + 512u) / 512u, 512, 0, s>>>(L, n, skeys, perm, cell_scan, pos_in,
+            launch_chained(k_cells_reorder<512>, (n + 512u) / 512u, 512, 0, s, L, n, skeys, perm, cell_scan, pos_in,
                                                                  vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl, sk.wcount);
             break;
         default:
-            k_cells_reorder<256><<<(n + 256u) / 256u, 256, 0, s>>>(L, n, skeys, perm, cell_scan, pos_in,
+            launch_chained(k_cells_reorder<256>, (n + 256u) / 256u, 256, 0, s, L, n, skeys, perm, cell_scan, pos_in,
                                                                  vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl, sk.wcount);
     }
     return cudaGetLastError();
@@ -2936,7 +2962,7 @@ cudaError_t launch_build(const StepLaunch& L, const float4* pos, const uint32_t*
     uint32_t blocks = 0u;
     const cudaError_t e = tile_blocks(k_skin_build<kBatch>, per_sm, L.total, blocks);
     if (e != cudaSuccess) return e;
-    k_skin_build<kBatch><<<blocks, kTileWarps * 32, kTileSmemBytes, s>>>(L, pos, cell_scan, sk);
+    launch_chained(k_skin_build<kBatch>, blocks, kTileWarps * 32, kTileSmemBytes, s, L, pos, cell_scan, sk);
     return cudaGetLastError();
 }
 
@@ -2948,7 +2974,7 @@ cudaError_t launch_walk_queue(const StepLaunch& L, const float4* pos, const floa
     uint32_t blocks = 0u;
     const cudaError_t e = tile_blocks(k_walk_queue, per_sm, L.total, blocks);
     if (e != cudaSuccess) return e;
-    k_walk_queue<<<blocks, kTileWarps * 32, kTileSmemBytes, s>>>(L, pos, vel, rec, cell_scan, aux, bnd, nbr,
+    launch_chained(k_walk_queue, blocks, kTileWarps * 32, kTileSmemBytes, s, L, pos, vel, rec, cell_scan, aux, bnd, nbr,
                                                                  nbr_count, sk, sched, tiles);
     return cudaGetLastError();
 }
@@ -2971,7 +2997,7 @@ cudaError_t launch_walk(const StepLaunch& L, const float4* pos, const float4* ve
     const int sms = sm_count();
     const uint32_t all_blocks = (L.total + B - 1) / B;
     const uint32_t blocks = sms > 0 ? min(all_blocks, (uint32_t)sms * (uint32_t)r) : all_blocks;
-    k_walk<kBatch, B, M><<<blocks, B, 0, s>>>(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, sched);
+    launch_chained(k_walk<kBatch, B, M>, blocks, B, 0, s, L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, sched);
     return cudaGetLastError();
 }
 
@@ -2996,12 +3022,11 @@ void force_shape(const StepLaunch& L, const float4* pos, const float4* vel, cons
                  const SkinLists& sk, cudaStream_t s, const HostOut& ho) {
     const uint32_t blocks = (L.total + B - 1) / B;
     if (L.n_scenes > 1)
-        k_force<true, B, M><<<blocks, B, 0, s>>>(L, pos, vel, aux, rec, bnd, cell_scan, nbr, nbr_count,
+        launch_chained(k_force<true, B, M>, blocks, B, 0, s, L, pos, vel, aux, rec, bnd, cell_scan, nbr, nbr_count,
                                                  pos_out, vel_out, acc_out, sk.stale, sk.ctl,
                                                  sk.wcount + 1, HostOut{});
     else  // shared memory only for host outputs: without them the whole on-chip memory stays L1
-        k_force<false, B, M><<<blocks, B, ho.any() ? 7 * B * sizeof(float) : 0, s>>>(
-            L, pos, vel, aux, rec, bnd, cell_scan, nbr, nbr_count, pos_out, vel_out, acc_out,
+        launch_chained(k_force<false, B, M>, blocks, B, ho.any() ? 7 * B * sizeof(float) : 0, s, L, pos, vel, aux, rec, bnd, cell_scan, nbr, nbr_count, pos_out, vel_out, acc_out,
             sk.stale, sk.ctl, sk.wcount + 1, ho);
 }
 
@@ -3018,10 +3043,10 @@ cudaError_t launch_density(const StepLaunch& L, const float4* pos, const float4*
     if (planes_mode(L.total)) {
         const uint32_t blocks = (L.total + 29u) / 30u;
         if (L.n_scenes > 1)
-            k_density_planes<true><<<blocks, kPlaneBlock, 0, s>>>(L, pos, vel, rec, cell_scan, aux, bnd,
+            launch_chained(k_density_planes<true>, blocks, kPlaneBlock, 0, s, L, pos, vel, rec, cell_scan, aux, bnd,
                                                                   nbr, nbr_count);
         else
-            k_density_planes<false><<<blocks, kPlaneBlock, 0, s>>>(L, pos, vel, rec, cell_scan, aux, bnd,
+            launch_chained(k_density_planes<false>, blocks, kPlaneBlock, 0, s, L, pos, vel, rec, cell_scan, aux, bnd,
                                                                    nbr, nbr_count);
         return cudaGetLastError();
     }
@@ -3033,9 +3058,9 @@ cudaError_t launch_density(const StepLaunch& L, const float4* pos, const float4*
         if (e != cudaSuccess) return e;
         const uint32_t lb = (L.total + kListBlock - 1) / kListBlock;
         if (batch) {
-            k_density_list<true><<<lb, kListBlock, 0, s>>>(L, pos, vel, rec, aux, bnd, nbr, nbr_count, sk);
+            launch_chained(k_density_list<true>, lb, kListBlock, 0, s, L, pos, vel, rec, aux, bnd, nbr, nbr_count, sk);
         } else {
-            k_density_list<false><<<lb, kListBlock, 0, s>>>(L, pos, vel, rec, aux, bnd, nbr, nbr_count, sk);
+            launch_chained(k_density_list<false>, lb, kListBlock, 0, s, L, pos, vel, rec, aux, bnd, nbr, nbr_count, sk);
             e = launch_walk_queue(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, walk_sched,
                                   kc.walk_staging != 0, s);
             if (e != cudaSuccess) return e;
