@@ -528,7 +528,6 @@ Model::~Model() {
     cudaFree(skin.stale);
     cudaFree(skin.ctl);
     cudaFree(skin.queue);
-    cudaFree(skin.seg_n);
     cudaFree(skin.wcount);
     cudaFree(scratch);
     cudaFree(err);
@@ -645,7 +644,6 @@ int Model::alloc_skin() {
         cudaMalloc(&s.stale, scenes.size() * sizeof(uint32_t)) != cudaSuccess ||
         cudaMalloc(&s.ctl, scenes.size() * kSkinCtl * sizeof(uint32_t)) != cudaSuccess ||
         cudaMalloc(&s.queue, N * sizeof(uint32_t)) != cudaSuccess ||
-        cudaMalloc(&s.seg_n, ((N + 127) / 128) * sizeof(uint32_t)) != cudaSuccess ||
         cudaMalloc(&s.wcount, 2 * sizeof(uint32_t)) != cudaSuccess) {
         cudaGetLastError();  // out of memory is not sticky: clear it and go on without lists
         cudaFree(s.list);
@@ -657,7 +655,6 @@ int Model::alloc_skin() {
         cudaFree(s.stale);
         cudaFree(s.ctl);
         cudaFree(s.queue);
-        cudaFree(s.seg_n);
         cudaFree(s.wcount);
         return VFS_OK;
     }

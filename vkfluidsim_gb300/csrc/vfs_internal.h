@@ -160,11 +160,9 @@ struct SkinLists {
                                   // index (w, as bits), written by the cell pass
     uint32_t* stale = nullptr;    // per scene: nonzero when some particle moved past h skin / 2
     uint32_t* ctl = nullptr;      // per scene, kSkinCtl words: the build policy's state (kCtl*)
-    uint32_t* queue = nullptr;    // the particles the density pass walks this substep; a batch's of
-                                  // list block b at [128 b, 128 b + seg_n[b]), in index order
-    uint32_t* seg_n = nullptr;    // batched: per list block (128 particles) its walkers
-    uint32_t* wcount = nullptr;   // two words: a single scene's walkers in `queue`, packed from 0;
-                                  // nonzero when some scene's build is due this substep
+    uint32_t* queue = nullptr;    // the particles the list pass leaves to a walk, packed from 0
+    uint32_t* wcount = nullptr;   // two words: the walkers in `queue`; nonzero when some scene's
+                                  // build is due this substep
     uint32_t cap = 0;             // slots per particle
 };
 constexpr uint32_t kSkinUsable = 1u << 31;

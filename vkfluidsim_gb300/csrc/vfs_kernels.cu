@@ -791,13 +791,16 @@ __device__ __forceinline__ float in_range2(const float4& xi, const float4& xj) {
     return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
 }
 
-// Threads per block of the density pass over the skin lists; the walk queue is kept in segments of
-// one such block.
+// Threads per block of the density pass over the skin lists.
 constexpr int kListBlock = 128;
 
 // A single scene's queue of at least this many walkers is walked in runs of 32 (where one wave of
 // warps, ~2,400, has three particles each to walk a warp per walker); a smaller one a warp per walker.
+// A batch's queue is walked a thread per walker above kBatchCrowd (64 scenes, 1.1M particles, density
+// passes of 32 substeps with 10,000 to 44,000 walkers: 7.90 ms always per thread, 7.50 with the line at
+// 16,384 or 32,768, 8.14 at 65,536).
 constexpr uint32_t kWalkerCrowd = 8192;
+constexpr uint32_t kBatchCrowd = 16384;
 
 // 1 / sqrt(x) for a normal x (the form without ftz spends four more instructions on denormals).
 __device__ __forceinline__ float rsqrt_normal(float x) {
@@ -1621,20 +1624,27 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
     // the launch's counter (sched[0]), until none is left. Walks differ widely in length (the
     // queued walkers of a batch, dense and sparse regions), and a warp that finishes early takes
     // the next run.
-    const uint32_t runs = (L.total + 31u) / 32u;
+    uint32_t slots = L.total;
     const uint32_t warps = gridDim.x * (uint32_t)(kNbrBlock / 32);
+    if (kBatch && sk.list) {
+        slots = min(*sk.wcount, L.total);
+        if (slots == 0u) chained_release();
+        if (slots <= kBatchCrowd) {
+            for (uint32_t k = blockIdx.x * (uint32_t)(kNbrBlock / 32) + (uint32_t)(tid >> 5); k < slots; k += warps) {
+                const uint32_t i = __ldg(sk.queue + k);
+                walk_by_warp(scene_params<kBatch>(L, i), i, L.total, pos, vel, rec, scan, aux, bnd, nbr, nbr_count,
+                             L.host_dens, L.defer_vel);
+            }
+            return;
+        }
+    }
+    const uint32_t runs = (slots + 31u) / 32u;
     uint32_t run = blockIdx.x * (uint32_t)(kNbrBlock / 32) + (uint32_t)(tid >> 5);
     for (; run < runs;) {
         const uint32_t t = run * 32u + lane;
-        bool act = t < L.total;
+        const bool act = t < slots;
         uint32_t i = act ? t : 0u;
-        if (kBatch && act && sk.list) {
-            // Slot t of the queue: valid below its list block's count of walkers.
-            if (t % kListBlock >= __ldg(sk.seg_n + t / kListBlock))
-                act = false;
-            else
-                i = __ldg(sk.queue + t);
-        }
+        if (kBatch && act && sk.list) i = __ldg(sk.queue + t);
         // The next run, claimed now so that the counter's latency hides behind this one.
         uint32_t next = 0u;
         if (lane == 0u) next = warps + atomicAdd(sched, 1u);
@@ -1780,9 +1790,8 @@ __global__ void __launch_bounds__(kListBlock, 9)
                            bnd, nbr_count, L.host_dens, L.defer_vel);
         }
     }
-    // The walkers go to the queue in index order within the block: batched, to this block's
-    // segment (k_walk takes slot t below its segment's count); a single scene, packed from 0
-    // in blocks claimed by one atomic each (k_walk_queue's slots).
+    // The walkers go to the queue, packed from 0 in blocks claimed by one atomic each, in index order
+    // within the block.
     __shared__ uint32_t s_cnt[kListBlock / 32];
     __shared__ uint32_t s_base;
     const uint32_t m = __ballot_sync(0xffffffffu, walk);
@@ -1795,14 +1804,9 @@ __global__ void __launch_bounds__(kListBlock, 9)
         base += w < warp ? s_cnt[w] : 0u;
         total += s_cnt[w];
     }
-    if (kBatch) {
-        base += blockIdx.x * kListBlock;
-        if (threadIdx.x == 0) sk.seg_n[blockIdx.x] = total;
-    } else {
-        if (threadIdx.x == 0) s_base = total ? atomicAdd(sk.wcount, total) : 0u;
-        __syncthreads();
-        base += s_base;  // at most L.total walkers in all: the slots stay inside the queue
-    }
+    if (threadIdx.x == 0) s_base = total ? atomicAdd(sk.wcount, total) : 0u;
+    __syncthreads();
+    base += s_base;  // at most L.total walkers in all: the slots stay inside the queue
     if (walk) sk.queue[base + (uint32_t)__popc(m & ((1u << lane) - 1u))] = i;
 }
 
