@@ -3,6 +3,8 @@ the one ahead of it ends. The same work with an event between any two phases (pr
 and a captured sort replayed on new keys, give the same bits."""
 from __future__ import annotations
 
+from dataclasses import replace
+
 import numpy as np
 import pytest
 
@@ -22,6 +24,23 @@ def test_substeps_equal_substeps_with_events_between(side, fast):
     b.profile_substeps(12)
     for x, y in zip(a.get_neighbor_arrays(), b.get_neighbor_arrays()):
         assert np.array_equal(x, y)
+    sa, sb = a.copy_data_buffers(), b.copy_data_buffers()
+    for k in sa:
+        assert np.array_equal(sa[k], sb[k]), k
+
+
+@pytest.mark.parametrize("side", [12, 36])
+def test_runs_equal_single_substeps(side):
+    """Runs replay graphs of four substeps and the rest one by one; a parameter change in between
+    captures both again."""
+    w = W.dam_break(dims=(side,) * 3, spacing=0.02, box=(side * 0.03,) * 3, map_res=0, jitter=0.3, seed=side)
+    a, b = W.build_model(w), W.build_model(w)
+    for count in (1, 3, 4, 5, 11):
+        a.substeps(count)
+        for _ in range(count):
+            b.substeps(1)
+        for m in (a, b):
+            m.set_parameters(wcsph=replace(w.wcsph, stiffness=40.0 + count))
     sa, sb = a.copy_data_buffers(), b.copy_data_buffers()
     for k in sa:
         assert np.array_equal(sa[k], sb[k]), k

@@ -111,7 +111,8 @@ struct Model {
     uint64_t substeps_done = 0;  // substeps run by run_substeps (the snapshot sidecar's counter)
     bool use_graph = true;
     bool stepped = false;
-    cudaGraphExec_t graph_exec = nullptr;
+    cudaGraphExec_t graph_exec = nullptr;  // one substep
+    cudaGraphExec_t run_graph = nullptr;   // several (run_substeps)
 
     ~Model();
     int init();
@@ -123,6 +124,7 @@ struct Model {
     SkinLists active_skin() const;
     int enqueue_substep(cudaEvent_t* ev);
     int run_substeps(int count);
+    int capture_substeps(int count, cudaGraphExec_t* exec);
     int check_device();
     // Scene-relative state I/O (offset and ids are scene-local).
     int set_state(uint32_t scene, const float* pos3, const float* vel3, uint32_t offset,
