@@ -2454,13 +2454,15 @@ __global__ void __launch_bounds__(256)
 // word. The incremental sort and the cell starts cost such a model six launches and 39 to 44 us under
 // ncu, nearly all of it launch and dependent-load latency (8 bytes a particle take under a
 // microsecond to move); this kernel and the gather take 15 us at 5,000 particles, 26 at 47,000 (30
-// with eight blocks), 28 at 65,536: block barriers, cluster barriers (seven) and the ranking of up to
-// four items per thread. More than 65,536 particles would need two words an item.
+// with eight blocks), 28 at 65,536: block barriers, cluster barriers (five, a microsecond or so each:
+// seven made the substep of 17,576 particles 38.5 us instead of 36.7) and the ranking of up to four items
+// per thread. More than 65,536 particles would need two words an item.
 // Block c holds positions [c S, c S + S) of the array being sorted, S = ceil(n / blocks / 32) 32. Each of one
 // or two LSD passes ranks its items as k_onesweep does (per-warp histograms, match.any), exchanges
 // the blocks' digit counts, and stores every item straight into its place in the owner's shared
 // memory. The heads of equal keys are then stored into a table over the keys, and a suffix minimum
-// over it gives every key's first position.
+// over it gives every key's first position; what a block's last keys take from the blocks after it,
+// the element where the owner of the keys changes has stored into its `s_rest`.
 constexpr uint32_t kSmallSort = 65536;
 
 template <bool kBatch, bool kHostIn, int kBlocks, int ITEMS>
@@ -2476,7 +2478,7 @@ __global__ void __launch_bounds__(1024, 1)
     uint32_t* const s_buf = s_mem;                      // [2][kSeg] key << 16 | index
     uint32_t* const s_head = s_mem + 2 * kSeg;          // [kSeg] first position of each key of this block's
     uint32_t* const s_whist = s_mem + 3 * kSeg;         // [32][256] per-warp digit counts, then prefixes
-    __shared__ uint32_t s_cnt[256], s_base[256], s_warp[32], s_min;
+    __shared__ uint32_t s_cnt[256], s_base[256], s_warp[32], s_rest;
     __shared__ float s_p[kHostIn ? 3072 : 1];
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t n = L.total, c = cluster.block_rank();
@@ -2513,6 +2515,7 @@ __global__ void __launch_bounds__(1024, 1)
         if (t < mine) s_buf[t] = particle_key<kBatch>(L, i, x) << 16 | i;
     }
     for (uint32_t k = tid; k < S; k += 1024u) s_head[k] = 0xFFFFFFFFu;
+    if (tid == 0u) s_rest = n;
     const uint32_t bins = 1u << digit_bits, mask = bins - 1u;
     uint32_t* cur = s_buf;
     uint32_t* nxt = s_buf + kSeg;
@@ -2597,8 +2600,9 @@ __global__ void __launch_bounds__(1024, 1)
         cur = nxt;
         nxt = t;
     }
-    // The sorted arrays, and the heads of equal keys into the table of their keys' owner (owner b
-    // holds keys [b S, b S + S)).
+    // The sorted arrays; the heads of equal keys into the table of their keys' owner (owner b holds keys
+    // [b S, b S + S)); and, where the owner changes, the position into the owners passed: the first
+    // past all their keys.
     for (uint32_t t = tid; t < mine; t += 1024u) {
         const uint32_t i = first + t, key = cur[t] >> 16;
         skeys[i] = key;
@@ -2609,9 +2613,10 @@ __global__ void __launch_bounds__(1024, 1)
         if (key != before) {
             const uint32_t b = __umulhi(key, magic);
             cluster.map_shared_rank(s_head, b)[key - b * S] = i;
+            for (uint32_t q = i ? __umulhi(before, magic) : 0u; q < b; q++) *cluster.map_shared_rank(&s_rest, q) = i;
         }
     }
-    cluster.sync();
+    cluster.sync();  // the last use of other blocks' shared memory is behind it
     // scan[k] = the smallest head of the keys >= k (n when none): a suffix minimum, ITEMS keys a thread.
     uint32_t h[ITEMS];
     uint32_t low = 0xFFFFFFFFu;
@@ -2629,14 +2634,7 @@ __global__ void __launch_bounds__(1024, 1)
     }
     if (lane == 0u) s_warp[warp] = after;
     __syncthreads();
-    if (tid == 0u) {
-        uint32_t m = 0xFFFFFFFFu;
-        for (uint32_t w = 0; w < 32u; w++) m = min(m, s_warp[w]);
-        s_min = m;
-    }
-    cluster.sync();
-    uint32_t rest = n;
-    for (uint32_t b = c + 1u; b < (uint32_t)kBlocks; b++) rest = min(rest, *cluster.map_shared_rank(&s_min, b));
+    uint32_t rest = s_rest;
     for (uint32_t w = warp + 1u; w < 32u; w++) rest = min(rest, s_warp[w]);
     const uint32_t later = __shfl_down_sync(0xffffffffu, after, 1);
     if (lane < 31u) rest = min(rest, later);
@@ -2646,7 +2644,6 @@ __global__ void __launch_bounds__(1024, 1)
         if (k < S && first + k < n) scan[first + k] = min(h[it], rest);
     }
     if (c == 0u && tid == 0u) scan[n] = n;
-    cluster.sync();  // no block leaves while another may read its shared memory
 }
 
 constexpr int kSortBlock = 256;
