@@ -629,7 +629,8 @@ struct Rollout {
 
     // Recomputes `len` substeps from the state in the model, keeping each substep's permutation,
     // force records (the sorted inputs among them), density products and neighbour lists: the model's buffers for those are pointed
-    // at the segment's per-substep records, so the passes write them in place.
+    // at the segment's per-substep records, so the passes write them in place (a copy of the permutation
+    // after each substep cost 2 us of it and a break in the chain of launches).
     int record_segment(int len) {
         if (m->nbr_cap != cap)
             return fail(VFS_ERR_INVALID_ARGUMENT, "the model's neighbour capacity changed after the rollout was created");
@@ -638,6 +639,7 @@ struct Rollout {
         float4* own_rec = m->rec;
         uint32_t* own_nbr = m->nbr;
         uint32_t* own_cnt = m->nbr_count;
+        uint32_t* own_perm = m->sp_buf;
         int rc = VFS_OK;
         for (int t = 0; t < len && rc == VFS_OK; t++) {
             m->aux = s_aux[t];
@@ -645,12 +647,15 @@ struct Rollout {
             m->rec = s_rec[t];
             m->nbr = s_nbr[t];
             m->nbr_count = s_cnt[t];
+            m->sp_buf = s_perm[t];
             rc = m->enqueue_substep(nullptr);
-            if (rc == VFS_OK) {
-                const cudaError_t e = cudaMemcpyAsync(s_perm[t], m->sperm, (size_t)m->n * 4,
-                                                      cudaMemcpyDeviceToDevice, m->stream);
-                if (e != cudaSuccess) rc = fail(VFS_ERR_CUDA, cudaGetErrorString(e));
-            }
+        }
+        // The last permutation stays the model's (get_neighbor_arrays).
+        m->sp_buf = m->sperm = own_perm;
+        if (rc == VFS_OK && len > 0) {
+            const cudaError_t e = cudaMemcpyAsync(own_perm, s_perm[len - 1], (size_t)m->n * 4,
+                                                  cudaMemcpyDeviceToDevice, m->stream);
+            if (e != cudaSuccess) rc = fail(VFS_ERR_CUDA, cudaGetErrorString(e));
         }
         m->aux = own_aux;
         m->bnd = own_bnd;
