@@ -1617,9 +1617,13 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
     __shared__ uint32_t s_j[kListCap * kNbrBlock];
     const int tid = threadIdx.x;
     const uint32_t lane = (uint32_t)(tid & 31);
-    // The force pass's blocks likewise: not beside a batch's walk (64 scenes: 27.1 ms, late 25.7).
-    if (!kBatch) chained_release();
-    if (!kBatch && sk.list && sums_lists(sk)) return;
+    // The force pass's blocks beside a walk run with what on-chip memory its lists leave as L1: let in
+    // only where there is nothing to walk (64 scenes 27.1 ms, late 25.7; 87,386 particles walking 111 us a
+    // substep, late 106).
+    if (!kBatch && sk.list && sums_lists(sk)) {
+        chained_release();
+        return;
+    }
     // Every warp takes runs of 32 slots: first the run of its own index, then runs claimed from
     // the launch's counter (sched[0]), until none is left. Walks differ widely in length (the
     // queued walkers of a batch, dense and sparse regions), and a warp that finishes early takes
