@@ -523,6 +523,7 @@ struct Rollout {
     uint32_t cap = 0;  // neighbour slots per particle of the segment records (the model's at creation)
     bool last_recorded = false;  // the segment records hold the last segment (set by forward)
     cudaGraphExec_t seg_graph = nullptr;  // recompute + reverse of one full segment
+    uint64_t seg_epoch = 0;               // the model's graph_epoch at its capture
 
     ~Rollout() {
         if (seg_graph) cudaGraphExecDestroy(seg_graph);
@@ -627,13 +628,19 @@ struct Rollout {
         return VFS_OK;
     }
 
+    int check_capacity() const {
+        if (m->nbr_cap != cap)
+            return fail(VFS_ERR_INVALID_ARGUMENT, "the model's neighbour capacity changed after the rollout was created");
+        return VFS_OK;
+    }
+
     // Recomputes `len` substeps from the state in the model, keeping each substep's permutation,
     // force records (the sorted inputs among them), density products and neighbour lists: the model's buffers for those are pointed
     // at the segment's per-substep records, so the passes write them in place (a copy of the permutation
     // after each substep cost 2 us of it and a break in the chain of launches).
     int record_segment(int len) {
-        if (m->nbr_cap != cap)
-            return fail(VFS_ERR_INVALID_ARGUMENT, "the model's neighbour capacity changed after the rollout was created");
+        const int rc_cap = check_capacity();
+        if (rc_cap) return rc_cap;
         float4* own_aux = m->aux;
         float4* own_bnd = m->bnd;
         float4* own_rec = m->rec;
@@ -672,10 +679,19 @@ struct Rollout {
         return rc;
     }
 
-    // Full segments replay one captured graph; a shorter last segment runs without one.
+    // Full segments replay one captured graph; a shorter last segment runs without one. The graph
+    // holds the model's parameters and the addresses of its buffers, so it is captured again once
+    // the model's own graphs have been dropped for a change of either.
     int run_segment(int len) {
         if (len != every) return segment_body(len);
+        const int rc_cap = check_capacity();
+        if (rc_cap) return rc_cap;
+        if (seg_graph && seg_epoch != m->graph_epoch) {
+            cudaGraphExecDestroy(seg_graph);
+            seg_graph = nullptr;
+        }
         if (!seg_graph) {
+            seg_epoch = m->graph_epoch;
             cudaGraph_t g = nullptr;
             VFS_ADJ_TRY(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
             const int rc = segment_body(len);

@@ -334,6 +334,7 @@ int Model::refresh_params() {
 }
 
 void Model::invalidate_graph() {
+    graph_epoch++;
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     graph_exec = nullptr;
     if (run_graph) cudaGraphExecDestroy(run_graph);

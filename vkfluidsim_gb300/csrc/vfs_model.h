@@ -113,6 +113,7 @@ struct Model {
     bool stepped = false;
     cudaGraphExec_t graph_exec = nullptr;  // one substep
     cudaGraphExec_t run_graph = nullptr;   // several (run_substeps)
+    uint64_t graph_epoch = 0;              // counts invalidate_graph (for graphs held elsewhere)
 
     ~Model();
     int init();
