@@ -610,8 +610,9 @@ __global__ void __launch_bounds__(kCellBlock)
                     uint32_t* __restrict__ pkeys_out, uint32_t* guess,
                     const uint32_t* __restrict__ b_of_id, float4* __restrict__ xcur,
                     const float4* __restrict__ x_build, uint32_t* __restrict__ stale,
-                    const uint32_t* __restrict__ ctl, uint32_t* __restrict__ wcount) {
-    VFS_CHAINED();
+                    const uint32_t* __restrict__ ctl, uint32_t* __restrict__ wcount, bool late) {
+    VFS_CHAINED_LATE();
+    if (!late) chained_release();
     __shared__ uint32_t s_lo, s_hi;
     if (wcount && blockIdx.x == 0 && threadIdx.x == 0) wcount[0] = 0u;  // the list pass's queue
     // The sort is done with its scratch (histograms, tile counters, look-back status): clear it
@@ -2901,28 +2902,6 @@ cudaError_t launch_vel_records(uint32_t n, const uint32_t* perm, const float* ve
     return cudaGetLastError();
 }
 
-cudaError_t launch_cells_reorder(const StepLaunch& L, uint32_t n, const uint32_t* skeys, const uint32_t* perm,
-                                 uint32_t* cell_scan, const float4* pos_in, const float4* vel_in,
-                                 float4* pos_out, float4* vel_out, uint32_t* zero,
-                                 uint32_t zero_words, uint32_t* pkeys_out, uint32_t* guess,
-                                 const SkinLists& sk, const KernelConfig& kc, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    switch (kc.cell_block) {
-        case 128:
-            launch_chained(k_cells_reorder<128>, (n + 128u) / 128u, 128, 0, s, L, n, skeys, perm, cell_scan, pos_in,
-                                                                 vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl, sk.wcount);
-            break;
-        case 512:
-            launch_chained(k_cells_reorder<512>, (n + 512u) / 512u, 512, 0, s, L, n, skeys, perm, cell_scan, pos_in,
-                                                                 vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl, sk.wcount);
-            break;
-        default:
-            launch_chained(k_cells_reorder<256>, (n + 256u) / 256u, 256, 0, s, L, n, skeys, perm, cell_scan, pos_in,
-                                                                 vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl, sk.wcount);
-    }
-    return cudaGetLastError();
-}
-
 // SMs of the current device (0 if unknown), cached per device.
 static int sm_count() {
     static std::atomic<int> sms[16];
@@ -2934,6 +2913,33 @@ static int sm_count() {
         sms[dev].store(n, std::memory_order_relaxed);
     }
     return n;
+}
+
+cudaError_t launch_cells_reorder(const StepLaunch& L, uint32_t n, const uint32_t* skeys, const uint32_t* perm,
+                                 uint32_t* cell_scan, const float4* pos_in, const float4* vel_in,
+                                 float4* pos_out, float4* vel_out, uint32_t* zero,
+                                 uint32_t zero_words, uint32_t* pkeys_out, uint32_t* guess,
+                                 const SkinLists& sk, const KernelConfig& kc, cudaStream_t s) {
+    if (n == 0) return cudaSuccess;
+    // Without lists the walk comes next. Less than a resident wave of its blocks (768 threads an SM in
+    // most of its shapes), let in while this kernel fills the SMs unevenly, crowds a few of them: us a
+    // substep let in early and late, 71,402 particles 110.4 / 99.4, 90,000 112.6 / 109.4, 110,000 117.4 /
+    // 116.8, 150,000 173.7 / 175.4.
+    const bool late = !sk.list && n < (uint32_t)sm_count() * 768u;
+    switch (kc.cell_block) {
+        case 128:
+            launch_chained(k_cells_reorder<128>, (n + 128u) / 128u, 128, 0, s, L, n, skeys, perm, cell_scan, pos_in,
+                                                                 vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl, sk.wcount, late);
+            break;
+        case 512:
+            launch_chained(k_cells_reorder<512>, (n + 512u) / 512u, 512, 0, s, L, n, skeys, perm, cell_scan, pos_in,
+                                                                 vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl, sk.wcount, late);
+            break;
+        default:
+            launch_chained(k_cells_reorder<256>, (n + 256u) / 256u, 256, 0, s, L, n, skeys, perm, cell_scan, pos_in,
+                                                                 vel_in, pos_out, vel_out, zero, zero_words, pkeys_out, guess, sk.b_of_id, sk.xcur, sk.x_build, sk.stale, sk.ctl, sk.wcount, late);
+    }
+    return cudaGetLastError();
 }
 
 constexpr size_t kTileSmemBytes = kTileWarps * sizeof(TileSmem);
