@@ -372,7 +372,8 @@ __global__ void k_lookback_selftest(const uint32_t* status, int bins, uint32_t s
 // One stable LSD radix pass (onesweep: Adinets & Merrill 2022). Tiles are claimed in launch
 // order through an atomic counter, so every predecessor of a tile is already resident and the
 // bounded look-back always terminates; a timeout sets an error bit instead of hanging.
-template <int BLOCK, int ITEMS>
+// kMatch: ranked by match.any instead of ballots (launch_onesweep_t).
+template <int BLOCK, int ITEMS, bool kMatch>
 __global__ void __launch_bounds__(BLOCK)
     k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n,
@@ -421,14 +422,18 @@ __global__ void __launch_bounds__(BLOCK)
         const uint32_t idx = base + it * 32u + lane;
         const bool valid = idx < n;
         const uint32_t d = valid ? ((k[it] >> shift) & mask) : (uint32_t)bins;
-        // Lanes with the same digit, a ballot per bit (one more than a digit's: the invalid lanes'):
-        // eight independent votes take less than a match.any (4M pairs: 309 against 336 us).
+        // Lanes with the same digit. A ballot per bit (one more than a digit's: the invalid lanes'):
+        // eight independent votes take less than a match.any in a sort that fills the GPU (4M pairs:
+        // 309 against 336 us).
         uint32_t peers = 0xffffffffu;
-        for (int b = 0; b <= bits; b++) {
-            const bool bit = (d >> b) & 1u;
-            const uint32_t vote = __ballot_sync(0xffffffffu, bit);
-            peers &= bit ? vote : ~vote;
-        }
+        if (kMatch)
+            peers = __match_any_sync(0xffffffffu, d);
+        else
+            for (int b = 0; b <= bits; b++) {
+                const bool bit = (d >> b) & 1u;
+                const uint32_t vote = __ballot_sync(0xffffffffu, bit);
+                peers &= bit ? vote : ~vote;
+            }
         const uint32_t pre = __popc(peers & lt_mask);
         uint32_t prev = 0u;
         if (valid) prev = s_whist[warp][d];
@@ -2463,7 +2468,7 @@ __global__ void __launch_bounds__(256)
 // seven made the substep of 17,576 particles 38.5 us instead of 36.7) and the ranking of up to four items
 // per thread. More than 65,536 particles would need two words an item.
 // Block c holds positions [c S, c S + S) of the array being sorted, S = ceil(n / blocks / 32) 32. Each of one
-// or two LSD passes ranks its items as k_onesweep does (per-warp histograms, match.any), exchanges
+// or two LSD passes ranks its items as the moved particles' sort does (per-warp histograms, match.any), exchanges
 // the blocks' digit counts, and stores every item straight into its place in the owner's shared
 // memory. The heads of equal keys are then stored into a table over the keys, and a suffix minimum
 // over it gives every key's first position; what a block's last keys take from the blocks after it,
@@ -2657,7 +2662,13 @@ template <int ITEMS>
 cudaError_t launch_onesweep_t(uint32_t n, const SortConfig& sc, const SortScratch& scr, int pass,
                               const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
                               uint32_t* vout, const uint32_t* n_dev, cudaStream_t s) {
-    launch_chained(k_onesweep<kSortBlock, ITEMS>, sc.tiles, kSortBlock, 0, s, kin, vin, kout, vout, n, pass * sc.digit_bits, sc.bins, scr.ghist + pass * sc.bins,
+    // The few moved particles of a substep (*n_dev of n) are one tile's chain or a few, where match.any is
+    // shorter than ballots: us a substep by ballots and match.any, 66,751 particles 88.7 / 85.7, 83,607
+    // 84.7 / 79.8, 150,000 172.5 / 168.7, 1M 646.6 / 644.6. Above kMatchMost that is lost beside a substep
+    // of milliseconds, and a whole new state (every particle moved) sorts the sooner by ballots.
+    constexpr uint32_t kMatchMost = 1u << 21;
+    auto* const kernel = n_dev && n <= kMatchMost ? k_onesweep<kSortBlock, ITEMS, true> : k_onesweep<kSortBlock, ITEMS, false>;
+    launch_chained(kernel, sc.tiles, kSortBlock, 0, s, kin, vin, kout, vout, n, pass * sc.digit_bits, sc.bins, scr.ghist + pass * sc.bins,
         scr.counters + pass, scr.status + (size_t)pass * sc.tiles * sc.bins, scr.err, n_dev);
     return cudaGetLastError();
 }
