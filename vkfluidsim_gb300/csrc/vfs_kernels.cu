@@ -1718,8 +1718,9 @@ template <bool kBatch>
 __global__ void __launch_bounds__(kListBlock, 9)
     k_density_list(StepLaunch L, const float4* __restrict__ pos, const float4* __restrict__ vel,
                    float4* __restrict__ rec, float4* __restrict__ aux, float4* __restrict__ bnd,
-                   uint32_t* __restrict__ nbr, uint32_t* __restrict__ nbr_count, SkinLists sk) {
-    VFS_CHAINED();
+                   uint32_t* __restrict__ nbr, uint32_t* __restrict__ nbr_count, SkinLists sk, bool late) {
+    VFS_CHAINED_LATE();
+    if (!late) chained_release();
     __shared__ uint32_t s_ring[8 * kListBlock];
     const uint32_t i = blockIdx.x * kListBlock + threadIdx.x;
     // A single scene that is stale and waits, or whose last build left most lists unusable: k_walk walks
@@ -2926,17 +2927,19 @@ static int sm_count() {
     return n;
 }
 
+// A walk of n particles has less than a resident wave of blocks (768 threads an SM in most of its
+// shapes). Let in while the kernel before it fills the SMs unevenly, they crowd a few of them.
+static bool walk_below_wave(uint32_t n) { return n < (uint32_t)sm_count() * 768u; }
+
 cudaError_t launch_cells_reorder(const StepLaunch& L, uint32_t n, const uint32_t* skeys, const uint32_t* perm,
                                  uint32_t* cell_scan, const float4* pos_in, const float4* vel_in,
                                  float4* pos_out, float4* vel_out, uint32_t* zero,
                                  uint32_t zero_words, uint32_t* pkeys_out, uint32_t* guess,
                                  const SkinLists& sk, const KernelConfig& kc, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    // Without lists the walk comes next. Less than a resident wave of its blocks (768 threads an SM in
-    // most of its shapes), let in while this kernel fills the SMs unevenly, crowds a few of them: us a
-    // substep let in early and late, 71,402 particles 110.4 / 99.4, 90,000 112.6 / 109.4, 110,000 117.4 /
-    // 116.8, 150,000 173.7 / 175.4.
-    const bool late = !sk.list && n < (uint32_t)sm_count() * 768u;
+    // Without lists the walk comes next: us a substep let in early and late, 71,402 particles 110.4 /
+    // 99.4, 90,000 112.6 / 109.4, 110,000 117.4 / 116.8, 150,000 173.7 / 175.4.
+    const bool late = !sk.list && walk_below_wave(n);
     switch (kc.cell_block) {
         case 128:
             launch_chained(k_cells_reorder<128>, (n + 128u) / 128u, 128, 0, s, L, n, skeys, perm, cell_scan, pos_in,
@@ -3080,9 +3083,13 @@ cudaError_t launch_density(const StepLaunch& L, const float4* pos, const float4*
         if (e != cudaSuccess) return e;
         const uint32_t lb = (L.total + kListBlock - 1) / kListBlock;
         if (batch) {
-            launch_chained(k_density_list<true>, lb, kListBlock, 0, s, L, pos, vel, rec, aux, bnd, nbr, nbr_count, sk);
+            // The walk comes next, as after launch_cells_reorder's pass: us a substep let in early and late,
+            // 13 scenes of 1,579 to 23,237 particles 184 / 172, 8 of up to 20,766 232 / 223 (the batches' host
+            // copies included).
+            const bool late = walk_below_wave(L.total);
+            launch_chained(k_density_list<true>, lb, kListBlock, 0, s, L, pos, vel, rec, aux, bnd, nbr, nbr_count, sk, late);
         } else {
-            launch_chained(k_density_list<false>, lb, kListBlock, 0, s, L, pos, vel, rec, aux, bnd, nbr, nbr_count, sk);
+            launch_chained(k_density_list<false>, lb, kListBlock, 0, s, L, pos, vel, rec, aux, bnd, nbr, nbr_count, sk, false);
             e = launch_walk_queue(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, walk_sched,
                                   kc.walk_staging != 0, s);
             if (e != cudaSuccess) return e;
