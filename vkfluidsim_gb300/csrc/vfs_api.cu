@@ -670,7 +670,7 @@ int Model::alloc_skin() {
         cudaMalloc(&s.stale, scenes.size() * sizeof(uint32_t)) != cudaSuccess ||
         cudaMalloc(&s.ctl, scenes.size() * kSkinCtl * sizeof(uint32_t)) != cudaSuccess ||
         cudaMalloc(&s.queue, N * sizeof(uint32_t)) != cudaSuccess ||
-        cudaMalloc(&s.wcount, 2 * sizeof(uint32_t)) != cudaSuccess) {
+        cudaMalloc(&s.wcount, 3 * sizeof(uint32_t)) != cudaSuccess) {
         cudaGetLastError();  // out of memory is not sticky: clear it and go on without lists
         cudaFree(s.list);
         cudaFree(s.count);
@@ -687,7 +687,6 @@ int Model::alloc_skin() {
     VFS_CUDA_TRY(cudaMemset(s.count, 0, N * sizeof(uint32_t)));
     VFS_CUDA_TRY(cudaMemset(s.b_of_id, 0, N * sizeof(uint32_t)));  // any index below n until a build
     VFS_CUDA_TRY(cudaMemset(s.stale, 0, scenes.size() * sizeof(uint32_t)));
-    VFS_CUDA_TRY(cudaMemset(s.wcount, 0, 2 * sizeof(uint32_t)));
     skin = s;
     return invalidate_skin();
 }
@@ -698,6 +697,7 @@ int Model::alloc_skin() {
 int Model::invalidate_skin() {
     if (!skin.x_build) return VFS_OK;
     VFS_CUDA_TRY(cudaMemsetAsync(skin.x_build, 0x7F, (size_t)n * sizeof(float4), stream));
+    VFS_CUDA_TRY(cudaMemsetAsync(skin.wcount, 0, 3 * sizeof(uint32_t), stream));
     std::vector<uint32_t> ctl(scenes.size() * kSkinCtl, 0u);
     for (size_t s = 0; s < scenes.size(); s++) ctl[s * kSkinCtl + kCtlAllow] = 1u;
     VFS_CUDA_TRY(cudaMemcpyAsync(skin.ctl, ctl.data(), ctl.size() * sizeof(uint32_t),

@@ -161,8 +161,8 @@ struct SkinLists {
     uint32_t* stale = nullptr;    // per scene: nonzero when some particle moved past h skin / 2
     uint32_t* ctl = nullptr;      // per scene, kSkinCtl words: the build policy's state (kCtl*)
     uint32_t* queue = nullptr;    // the particles the list pass leaves to a walk, packed from 0
-    uint32_t* wcount = nullptr;   // two words: the walkers in `queue`; nonzero when some scene's
-                                  // build is due this substep
+    uint32_t* wcount = nullptr;   // three words: the walkers in `queue`; nonzero when some scene's
+                                  // build is due this substep; nonzero when a batch's scenes all walk
     uint32_t cap = 0;             // slots per particle
 };
 constexpr uint32_t kSkinUsable = 1u << 31;
