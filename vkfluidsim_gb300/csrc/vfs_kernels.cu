@@ -1614,11 +1614,12 @@ __global__ void __launch_bounds__(kTileWarps * 32, 5)
 // exactly the force pass's neighbour set. It walks whole scenes in index order (no skin lists; a
 // single scene that is stale and may not rebuild, or whose lists are mostly unusable) and a batch's
 // queue. A single scene whose lists are summed returns at the kernel's top. One
-// resident wave whose warps claim runs of 32 slots. The tiles above are no faster for a fluid's ~43
+// resident wave whose warps claim runs of 32 slots; a single scene's shapes of 768 threads an SM are held
+// to the 72 registers that let 28 warps in (74, 24 warps: 130,000 particles walking 92 us, 72 76). The tiles above are no faster for a fluid's ~43
 // neighbours: 515 us against 450 us for 1M particles (their sum phase runs at 16 warps per SM, this
-// kernel at 24, and it tests only ~200 candidates per particle after pruning).
+// kernel at 27, and it tests only ~200 candidates per particle after pruning).
 template <bool kBatch, int kNbrBlock, int kMinBlocks>
-__global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
+__global__ void __launch_bounds__(kNbrBlock, kBatch || kMinBlocks * kNbrBlock > 768 ? kMinBlocks : 896 / kNbrBlock)
     k_walk(StepLaunch L, const float4* __restrict__ pos, const float4* __restrict__ vel,
            float4* __restrict__ rec, const uint32_t* __restrict__ scan,
            float4* __restrict__ aux, float4* __restrict__ bnd, uint32_t* __restrict__ nbr,
@@ -2945,7 +2946,7 @@ static int sm_count() {
     return n;
 }
 
-// A walk of n particles has less than a resident wave of blocks (768 threads an SM in most of its
+// A walk of n particles has less than a resident wave of blocks (768 to 896 threads an SM in most of its
 // shapes). Let in while the kernel before it fills the SMs unevenly, they crowd a few of them.
 static bool walk_below_wave(uint32_t n) { return n < (uint32_t)sm_count() * 768u; }
 
