@@ -235,12 +235,11 @@ int32_t vfs_model_get_neighbor_capacity(const vfs_model* m);
  * per particle) have no lists; the getter then reports 0. */
 int vfs_model_set_skin(vfs_model* m, float skin);
 int vfs_model_get_skin(const vfs_model* m, float* skin);
-/* Block-per-cell staging in the density pass's bucket walk (CalculateDensities,
- * wcsph_with_boundary_model.slang:153-197) where a crowd of a single scene's particles has no
- * usable skin list (a dense blob): a warp whose particles share a few rows of cells loads the
- * 3 x 3 rows of cells around them into shared memory once and tests every staged particle against
- * each of its own on the tensor cores, instead of a warp walking one particle's 27 buckets.
- * Results are bit-identical either way. On by default (vfs_tune_config.walk_staging). */
+/* Kept for programs that set it: the value is stored (vfs_tune_config.walk_staging, off by default) and
+ * has no effect, on a model or on a batch. Block-per-cell staging in shared memory of the density pass's
+ * bucket walk (CalculateDensities, wcsph_with_boundary_model.slang:153-197) was 1 to 21% slower than the
+ * walk without it in every workload measured; a dense crowd without usable skin lists is walked as
+ * staged tiles by itself. Results were and are the same bits. */
 int vfs_model_set_walk_staging(vfs_model* m, int32_t enable);
 /* Number of list builds so far (synchronises the handle's stream). */
 int vfs_model_get_skin_builds(vfs_model* m, uint32_t* builds);
@@ -312,7 +311,7 @@ typedef struct vfs_tune_config {
     int32_t cell_block;      /* keys per block of the cell-range / reorder kernel: 128, 256, 512 */
     int32_t force_block;     /* force pass: threads per block and minimum resident blocks per */
     int32_t force_min_blocks;/* SM, the same four shapes; 0, 0 = the neighbour passes' shape */
-    int32_t walk_staging;    /* block-per-cell staging of a crowd's density walk: 1 on, 0 off */
+    int32_t walk_staging;    /* 0 or 1, no effect (vfs_model_set_walk_staging) */
 } vfs_tune_config;
 /* Times every candidate of each stage (sort, neighbour passes, cell ranges) for `repeats`
  * substeps from the model's current state, keeps the fastest, and restores the state (the
@@ -364,7 +363,7 @@ int vfs_batch_profile_substeps(vfs_batch* b, int32_t count, float* phase_ms);
 int vfs_batch_set_sort_config(vfs_batch* b, int32_t digit_bits, int32_t tile_items);
 int vfs_batch_set_neighbor_capacity(vfs_batch* b, int32_t slots);
 int vfs_batch_set_skin(vfs_batch* b, float skin);
-int vfs_batch_set_walk_staging(vfs_batch* b, int32_t enable);
+int vfs_batch_set_walk_staging(vfs_batch* b, int32_t enable); /* no effect, as for a model */
 int vfs_batch_get_skin(const vfs_batch* b, float* skin);
 int vfs_batch_get_skin_builds(vfs_batch* b, uint32_t scene, uint32_t* builds);
 int vfs_batch_export_state(vfs_batch* b, int32_t scene, const char* path_prefix);

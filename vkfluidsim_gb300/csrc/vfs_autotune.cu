@@ -267,7 +267,7 @@ int tune_cache_load(const char* path) {
         char key[256];
         vfs_tune_config c{};
         // Lines of 6 values (no force shape) take the neighbour shape for the force pass; lines
-        // without the walk-staging value (6 or 8 values) walk a crowd without tiles.
+        // without the walk-staging value (6 or 8 values) have it off.
         c.walk_staging = 0;
         const int got = std::sscanf(line, "%255s %d %d %d %d %d %d %d %d", key, &c.sort_digit_bits,
                                     &c.sort_tile_items, &c.nbr_block, &c.nbr_min_blocks,

@@ -202,7 +202,7 @@ struct KernelConfig {
     int nbr_shape = kNbr96x8;     // density pass's per-thread walk (and the adjoint's recomputed forward)
     int force_shape = kNbr128x8;  // force pass (no shared memory: it takes the larger blocks)
     int cell_block = 256;  // keys per block of the cell-range / reorder kernel: 128, 256 or 512
-    int walk_staging = 1;  // a crowd of queued walkers is walked as staged tiles (0: a warp per walker)
+    int walk_staging = 0;  // read by nothing: the value a caller set (vfs_model_set_walk_staging)
 };
 size_t sort_scratch_words(const SortConfig& c);
 
@@ -277,7 +277,7 @@ bool planes_mode(uint32_t total);
 // Boundary volume + density + EOS epilogue; writes each particle's neighbour list.
 // Also writes rec[2i], rec[2i+1] = (x, y, z, p/rho^2), (v, m/max(rho, 1e-6)) for the force pass.
 // With skin lists (sk.list set): rebuilds flagged scenes, sums the lists where they are usable and
-// walks the rest (kc.walk_staging: see KernelConfig).
+// walks the rest.
 // walk_sched: two device words, zero between launches (the walk kernel's run counter, put back to
 // zero by its last warp).
 cudaError_t launch_density(const StepLaunch& L, const float4* pos, const float4* vel, float4* rec,

@@ -1516,7 +1516,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 5)
     k_walk_queue(StepLaunch L, const float4* __restrict__ pos, const float4* __restrict__ vel,
                  float4* __restrict__ rec, const uint32_t* __restrict__ scan,
                  float4* __restrict__ aux, float4* __restrict__ bnd, uint32_t* __restrict__ nbr,
-                 uint32_t* __restrict__ nbr_count, SkinLists sk, uint32_t* __restrict__ sched, bool tiles) {
+                 uint32_t* __restrict__ nbr_count, SkinLists sk, uint32_t* __restrict__ sched) {
     VFS_CHAINED();
     extern __shared__ __align__(16) unsigned char s_raw[];
     TileSmem& S = reinterpret_cast<TileSmem*>(s_raw)[threadIdx.x >> 5];
@@ -1525,7 +1525,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 5)
     if (!sums_lists(sk)) return;  // k_walk walks every particle
     const SceneParams& p = L.one;
     const uint32_t slots = min(*sk.wcount, L.total);
-    if (slots < kWalkerCrowd || !tiles) {
+    if (slots < kWalkerCrowd) {
         for (uint32_t k = blockIdx.x * (uint32_t)kTileWarps + (threadIdx.x >> 5); k < slots;
              k += gridDim.x * (uint32_t)kTileWarps)
             walk_by_warp(p, __ldg(sk.queue + k), L.total, pos, vel, rec, scan, aux, bnd, nbr, nbr_count,
@@ -3012,14 +3012,13 @@ cudaError_t launch_build(const StepLaunch& L, const float4* pos, const uint32_t*
 
 cudaError_t launch_walk_queue(const StepLaunch& L, const float4* pos, const float4* vel, float4* rec,
                               const uint32_t* cell_scan, float4* aux, float4* bnd, uint32_t* nbr,
-                              uint32_t* nbr_count, const SkinLists& sk, uint32_t* sched, bool tiles,
-                              cudaStream_t s) {
+                              uint32_t* nbr_count, const SkinLists& sk, uint32_t* sched, cudaStream_t s) {
     static std::atomic<int> per_sm[16];
     uint32_t blocks = 0u;
     const cudaError_t e = tile_blocks(k_walk_queue, per_sm, L.total, blocks);
     if (e != cudaSuccess) return e;
     launch_chained(k_walk_queue, blocks, kTileWarps * 32, kTileSmemBytes, s, L, pos, vel, rec, cell_scan, aux, bnd, nbr,
-                                                                 nbr_count, sk, sched, tiles);
+                                                                 nbr_count, sk, sched);
     return cudaGetLastError();
 }
 
@@ -3109,8 +3108,7 @@ cudaError_t launch_density(const StepLaunch& L, const float4* pos, const float4*
             launch_chained(k_density_list<true>, lb, kListBlock, 0, s, L, pos, vel, rec, aux, bnd, nbr, nbr_count, sk, late);
         } else {
             launch_chained(k_density_list<false>, lb, kListBlock, 0, s, L, pos, vel, rec, aux, bnd, nbr, nbr_count, sk, false);
-            e = launch_walk_queue(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, walk_sched,
-                                  kc.walk_staging != 0, s);
+            e = launch_walk_queue(L, pos, vel, rec, cell_scan, aux, bnd, nbr, nbr_count, sk, walk_sched, s);
             if (e != cudaSuccess) return e;
         }
     }

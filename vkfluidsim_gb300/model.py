@@ -489,7 +489,7 @@ class WCSPHWithBoundaryModel:
         check(self._lib.vfs_model_set_skin(self._h, skin))
 
     def set_walk_staging(self, enable: bool) -> None:
-        """Block-per-cell staging of a crowd's density walk (on by default; bit-identical results)."""
+        """Kept for programs that call it: no effect (staging made the density walk slower)."""
         check(self._lib.vfs_model_set_walk_staging(self._h, int(bool(enable))))
 
     def skin_builds(self) -> int:
@@ -725,6 +725,7 @@ class Batch:
         check(self._lib.vfs_batch_set_skin(self._h, skin))
 
     def set_walk_staging(self, enable: bool) -> None:
+        """Kept for programs that call it: no effect (staging made the density walk slower)."""
         check(self._lib.vfs_batch_set_walk_staging(self._h, int(bool(enable))))
 
     def skin_builds(self, scene: int) -> int:
