@@ -941,6 +941,13 @@ struct TileSmem {
     };
 };
 
+// Blocks of a tile kernel that an SM's shared memory holds (1 KB a block is the system's): a bound of five
+// would only take registers away (96 instead of 128: 1.5% of a substep of the 4.6M stress cloud).
+constexpr int kTileResident = 4;
+static_assert(kTileResident * (kTileWarps * sizeof(TileSmem) + 1024) <= 228u * 1024u &&
+                  (kTileResident + 1) * (kTileWarps * sizeof(TileSmem) + 1024) > 228u * 1024u,
+              "kTileResident is what fits");
+
 __device__ __forceinline__ float to_tf32(float x) {
     uint32_t r;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
@@ -1310,7 +1317,7 @@ __device__ __forceinline__ bool sums_lists(const SkinLists& sk) {
 // or that has more than sk.cap candidates gets no usable list. Other scenes are left alone, and
 // the launch returns at its top when no build is due.
 template <bool kBatch>
-__global__ void __launch_bounds__(kTileWarps * 32, 4)
+__global__ void __launch_bounds__(kTileWarps * 32, kTileResident)
     k_skin_build(StepLaunch L, const float4* __restrict__ pos, const uint32_t* __restrict__ scan, SkinLists sk) {
     VFS_CHAINED_LATE();
     static_assert(kSkinCap * 32 * sizeof(uint16_t) <= sizeof(float4) * kTileBlocks * 4 * kTileWordStride,
@@ -1512,7 +1519,7 @@ __device__ __forceinline__ void walk_by_warp(const SceneParams& p, uint32_t i, u
 // tiles pay most: the filter's cost per candidate is a seventh of a thread's own test (419,000
 // particles with ~900 neighbours each: 3.1 ms against 7.5 ms a warp per particle and 8.7 ms a thread
 // per particle).
-__global__ void __launch_bounds__(kTileWarps * 32, 5)
+__global__ void __launch_bounds__(kTileWarps * 32, kTileResident)
     k_walk_queue(StepLaunch L, const float4* __restrict__ pos, const float4* __restrict__ vel,
                  float4* __restrict__ rec, const uint32_t* __restrict__ scan,
                  float4* __restrict__ aux, float4* __restrict__ bnd, uint32_t* __restrict__ nbr,
