@@ -2,8 +2,8 @@
 // dispatch sizes are fixed in the shaders' numthreads). It chooses, per model or batch:
 //   * the radix sort's digit width (6, 7 or 8 bits) and items per thread (8, 12 or 16),
 //   * the neighbour passes' block shape (threads per block x minimum resident blocks per SM),
-//   * the cells-per-block of the cell-range / reorder kernel (128, 256 or 512 keys),
-// None of these changes any result: the sort is stable whatever its digits, and every particle's
+//   * the cells-per-block of the cell-range / reorder kernel (128, 256 or 512 keys).
+// What a model's size leaves unused is not timed. None of these changes any result: the sort is stable whatever its digits, and every particle's
 // sums are accumulated by one thread in the same order whatever the block shape. Candidates are
 // timed with CUDA events on the model's stream from the same saved state (restored before every
 // candidate and at the end), one stage at a time, each stage by the phases it affects. Choices are
@@ -160,8 +160,11 @@ int autotune(Model& m, int repeats, bool use_cache, vfs_tune_config* chosen) {
     };
     vfs_tune_config best = current(m);
     float ph[6];
+    // Models that sort in one launch run neither the radix passes nor the cell-range kernel: nothing
+    // to time there (a comparison would pick by noise), the present choices stay.
+    const bool one_sort = small_sort(m.n);
     // Stage 1: sort digits and items (keys + sort phases: the key pass builds the digit histograms).
-    {
+    if (!one_sort) {
         float best_t = 1e30f;
         vfs_tune_config c = best;
         for (int bits : {8, 7, 6})
@@ -183,16 +186,22 @@ int autotune(Model& m, int repeats, bool use_cache, vfs_tune_config* chosen) {
     // back on afterwards, and rebuilt by the next substep.
     const float keep_skin = m.skin_fraction;
     if (rc == VFS_OK && keep_skin > 0.0f) rc = set_skin(m, 0.0f);
-    // Stage 2: block shapes of the density and force passes (independent kernels, one sweep).
+    // Stage 2: block shapes of the density and force passes (independent kernels, one sweep). The
+    // three-lane density pass of small models has one shape.
+    const bool one_walk = planes_mode(m.n);
     if (rc == VFS_OK) {
         float best_d = 1e30f, best_f = 1e30f;
         vfs_tune_config c = best;
         for (int k = 0; k < kNumNbrShapes && rc == VFS_OK; k++) {
-            c.nbr_block = c.force_block = kShapes[k].threads;
-            c.nbr_min_blocks = c.force_min_blocks = kShapes[k].min_blocks;
+            c.force_block = kShapes[k].threads;
+            c.force_min_blocks = kShapes[k].min_blocks;
+            if (!one_walk) {
+                c.nbr_block = c.force_block;
+                c.nbr_min_blocks = c.force_min_blocks;
+            }
             measure(c, ph);
             if (rc) break;
-            if (ph[3] < best_d) {
+            if (!one_walk && ph[3] < best_d) {
                 best_d = ph[3];
                 best.nbr_block = c.nbr_block;
                 best.nbr_min_blocks = c.nbr_min_blocks;
@@ -209,7 +218,7 @@ int autotune(Model& m, int repeats, bool use_cache, vfs_tune_config* chosen) {
         if (rc == VFS_OK) rc = rs;
     }
     // Stage 3: cells per block of the cell-range / reorder kernel.
-    if (rc == VFS_OK) {
+    if (rc == VFS_OK && !one_sort) {
         float best_t = 1e30f;
         vfs_tune_config c = best;
         for (int cb : {256, 128, 512}) {
