@@ -413,7 +413,8 @@ int vfs_scene_reset(vfs_model* m);
 /* GPUCountSort::Run (src/compute/sort.cpp:107-143, sort.slang:13-55): sorts the n (key, item)
  * pairs in place by key, stably; items are first set to 0..n-1 (ClearCounts), so on return
  * items[] is the sorting permutation and keys[] the sorted keys. Keys must be <= max_value.
- * Temporary buffers come from the stream-ordered allocator. */
+ * Temporary buffers come from the stream-ordered allocator: 8 bytes a pair, 16 from three passes on
+ * (max_value above 65,535) where memory allows it, and the sort scratch. */
 int vfs_sort_pairs(uint32_t* items, uint32_t* keys, uint32_t n, uint32_t max_value, void* stream);
 /* Status of the pair sorts (vfs_sort_pairs, vfs_sort_pairs_noalloc) enqueued on the current device
  * since the previous status call: synchronises `stream`, returns the OR of their device error

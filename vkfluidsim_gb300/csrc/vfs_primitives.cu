@@ -129,10 +129,19 @@ int vfs_sort_pairs(uint32_t* items, uint32_t* keys, uint32_t n, uint32_t max_val
     uint32_t* err = nullptr;
     int rc = vfs::sort_status_address(&err);
     if (rc) return rc;
-    // One allocation: the temporaries (two pairs from three passes on), then the sort scratch.
-    const size_t pairs = sc.passes > 2 ? 2 : 1, stride = ((size_t)n + 63) & ~(size_t)63;
+    // One allocation: the temporaries (two pairs from three passes on), then the sort scratch. Where
+    // memory for a second pair is short, one will do: an odd number of passes then ends in copies back
+    // (8 bytes a pair more to move).
+    size_t pairs = sc.passes > 2 ? 2 : 1;
+    const size_t stride = ((size_t)n + 63) & ~(size_t)63;
     uint32_t* mem = nullptr;
-    VFS_PRIM_TRY(cudaMallocAsync(&mem, (2 * pairs * stride + vfs::sort_scratch_words(sc)) * 4, s));
+    cudaError_t e = cudaErrorMemoryAllocation;
+    for (;; pairs--) {
+        e = cudaMallocAsync(&mem, (2 * pairs * stride + vfs::sort_scratch_words(sc)) * 4, s);
+        if (e != cudaErrorMemoryAllocation || pairs == 1) break;
+        cudaGetLastError();
+    }
+    VFS_PRIM_TRY(e);
     uint32_t* const two = pairs > 1 ? mem + 2 * stride : nullptr;
     rc = vfs::enqueue_sort_pairs(items, keys, n, sc, mem, mem + stride, two, two ? two + stride : nullptr,
                                  mem + 2 * pairs * stride, err, s);
