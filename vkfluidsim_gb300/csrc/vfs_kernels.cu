@@ -28,27 +28,12 @@
 
 #include "vfs_chain.h"
 #include "vfs_internal.h"
+#include "vfs_tile_rule.h"
 
 namespace vfs {
 namespace {
 
 // ---------------------------------------------------------------- hashing
-
-// HashCell3D, assets/shaders/simulation/spatial_hash/spatial_hash_3d.slang:20-28.
-__device__ __forceinline__ uint32_t hash_cell(uint32_t cx, uint32_t cy, uint32_t cz) {
-    const uint32_t ux = cx + 25u, uy = cy + 25u, uz = cz + 25u;
-    const uint32_t lx = ux % 50u, ly = uy % 50u, lz = uz % 50u;
-    const uint32_t bx = ux / 50u, by = uy / 50u, bz = uz / 50u;
-    const uint32_t block_hash = bx * 15823u + by * 9737333u + bz * 440817757u;
-    return lx + 50u * (ly + 50u * lz) + block_hash;
-}
-
-// KeyFromHash (spatial_hash_3d.slang:30-32): hash % n, computed as the high word of
-// (magic * hash mod 2^64) * n with magic = ceil(2^64 / n) (exact for 32-bit operands).
-__device__ __forceinline__ uint32_t key_mod(uint32_t hash, uint64_t magic, uint32_t n) {
-    const uint64_t low = magic * (uint64_t)hash;
-    return (uint32_t)__umul64hi(low, (uint64_t)n);
-}
 
 // GetCell3D (spatial_hash_3d.slang:16-18): IEEE division, floor, saturating conversion.
 __device__ __forceinline__ uint32_t cell_coord(float x, float h) {
@@ -1047,42 +1032,19 @@ __device__ __forceinline__ bool tile_group(TileSmem& S, TileFill& f, uint32_t gr
     const float rx = xi.x - ox, ry = xi.y - oy, rz = xi.z - oz;
     const bool near = fabsf(rx) <= (hw + 0.02f) * h && fabsf(ry) <= 0.52f * h && fabsf(rz) <= 0.52f * h;
     if (!__all_sync(0xffffffffu, !mine || near)) return false;
-    // Lane r holds row r of the union's cells, in visiting order: one run of keys, or two when it
-    // crosses a 50-cell hash block along x or its keys pass n - 1.
+    // Lane r holds row r of the union's cells, in visiting order: one run of keys or two.
     const uint32_t xa = c0 - kReach, width = c1 - c0 + 1u + 2u * kReach;
-    const uint32_t block_a = (xa + 25u) / 50u, block_b = (xa + width + 24u) / 50u;
-    uint32_t n_first = width;  // cells of a row in the hash block of its first cell
-    if (block_a != block_b) {
-        n_first = 1u;
-        while ((xa + n_first + 25u) / 50u == block_a) n_first++;
-        if ((xa + n_first + 25u) / 50u != block_b) return false;
-    }
+    uint32_t n_first;  // cells of a row in the hash block of its first cell
+    if (!tile_first_cells(xa, width, n_first)) return false;
     const uint32_t row_y = lane % kSide, row_z = lane / kSide;  // cell offsets from -kReach
-    uint32_t k0 = 0u, l0 = 0u, k1 = 0u, l1 = 0u;
-    bool ok = true;
-    if (lane < kRows) {
-        const uint32_t y = cy + row_y - kReach, z = cz + row_z - kReach;
-        const uint32_t hash = hash_cell(xa, y, z);
-        k0 = key_mod(hash, p.mod_magic, p.n);
-        l0 = n_first;
-        ok = hash <= 0xFFFFFFFFu - l0;
-        if (n_first != width) {
-            const uint32_t hash1 = hash_cell(xa + n_first, y, z);
-            k1 = key_mod(hash1, p.mod_magic, p.n);
-            l1 = width - n_first;
-            ok = ok && hash1 <= 0xFFFFFFFFu - l1 && k0 + l0 <= p.n && k1 + l1 <= p.n;
-        } else if (k0 + l0 > p.n) {
-            l1 = k0 + l0 - p.n;  // continues at key 0
-            l0 -= l1;
-            ok = ok && l1 <= p.n;
-        }
-    }
+    TileRow row{0u, 0u, 0u, 0u, true};
+    if (lane < kRows)
+        row = tile_row(xa, cy + row_y - kReach, cz + row_z - kReach, width, n_first, p.n, p.mod_magic);
+    const uint32_t k0 = row.k0, l0 = row.l0, k1 = row.k1, l1 = row.l1;
+    bool ok = row.ok;
     const bool two = __any_sync(0xffffffffu, l1 != 0u);
     // Pairwise disjoint runs modulo n, so every key of the union is met once.
-    auto apart = [&](uint32_t ka, uint32_t la, uint32_t kb, uint32_t lb) {
-        const uint32_t up = kb >= ka ? kb - ka : kb + (p.n - ka), dn = ka >= kb ? ka - kb : ka + (p.n - kb);
-        return la == 0u || lb == 0u || (up >= la && dn >= lb);
-    };
+    auto apart = [&](uint32_t ka, uint32_t la, uint32_t kb, uint32_t lb) { return runs_apart(ka, la, kb, lb, p.n); };
     if (two) ok = ok && apart(k0, l0, k1, l1);
     for (uint32_t s = 1u; s <= kRows / 2u; s++) {
         const int o = (int)((lane + s >= kRows ? lane + s - kRows : lane + s) & 31u);
