@@ -223,16 +223,20 @@ int32_t vfs_model_get_neighbor_capacity(const vfs_model* m);
 /* Candidate lists with a skin (Verlet lists). At a build, each particle lists the particles within
  * h (1 + skin); until some particle of the scene has moved more than h skin / 2 since then
  * (checked every substep from the current positions, so state set by any route is seen), a
- * particle whose list was built from 125 provably distinct cell keys sums the list instead of
- * walking the 27 buckets of CalculateDensities (wcsph_with_boundary_model.slang:153-197). The
- * in-range sets are the reference's; the sums follow the visiting order of the last build. Lists
- * that go stale within 4 substeps of their build (12 in scenes below 32,768 particles, 2 from
- * 262,144 on, where a build substep costs about one and a half walks) make the scene wait up to 256 substeps before
- * building again (it walks meanwhile), so the lists pay off where the fastest particle moves less
- * than about h skin / 4 per substep and cost a few percent where particles move faster. skin in [0, 0.5],
- * default 0.05; 0 walks the buckets every substep. Models of up to ~39,000 particles (three lanes
- * per particle in the density pass) and models whose lists do not fit in device memory (433 bytes
- * per particle) have no lists; the getter then reports 0. */
+ * particle with a usable list sums it instead of walking the 27 buckets of CalculateDensities
+ * (wcsph_with_boundary_model.slang:153-197). A list is usable where it has at most 96 candidates and
+ * was built from cells (5 x 5 rows of them, around a group of particles of one row) whose runs of keys
+ * are disjoint, so that every cell's key occurs once. The in-range sets are the reference's; the sums
+ * follow the visiting order of the last build. Lists that go stale within 4 substeps of their build (12
+ * in scenes below 32,768 particles, 2 from 262,144 on) make the scene wait up to 256 substeps before
+ * building again (it walks meanwhile), so lists pay off where the fastest particle moves less than about
+ * h skin / 8 per substep (h skin / 24 in the smaller scenes, h skin / 4 in the larger ones) and cost a few
+ * percent where particles move faster; a run that is put back to one state again and again counts as
+ * moving by what it is put back by. A batch whose scenes with lists hold fewer than 98,304 particles,
+ * beside more than 16,384 others, walks all of them. skin in [0, 0.5], default 0.05; 0 walks the buckets
+ * every substep. Models of up to ~39,000 particles (three lanes per particle in the density pass) and
+ * models whose lists do not fit in device memory (433 bytes per particle, allocated with the model
+ * whether they come to be used or not) have no lists; the getter then reports 0. */
 int vfs_model_set_skin(vfs_model* m, float skin);
 int vfs_model_get_skin(const vfs_model* m, float* skin);
 /* Kept for programs that set it: the value is stored (vfs_tune_config.walk_staging, off by default) and

@@ -269,7 +269,7 @@ static void derive_scene_params(const SceneHost& sh, SceneParams& p) {
     p.bnd_eighth = 0.125f * r;
     p.bnd_half = 0.5f * r;
     p.nbr_cap = kNbrCap;
-    p.skin_r2 = p.skin_half2 = p.skin_lim = 0.0f;  // set by refresh_params when lists are on
+    p.skin_r2 = p.skin_half2 = 0.0f;  // set by refresh_params when lists are on
     p.n_objects = (uint32_t)sh.objects.size();
     p.objects = nullptr;
 }
@@ -296,7 +296,6 @@ int Model::refresh_params() {
             const float r = sh.params.h * (1.0f + skin_fraction), half = 0.5f * sh.params.h * skin_fraction;
             sh.params.skin_r2 = r * r;
             sh.params.skin_half2 = half * half;
-            sh.params.skin_lim = (1.0f + skin_fraction) * (1.0f + skin_fraction) * 1.002f;
         }
         for (const ObjectStore& o : sh.objects) {
             DevObject d{};

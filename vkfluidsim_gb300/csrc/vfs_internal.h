@@ -87,7 +87,6 @@ struct SceneParams {
     uint32_t nbr_cap;   // neighbour-list slots per particle
     float skin_r2;      // (h (1 + skin))^2: radius of the candidate lists (0: no lists)
     float skin_half2;   // (h skin / 2)^2: displacement since the last build that forces a rebuild
-    float skin_lim;     // (1 + skin)^2 x 1.002: cell pruning limit of the list build, in h^2
     uint32_t n_objects;
     const DevObject* objects;  // device array of n_objects
 };
@@ -176,17 +175,18 @@ constexpr uint32_t kCtlSince = 5;      //   stale substeps since the lists went 
 constexpr uint32_t kCtlUsable = 6;     //   usable lists left by this substep's build
 constexpr uint32_t kCtlPoor = 7;       //   the last build left too few of them usable
 constexpr uint32_t kCtlYoung = 8;      //   lists in a row that died young
-// Lists that die younger than this were not worth their build. A full GPU (1M particles): a build
-// substep 650 us, a list pass 195, a walk 450, so two substeps of use pay; a scene of 64,000
-// particles, where all three are latency: 90, 33 and 49 us, so four do; a small scene of a batch
-// walks beside the others' queues for nothing, while its build's 40 us are on the batch's critical
-// path (20 scenes of 2,500 to 21,500 particles: 194 us a substep at four, 184 at twelve).
+// Lists that die younger than this were not worth their build. A full GPU (1M flowing particles): a
+// build substep 617 us (build 475, list pass 142), a walk 448, so two substeps of use pay; a scene of
+// 64,000 particles, where all three are latency: 55 us (37 and 18) and 46
+// so four do; a small scene of a batch walks beside the others' queues for nothing, while its
+// build's 40 us are on the batch's critical path (20 scenes of 2,500 to 21,500 particles: 194 us a
+// substep at four, 184 at twelve).
 constexpr uint32_t kSkinSmallScene = 32768u, kSkinFullScene = 262144u;
 constexpr uint32_t kSkinMinLifeSmall = 12;
 constexpr uint32_t kSkinMinLife = 4;
 constexpr uint32_t kSkinMinLifeFull = 2;
 // A full scene's lists that die young once (a state set from outside just after a build) are
-// rebuilt all the same: that costs a third of a walk, waiting would cost half a walk each substep.
+// rebuilt all the same: that costs a third of a walk more, waiting two thirds of one each substep.
 constexpr uint32_t kSkinGrace = 1;
 // More than one in so many without a usable list: the list pass and their scattered walk together
 // cost more than walking every particle (1M settled particles, a third over 64 slots: 910 us against 690
