@@ -142,7 +142,7 @@ enum NbrShape : int { kNbr128x6 = 0, kNbr128x8 = 1, kNbr96x8 = 2, kNbr64x12 = 3,
 // in-range set, multiplicity one). The cell pass keeps `cur`, the current sorted index of every
 // build index, checks every displacement against `x_build` and marks the scene stale; in a stale
 // scene every particle walks, and the lists are rebuilt when the scene's build policy allows it.
-// The force pass runs the policy: lists that went stale within kSkinMinLife... substeps of their
+// The force pass runs the policy: lists that went stale within kSkinMinLife (Small, Full) substeps of their
 // build (by the scene's size), or a build that left more than one in kSkinPoorPart particles
 // without a usable list, double the substeps the scene walks before the next build (from
 // kSkinMinWait to kSkinMaxWait); longer-lived lists are rebuilt in the substep they go stale in
@@ -175,12 +175,13 @@ constexpr uint32_t kCtlSince = 5;      //   stale substeps since the lists went 
 constexpr uint32_t kCtlUsable = 6;     //   usable lists left by this substep's build
 constexpr uint32_t kCtlPoor = 7;       //   the last build left too few of them usable
 constexpr uint32_t kCtlYoung = 8;      //   lists in a row that died young
-// Lists that die younger than this were not worth their build. A full GPU (1M flowing particles): a
-// build substep 617 us (build 475, list pass 142), a walk 448, so two substeps of use pay; a scene of
-// 64,000 particles, where all three are latency: 55 us (37 and 18) and 46
-// so four do; a small scene of a batch walks beside the others' queues for nothing, while its
-// build's 40 us are on the batch's critical path (20 scenes of 2,500 to 21,500 particles: 194 us a
-// substep at four, 184 at twelve).
+// Lists that die younger than this were not worth their build. 1M flowing particles: a build substep 617
+// us (build 475, list pass 142), a walk 448; 64,000 particles: 55 (37 and 18) and 46: either way two
+// substeps of use pay. The smaller scenes' four keeps a fast flow, whose lists may die at once, to few
+// builds (ms for 24 substeps of lists that live two to five, at two, four and six: 47,000 particles 1.42 /
+// 1.84 / 1.84, 150,000 2.90 / 4.35 / 4.30; of longer-lived ones the same at two and four, at six up to 1.81 for 1.26). A
+// small scene of a batch walks beside the others' queues for nothing, while its build's 40 us are on the
+// batch's critical path (20 scenes of 2,500 to 21,500 particles: 194 us a substep at four, 184 at twelve).
 constexpr uint32_t kSkinSmallScene = 32768u, kSkinFullScene = 262144u;
 constexpr uint32_t kSkinMinLifeSmall = 12;
 constexpr uint32_t kSkinMinLife = 4;
