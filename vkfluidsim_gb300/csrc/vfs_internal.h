@@ -146,8 +146,14 @@ enum NbrShape : int { kNbr128x6 = 0, kNbr128x8 = 1, kNbr96x8 = 2, kNbr64x12 = 3,
 // build (by the scene's size), or a build that left more than one in kSkinPoorPart particles
 // without a usable list, double the substeps the scene walks before the next build (from
 // kSkinMinWait to kSkinMaxWait); longer-lived lists are rebuilt in the substep they go stale in
-// (small scenes: in the next). A single scene whose last build left too many lists unusable is
-// walked in index order, as a stale one that waits is, until its next build.
+// (small scenes: in the next). A single scene whose last build left too many lists unusable is walked in
+// index order, as a stale one that waits is, until its next build.
+// A state put back from outside between runs of substeps (a jump) costs the lists rebuilt shortly before
+// the run's end and the next run's first ones, a build each, run after run. Where lists of the middle of
+// the run would reach both its ends (runs of up to twice their life), they are built there (skin_middle),
+// and last from then on: ms for 6 substeps put back each time, 666,453 particles 1.83 -> 1.32, 770,298 2.17
+// -> 1.60 (1.45 and 1.91 with lists that a longer wait happened to build there). Where they did not last
+// (the states were new ones), 2, 4, ... 64 jumps pass before the next try, whose cost is one build.
 struct SkinLists {
     uint32_t* list = nullptr;     // in quads (nbr_word_at): the build indices of b's candidates
     uint32_t* count = nullptr;    // per build index: list length, kSkinUsable when it can be summed
@@ -157,7 +163,7 @@ struct SkinLists {
                                   // the build index of the particle the slot held), copied back
     float4* xcur = nullptr;       // per build index: current position (x, y, z) and current sorted
                                   // index (w, as bits), written by the cell pass
-    uint32_t* stale = nullptr;    // per scene: nonzero when some particle moved past h skin / 2
+    uint32_t* stale = nullptr;    // per scene: nonzero when some particle moved past h skin / 2 (kSkinStale...)
     uint32_t* ctl = nullptr;      // per scene, kSkinCtl words: the build policy's state (kCtl*)
     uint32_t* queue = nullptr;    // the particles the list pass leaves to a walk, packed from 0
     uint32_t* wcount = nullptr;   // three words: the walkers in `queue`; nonzero when some scene's
@@ -175,6 +181,15 @@ constexpr uint32_t kCtlSince = 5;      //   stale substeps since the lists went 
 constexpr uint32_t kCtlUsable = 6;     //   usable lists left by this substep's build
 constexpr uint32_t kCtlPoor = 7;       //   the last build left too few of them usable
 constexpr uint32_t kCtlYoung = 8;      //   lists in a row that died young
+constexpr uint32_t kCtlRun = 9;        //   substeps since the state last jumped (kSkinJump)
+constexpr uint32_t kCtlLife = 10;      //   substeps that lists of this run lasted (0: none died yet)
+constexpr uint32_t kCtlMiddle = 11;    //   substeps until a build in the middle of the run (0: none)
+constexpr uint32_t kCtlTried = 12;     //   the last build was one
+constexpr uint32_t kCtlFails = 13;     //   such builds in a row that were for nothing
+constexpr uint32_t kCtlPass = 14;      //   jumps to let pass before the next
+// A scene's stale word: lists out of reach, and, when fresh lists went so in a jump (one substep moved a
+// particle by more than h skin / 2, as no flow does whose lists are worth their build), bit 1.
+constexpr uint32_t kSkinStale = 1u, kSkinJump = 2u;
 // Lists that die younger than this were not worth their build. 1M flowing particles: a build substep 617
 // us (build 475, list pass 142), a walk 448; 64,000 particles: 55 (37 and 18) and 46: either way two
 // substeps of use pay. The smaller scenes' four keeps a fast flow, whose lists may die at once, to few
@@ -193,6 +208,8 @@ constexpr uint32_t kSkinGrace = 1;
 // cost more than walking every particle (1M settled particles, a third over 64 slots: 910 us against 690
 // a substep).
 constexpr uint32_t kSkinPoorPart = 8;
+// Lists built in the middle of a run that lasted longer than this have proved themselves.
+constexpr uint32_t kSkinMiddleKept = 64;
 constexpr uint32_t kSkinMinWait = 8;
 constexpr uint32_t kSkinMaxWait = 256;
 constexpr uint32_t kSkinCap = 96;  // candidates within 1.05 h: ~39 at spacing h / 2, ~49 in a settled fluid (0.46 h),

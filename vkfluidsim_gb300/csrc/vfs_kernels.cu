@@ -546,6 +546,7 @@ __device__ __forceinline__ void reorder_particle(
     const float4* __restrict__ x_build, uint32_t* __restrict__ stale, const uint32_t* __restrict__ ctl,
     uint32_t* __restrict__ wcount) {
     bool exceed = false;  // skin lists: the particle moved past h skin / 2 since its list build
+    bool jump = false;    // and as far since the last substep
     uint32_t exceed_sc = 0u;
     if (i < n) {
         uint32_t src = perm[i];
@@ -568,11 +569,16 @@ __device__ __forceinline__ void reorder_particle(
                 const uint32_t id = __float_as_uint(x.w);
                 const uint32_t bi = id < n ? __ldg(b_of_id + id) : n;
                 if (bi < n) {
-                    xcur[bi] = make_float4(x.x, x.y, x.z, __uint_as_float(i));
                     const float4 b = __ldg(x_build + bi);
                     const float dx = x.x - b.x, dy = x.y - b.y, dz = x.z - b.z;
                     const float lim = L.n_scenes > 1 ? L.scenes[sc].skin_half2 : L.one.skin_half2;
                     exceed = !(dx * dx + dy * dy + dz * dz <= lim);
+                    if (exceed) {
+                        const float4 o = xcur[bi];
+                        const float ex = x.x - o.x, ey = x.y - o.y, ez = x.z - o.z;
+                        jump = !(ex * ex + ey * ey + ez * ez <= lim);
+                    }
+                    xcur[bi] = make_float4(x.x, x.y, x.z, __uint_as_float(i));
                 }
             }
         }
@@ -582,8 +588,9 @@ __device__ __forceinline__ void reorder_particle(
         const uint32_t m = __ballot_sync(0xffffffffu, exceed);
         if (exceed) {
             const uint32_t g = __match_any_sync(m, exceed_sc);
-            if ((threadIdx.x & 31u) == (uint32_t)(__ffs(g) - 1) && ld_volatile(stale + exceed_sc) == 0u) {
-                atomicOr(stale + exceed_sc, 1u);
+            const uint32_t word = __any_sync(g, jump) ? kSkinStale | kSkinJump : kSkinStale;
+            if ((threadIdx.x & 31u) == (uint32_t)(__ffs(g) - 1) && (word & ~ld_volatile(stale + exceed_sc))) {
+                atomicOr(stale + exceed_sc, word);
                 if (ctl[exceed_sc * kSkinCtl + kCtlAllow]) wcount[1] = 1u;  // a build is due
             }
         }
@@ -2002,6 +2009,31 @@ __device__ __forceinline__ void force_finish(const SceneParams& p, uint32_t i, c
 // CalculatePressureAccel + CalculateViscousAccel + UpdatePositions
 // (wcsph_with_boundary_model.slang:205-360), fused: both sums are accumulated separately in the
 // reference's visiting order, then a = ((g - P) + V) + wall, v += a dt, x += v dt.
+// Fresh lists have gone stale, `age` substeps after their build, in a jump or by drift: the substep of the
+// run that has just begun at which to build lists that reach both its ends, if it is like the last one and
+// they can (0: no such build).
+__device__ __forceinline__ uint32_t skin_middle(uint32_t* c, uint32_t age, bool jump) {
+    if (c[kCtlTried]) {
+        const uint32_t fails = age > kSkinMiddleKept ? 0u : min(c[kCtlFails] + 1u, 6u);
+        c[kCtlTried] = 0u;
+        c[kCtlFails] = fails;
+        c[kCtlPass] = fails ? 1u << fails : 0u;
+    }
+    if (!jump) {
+        c[kCtlLife] = age;
+        return 0u;
+    }
+    const uint32_t run = c[kCtlRun], life = c[kCtlLife];
+    c[kCtlRun] = c[kCtlLife] = 0u;
+    if (c[kCtlPass]) {
+        c[kCtlPass]--;
+        return 0u;
+    }
+    if (life == 0u || run > 2u * life + 1u || c[kCtlPoor]) return 0u;
+    c[kCtlTried] = 1u;
+    return run / 2u;
+}
+
 template <bool kBatch, int kNbrBlock, int kMinBlocks>
 __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
     k_force(StepLaunch L, const float4* __restrict__ pos, const float4* __restrict__ vel,
@@ -2030,8 +2062,13 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
                                                            : kSkinMinLifeFull;
             const uint32_t grace = n < kSkinFullScene ? 0u : kSkinGrace;
             uint32_t age = c[kCtlAge], wait = c[kCtlWait], since = c[kCtlSince], young = c[kCtlYoung];
+            uint32_t middle = c[kCtlMiddle];
             if (stale && c[kCtlFresh]) {  // the last build's lists just went stale: were they worth it?
-                if (age < min_life || c[kCtlPoor]) {
+                middle = n >= kSkinSmallScene ? skin_middle(c, age, (skin_stale[sc] & kSkinJump) != 0u) : 0u;
+                if (middle && !c[kCtlAllow]) {  // not rebuilt now: it walks until then
+                    wait = middle;
+                    middle = 0u;
+                } else if (age < min_life || c[kCtlPoor]) {
                     young++;
                     if (young > grace || c[kCtlPoor]) wait = min(max(2u * wait, kSkinMinWait), kSkinMaxWait);
                 } else {
@@ -2050,7 +2087,13 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
                 age++;
                 if (stale) since++;
             }
+            if (middle && --middle == 0u) {  // the lists rebuilt at the jump have served
+                c[kCtlFresh] = 0u;
+                wait = since = 0u;
+            }
             skin_stale[sc] = 0u;
+            c[kCtlRun]++;
+            c[kCtlMiddle] = middle;
             c[kCtlAge] = age;
             c[kCtlWait] = wait;
             c[kCtlSince] = since;
