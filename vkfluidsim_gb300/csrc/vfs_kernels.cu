@@ -799,10 +799,15 @@ constexpr int kListBlock = 128;
 // 16,384 or 32,768, 8.14 at 65,536).
 constexpr uint32_t kWalkerCrowd = 8192;
 constexpr uint32_t kBatchCrowd = 16384;
-// Lists of fewer particles than this beside a crowd of walkers are left alone in a batch: every scene
-// walks. The list pass costs ~25 us however few it sums, a walk less its lists' particles saves ~0.3 us
-// for every thousand (ms a pass, lists always / from 49,152 / 98,304 / 147,456: 32 scenes of up to 20,098
-// particles 8.58 / 8.60 / 8.46 / 8.45, 13 of up to 23,237 4.95 / 4.52 / 4.52 / 4.53, 64 of up to 65,536 the same).
+// Lists of fewer particles than kBatchListed are left alone in a batch beside a crowd of walkers, or beside
+// more than one in kBatchWalked of its particles: every scene walks. The list pass costs ~25 us however few
+// it sums, a walk less its lists' particles saves ~0.3 us for every thousand (ms a pass, lists always /
+// from 49,152 / 98,304 / 147,456: 32 scenes of up to 20,098 particles 8.58 / 8.60 / 8.46 / 8.45, 13 of up to
+// 23,237 4.95 / 4.52 / 4.52 / 4.53, 64 of up to 65,536 the same), and the smallest batches walk in less than
+// a wave whatever is left (crowds alone / one in four / six / eight: 39,742 particles 4.64 / 4.36 / 4.40 /
+// 4.39, 40,403 4.05 / 3.52 / 3.52 / 3.50, 56,717 4.24 / 4.25 / 3.67 / 3.64, 49,754 4.32 / 4.33 / 4.69 / 4.67; calm
+// batches the same).
+constexpr uint32_t kBatchWalked = 6;
 constexpr uint32_t kBatchListed = 98304;
 
 // 1 / sqrt(x) for a normal x (the form without ftz spends four more instructions on denormals).
@@ -2108,7 +2113,7 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
             __syncthreads();
             if (listed) atomicAdd(&s_listed, listed);
             __syncthreads();
-            const bool off = s_listed < kBatchListed && L.total - s_listed > kBatchCrowd;
+            const bool off = s_listed < kBatchListed && L.total - s_listed > min(kBatchCrowd, L.total / kBatchWalked);
             if (threadIdx.x == 0) skin_due[1] = off ? 1u : 0u;
             if (off)
                 for (uint32_t sc = threadIdx.x; sc < L.n_scenes; sc += blockDim.x) skin_ctl[sc * kSkinCtl + kCtlAllow] = 0u;
