@@ -1623,7 +1623,8 @@ __global__ void __launch_bounds__(kNbrBlock, kBatch || kMinBlocks * kNbrBlock > 
     // the next run.
     uint32_t slots = L.total;
     const uint32_t warps = gridDim.x * (uint32_t)(kNbrBlock / 32);
-    if (kBatch && sk.list) {
+    const bool queued = kBatch && sk.list && sk.wcount[2] == 0u;  // (else every particle, in index order)
+    if (queued) {
         slots = min(*sk.wcount, L.total);
         if (slots == 0u) chained_release();
         if (slots <= kBatchCrowd) {
@@ -1641,7 +1642,7 @@ __global__ void __launch_bounds__(kNbrBlock, kBatch || kMinBlocks * kNbrBlock > 
         const uint32_t t = run * 32u + lane;
         const bool act = t < slots;
         uint32_t i = act ? t : 0u;
-        if (kBatch && act && sk.list) i = __ldg(sk.queue + t);
+        if (queued && act) i = __ldg(sk.queue + t);
         // The next run, claimed now so that the counter's latency hides behind this one.
         uint32_t next = 0u;
         if (lane == 0u) next = warps + atomicAdd(sched, 1u);
@@ -1712,14 +1713,14 @@ __global__ void __launch_bounds__(kListBlock, 9)
     const uint32_t i = blockIdx.x * kListBlock + threadIdx.x;
     // A single scene that is stale and waits, or whose last build left most lists unusable: k_walk walks
     // it in index order.
-    if (!kBatch && !sums_lists(sk)) return;
+    if (kBatch ? sk.wcount[2] != 0u : !sums_lists(sk)) return;
     bool walk = false;
     if (i < L.total) {
         const SceneParams& p = scene_params<kBatch>(L, i);
         uint32_t c = 0u, row = 0u;
         const uint32_t scene = kBatch ? (uint32_t)__ldg(L.scene_of + i) : 0u;
         const bool built = sk.stale[scene] != 0u;  // this substep, unless the scene is walked
-        walk = !lists_in_use(sk, scene) || (kBatch && sk.wcount[2] != 0u);
+        walk = !lists_in_use(sk, scene);
         // A particle of a stale scene only joins the queue: its position is not read.
         const float4 xi = walk ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : __ldg(pos + i);
         if (!walk) {
