@@ -1,6 +1,6 @@
-"""A batch of fewer than 98,304 particles in scenes with lists walks them all where more than one in six of
-its particles has no list to sum (scenes of 3,400 whose keys collide), and builds no more lists; otherwise
-the moving scene's are rebuilt. The fields hold the parity bar against the batch without lists."""
+"""A batch of few particles in scenes with lists (three eighths of it, at least 49,152) walks them all where
+more than one in six of its particles has no list to sum (scenes of 3,400 whose keys collide), and builds no
+more lists; otherwise the moving scene's are rebuilt. The fields hold the parity bar against the batch without lists."""
 from __future__ import annotations
 
 import numpy as np
@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("large, small, lists_used", [
-    (39_999, 2, True), (34_000, 2, True), (33_999, 2, False), (40_000, 4, False), (68_000, 4, True)])
+    (39_999, 2, True), (34_000, 2, True), (33_999, 2, False), (40_000, 4, False), (68_000, 4, True),
+    (49_151, 4, False), (49_152, 4, True), (56_000, 28, False), (60_000, 28, True)])
 def test_one_walker_in_six(large, small, lists_used):
     scenes = [scene(large, 1)] + [scene(3400, 2 + k) for k in range(small)]
     scenes[0].objects = []  # (the container's map would throw its wall particles)

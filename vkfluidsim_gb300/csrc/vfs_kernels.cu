@@ -799,14 +799,15 @@ constexpr int kListBlock = 128;
 // 16,384 or 32,768, 8.14 at 65,536).
 constexpr uint32_t kWalkerCrowd = 8192;
 constexpr uint32_t kBatchCrowd = 16384;
-// Lists of fewer particles than kBatchListed are left alone in a batch beside a crowd of walkers, or beside
-// more than one in kBatchWalked of its particles: every scene walks. The list pass costs ~25 us however few
-// it sums, a walk less its lists' particles saves ~0.3 us for every thousand (ms a pass, lists always /
-// from 49,152 / 98,304 / 147,456: 32 scenes of up to 20,098 particles 8.58 / 8.60 / 8.46 / 8.45, 13 of up to
-// 23,237 4.95 / 4.52 / 4.52 / 4.53, 64 of up to 65,536 the same), and the smallest batches walk in less than
-// a wave whatever is left (crowds alone / one in four / six / eight: 39,742 particles 4.64 / 4.36 / 4.40 /
-// 4.39, 40,403 4.05 / 3.52 / 3.52 / 3.50, 56,717 4.24 / 4.25 / 3.67 / 3.64, 49,754 4.32 / 4.33 / 4.69 / 4.67; calm
-// batches the same).
+// A batch's lists of fewer particles than a line are left alone beside a crowd of walkers, or beside more
+// than one in kBatchWalked of its particles: every scene walks. The line is three eighths of the batch,
+// between half of kBatchListed and kBatchListed: the list pass costs ~25 us however few it sums, a walk less
+// its lists' particles saves ~0.3 us for every thousand, the less the more there are (ms a pass at lines of
+// 49,152 / 65,536 / 98,304: 117,906 particles 5.93 / 6.19 / 6.13, 140,822 5.53 / 5.85 / 5.80, 165,121 5.60 / 5.67 /
+// 5.89, 231,700 9.49 / 9.38 / 8.84, 245,147 16.60 / 16.01 / 15.92; a third, three eighths, two fifths: 140,822
+// 5.57 / 5.51 / 5.84, 22 others within 2%). The smallest batches walk in less than a wave whatever is left
+// (crowds alone / one in four / six / eight: 39,742 particles 4.64 / 4.36 / 4.40 / 4.39, 40,403 4.05 / 3.52 / 3.52 /
+// 3.50, 56,717 4.24 / 4.25 / 3.67 / 3.64, 49,754 4.32 / 4.33 / 4.69 / 4.67; calm batches the same).
 constexpr uint32_t kBatchWalked = 6;
 constexpr uint32_t kBatchListed = 98304;
 
@@ -2114,7 +2115,8 @@ __global__ void __launch_bounds__(kNbrBlock, kMinBlocks)
             __syncthreads();
             if (listed) atomicAdd(&s_listed, listed);
             __syncthreads();
-            const bool off = s_listed < kBatchListed && L.total - s_listed > min(kBatchCrowd, L.total / kBatchWalked);
+            const uint32_t line = min(kBatchListed, max(kBatchListed / 2u, L.total / 8u * 3u));
+            const bool off = s_listed < line && L.total - s_listed > min(kBatchCrowd, L.total / kBatchWalked);
             if (threadIdx.x == 0) skin_due[1] = off ? 1u : 0u;
             if (off)
                 for (uint32_t sc = threadIdx.x; sc < L.n_scenes; sc += blockDim.x) skin_ctl[sc * kSkinCtl + kCtlAllow] = 0u;
