@@ -232,12 +232,12 @@ int32_t vfs_model_get_neighbor_capacity(const vfs_model* m);
  * building again (it walks meanwhile), so lists pay off where the fastest particle moves less than about
  * h skin / 8 per substep (h skin / 24 in the smaller scenes, h skin / 4 in the larger ones) and cost a few
  * percent where particles move faster. A run that is put back to one state again and again, and whose
- * lists would last half of it, is given lists from its middle, which last. A batch whose scenes with
- * lists hold fewer than 98,304 particles, beside more than 16,384 others or more than one in six of all,
- * walks all of them. skin in [0, 0.5], default 0.05; 0 walks the buckets every substep. Models of up to
- * ~39,000 particles (three lanes per particle in the density pass) and models whose lists do not fit in
- * device memory (433 bytes per particle, allocated with the model whether they come to be used or not)
- * have no lists; the getter then reports 0. */
+ * lists would last half of it, is given lists from its middle, which last. A batch walks all of its
+ * scenes where those with lists hold less than three eighths of its particles (a line kept between 49,152
+ * and 98,304) and leave more than 16,384 others or more than one in six. skin in [0, 0.5], default 0.05; 0
+ * walks the buckets every substep. Models of up to ~39,000 particles (three lanes per particle in the
+ * density pass) and models whose lists do not fit in device memory (433 bytes per particle, allocated with
+ * the model whether they come to be used or not) have no lists; the getter then reports 0. */
 int vfs_model_set_skin(vfs_model* m, float skin);
 int vfs_model_get_skin(const vfs_model* m, float* skin);
 /* Kept for programs that set it: the value is stored (vfs_tune_config.walk_staging, off by default) and

@@ -1594,8 +1594,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileResident)
 // except i itself, in visiting order, in quads (nbr_word_at), and its length in nbr_count[i] (a length above nbr_cap means the list
 // overflowed and was truncated). Positions do not change before the force pass, so that list is
 // exactly the force pass's neighbour set. It walks whole scenes in index order (no skin lists; a
-// single scene that is stale and may not rebuild, or whose lists are mostly unusable) and a batch's
-// queue. A single scene whose lists are summed returns at the kernel's top. One
+// single scene that is stale and may not rebuild, or whose lists are mostly unusable; a batch whose lists
+// are left alone) and a batch's queue. A single scene whose lists are summed returns at the kernel's top. One
 // resident wave whose warps claim runs of 32 slots; a single scene's shapes of 768 threads an SM are held
 // to the 72 registers that let 28 warps in (74, 24 warps: 130,000 particles walking 92 us, 72 76). The tiles above are no faster for a fluid's ~43
 // neighbours: 515 us against 450 us for 1M particles (their sum phase runs at 16 warps per SM, this
@@ -1712,8 +1712,8 @@ __global__ void __launch_bounds__(kListBlock, 9)
     if (!late) chained_release();
     __shared__ uint32_t s_ring[8 * kListBlock];
     const uint32_t i = blockIdx.x * kListBlock + threadIdx.x;
-    // A single scene that is stale and waits, or whose last build left most lists unusable: k_walk walks
-    // it in index order.
+    // A single scene that is stale and waits, or whose last build left most lists unusable, or a batch whose
+    // lists are left alone: k_walk walks it in index order (queueing all of a batch took 7 to 11 us a substep).
     if (kBatch ? sk.wcount[2] != 0u : !sums_lists(sk)) return;
     bool walk = false;
     if (i < L.total) {
